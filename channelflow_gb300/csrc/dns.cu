@@ -622,6 +622,7 @@ struct cfgpu_dns_s {
   // transforms
   FftPlan px{}, pz{};
   void *twx = nullptr, *twz = nullptr;  // R-typed complex
+  void *twxq = nullptr, *twzq = nullptr;  // FP64: the same as fixed-point splits (fx_twiddles)
   // fused x/z pass (rotational form): full-circle twiddle tables exp(-2 pi i e/L), cluster shape
   void *twxf = nullptr, *twzf = nullptr;
   bool xzf = false;
@@ -854,11 +855,11 @@ int nonlinear_impl(cfgpu_dns d, const double* U, void* Nout, int form) {
                      (const cpx<R>*)d->twzf, d->st, dt));
     d->launches += 1;
   } else {
-    CK(launch_xinv<R>(gp, d->px, (const cpx<R>*)d->twx, (const cpx<R>*)W, (cpx<R>*)d->X6, nin, d->st, d->xcols,
+    CK(launch_xinv<R>(gp, d->px, (const cpx<R>*)d->twx, d->twxq, (const cpx<R>*)W, (cpx<R>*)d->X6, nin, d->st, d->xcols,
                       dt));
-    CK(launch_zphys<R>(gp, form, d->pz, (const cpx<R>*)d->twz, d->RP, (const cpx<R>*)d->X6, (cpx<R>*)d->Z3, d->st,
+    CK(launch_zphys<R>(gp, form, d->pz, (const cpx<R>*)d->twz, d->twzq, d->RP, (const cpx<R>*)d->X6, (cpx<R>*)d->Z3, d->st,
                        dt, (const cpx<R>*)d->twzf));
-    CK(launch_xfwd<R>(gp, d->px, (const cpx<R>*)d->twx, (const cpx<R>*)d->Z3, (cpx<R>*)d->F3, nout, d->st,
+    CK(launch_xfwd<R>(gp, d->px, (const cpx<R>*)d->twx, d->twxq, (const cpx<R>*)d->Z3, (cpx<R>*)d->F3, nout, d->st,
                       d->xcols, dt));
     d->launches += 3;
   }
@@ -1424,6 +1425,14 @@ int upload_as(const std::vector<double>& v, void** dst, long long& bytes, cudaSt
   return CFGPU_OK;
 }
 
+int upload_ints(const std::vector<int>& t, void** dst, long long& bytes, cudaStream_t st) {
+  int* p;
+  CKS(dalloc(&p, t.size(), bytes));
+  CK(cudaMemcpyAsync(p, t.data(), t.size() * sizeof(int), cudaMemcpyHostToDevice, st));
+  *dst = p;
+  return CFGPU_OK;
+}
+
 template <typename R>
 int upload_tw(const std::vector<std::complex<long double>>& tw, void** dst, long long& bytes, cudaStream_t st) {
   std::vector<cpx<R>> t(tw.size() ? tw.size() : 1);
@@ -1494,9 +1503,9 @@ int autotune(cfgpu_dns d, int form, int nin, int nout) {
     const int c = (gp.NKz + div - 1) / div;
     if (c < 2 || xfft_smem_bytes<R>(gp, c) > 200 * 1024) continue;
     const float t = time_ms<R>(d, [&]() {
-      cudaError_t e = launch_xinv<R>(gp, d->px, tw, (const cpx<R>*)d->W6, (cpx<R>*)d->X6, nin, d->st, c);
+      cudaError_t e = launch_xinv<R>(gp, d->px, tw, d->twxq, (const cpx<R>*)d->W6, (cpx<R>*)d->X6, nin, d->st, c);
       if (e != cudaSuccess) return e;
-      return launch_xfwd<R>(gp, d->px, tw, (const cpx<R>*)d->Z3, (cpx<R>*)d->F3, nout, d->st, c);
+      return launch_xfwd<R>(gp, d->px, tw, d->twxq, (const cpx<R>*)d->Z3, (cpx<R>*)d->F3, nout, d->st, c);
     });
     if (t < best) {
       best = t;
@@ -1510,7 +1519,7 @@ int autotune(cfgpu_dns d, int form, int nin, int nout) {
     for (int rp = d->RP; rp >= 2; rp /= 2) {
       if (zphys_smem_bytes<R>(gp, form, rp) > 200 * 1024) continue;
       const float t = time_ms<R>(d, [&]() {
-        return launch_zphys<R>(gp, form, d->pz, (const cpx<R>*)d->twz, rp, (const cpx<R>*)d->X6, (cpx<R>*)d->Z3,
+        return launch_zphys<R>(gp, form, d->pz, (const cpx<R>*)d->twz, d->twzq, rp, (const cpx<R>*)d->X6, (cpx<R>*)d->Z3,
                                d->st, kNoDither, (const cpx<R>*)d->twzf);
       });
       if (t < best) {
@@ -1568,13 +1577,13 @@ int tune_xz(cfgpu_dns d) {
       }
       // the three-kernel path (x inverse, z pass, x forward) with its own tuned shapes, if faster
       const float t3 = time_ms<R>(d, [&]() {
-        cudaError_t e = launch_xinv<R>(gp, d->px, (const cpx<R>*)d->twx, (const cpx<R>*)d->W6, (cpx<R>*)d->X6, 6,
+        cudaError_t e = launch_xinv<R>(gp, d->px, (const cpx<R>*)d->twx, d->twxq, (const cpx<R>*)d->W6, (cpx<R>*)d->X6, 6,
                                        d->st, d->xcols);
         if (e == cudaSuccess)
-          e = launch_zphys<R>(gp, NL_ROTATIONAL, d->pz, (const cpx<R>*)d->twz, d->RP, (const cpx<R>*)d->X6,
+          e = launch_zphys<R>(gp, NL_ROTATIONAL, d->pz, (const cpx<R>*)d->twz, d->twzq, d->RP, (const cpx<R>*)d->X6,
                               (cpx<R>*)d->Z3, d->st, kNoDither, (const cpx<R>*)d->twzf);
         if (e == cudaSuccess)
-          e = launch_xfwd<R>(gp, d->px, (const cpx<R>*)d->twx, (const cpx<R>*)d->Z3, (cpx<R>*)d->F3, 3, d->st,
+          e = launch_xfwd<R>(gp, d->px, (const cpx<R>*)d->twx, d->twxq, (const cpx<R>*)d->Z3, (cpx<R>*)d->F3, 3, d->st,
                              d->xcols);
         return e;
       });
@@ -1841,6 +1850,8 @@ int dns_create_impl(cfgpu_dns d, const cfgpu_grid* grid, const cfgpu_flags* flag
   if (fp64) {
     CKS(upload_tw<double>(twx, &d->twx, B, d->st));
     CKS(upload_tw<double>(twz, &d->twz, B, d->st));
+    CKS(upload_ints(fx_twiddles(twx), &d->twxq, B, d->st));
+    CKS(upload_ints(fx_twiddles(twz), &d->twzq, B, d->st));
     CKS(upload_as<double>(circx, &d->twxf, B, d->st));
     CKS(upload_as<double>(circz, &d->twzf, B, d->st));
     CKS(upload_as<double>(cm.invA, &d->cinvA, B, d->st));
@@ -2038,7 +2049,7 @@ void dns_free(cfgpu_dns d) {
   F(d->twxf); F(d->twzf); F(d->cdct); F(d->ctc); F(d->dtcerr);
   F(d->dUbase); F(d->dWbase); F(d->dUbaseyy); F(d->dWbaseyy); F(d->ddPdx);
   F(d->hb_lo); F(d->hb_di); F(d->hb_up);
-  F(d->twx); F(d->twz); F(d->cinvA); F(d->cinvB); F(d->cfwdA); F(d->cfwdB);
+  F(d->twx); F(d->twz); F(d->twxq); F(d->twzq); F(d->cinvA); F(d->cinvB); F(d->cfwdA); F(d->cfwdB);
   F(d->cderA); F(d->cderB); F(d->basey); F(d->cdfA); F(d->cdfB); F(d->dyc); F(d->dred); F(d->dmodes);
   F(d->dslot); F(d->dbaseS); F(d->baseyS); F(d->zbasey); F(d->cblock); F(d->dver);
   F(d->Ucur); F(d->Qcur);
@@ -2088,7 +2099,7 @@ int cfl_enqueue(cfgpu_dns d) {
                            (const R*)d->cderB, (const R*)(d->hetero ? d->baseyS : d->basey), 0.0, d->st,
                            d->hetero ? 4 * d->N : 0));
   }
-  CK(launch_xinv<R>(d->gp, d->px, (const cpx<R>*)d->twx, (const cpx<R>*)W, (cpx<R>*)d->X6, 3, d->st, d->xcols));
+  CK(launch_xinv<R>(d->gp, d->px, (const cpx<R>*)d->twx, d->twxq, (const cpx<R>*)W, (cpx<R>*)d->X6, 3, d->st, d->xcols));
   CK(cudaMemsetAsync(d->dred, 0, d->nb * sizeof(unsigned long long), d->st));
   CK(launch_zcfl<R>(d->gp, d->pz, (const cpx<R>*)d->twz, d->RP, (const cpx<R>*)d->X6, d->dyc, g.Lx / g.Nx,
                     g.Lz / g.Nz, d->nb, d->dred, d->st));

@@ -2,6 +2,7 @@
 // the host runtime (not part of the public C ABI).
 #pragma once
 
+#include <complex>
 #include <cstdint>
 #include <string>
 #include <vector>
@@ -68,10 +69,12 @@ template <typename R>
 size_t zphys_smem_bytes(const GridDev& g, int form, int RP);
 // z pass of the x/z path (c2r, the form's products, r2c).  With twzf (the full-circle twiddle table
 // exp(-2 pi i e / Nz), e < Nz) the FP32 rotational form runs with register-resident FFTs where Nz allows
-// (launch_zrot, csrc/z_reg.cu), else the generic Stockham kernel.
+// (launch_zrot, csrc/z_reg.cu), else the generic Stockham kernel.  FP64 runs on 64-bit integers (csrc/xz_fx.cu) with
+// the twiddles twq = fx_twiddles of the plan's table; twz is unused there.
 template <typename R>
-cudaError_t launch_zphys(const GridDev& g, int form, const FftPlan& pz, const cpx<R>* twz, int RP, const cpx<R>* X,
-                         cpx<R>* Z, cudaStream_t st, const Dither& dt = kNoDither, const cpx<R>* twzf = nullptr);
+cudaError_t launch_zphys(const GridDev& g, int form, const FftPlan& pz, const cpx<R>* twz, const void* twq, int RP,
+                         const cpx<R>* X, cpx<R>* Z, cudaStream_t st, const Dither& dt = kNoDither,
+                         const cpx<R>* twzf = nullptr);
 // Rotational z pass with register FFTs, FP32 (Nz in {32, 48, 64, 96, 128}, RC x rows per CTA);
 // cudaErrorNotSupported, with nothing launched, for other lengths or when switched off (set_zpass_register(0)).
 cudaError_t launch_zrot(const GridDev& g, int RC, const cpx<float>* X, cpx<float>* Z, const cpx<float>* twzf,
@@ -96,13 +99,22 @@ cudaError_t launch_rotation(const GridDev& g, int N, const double* U, const doub
 template <typename R>
 size_t xfft_smem_bytes(const GridDev& g, int czc = 0);  // czc <= 0: all solved kz columns that fit
 
-// x passes: czc kz columns per block (0: as many as fit in shared memory)
+// x passes: czc kz columns per block (0: as many as fit in shared memory); FP64 on 64-bit integers, as the z pass
 template <typename R>
-cudaError_t launch_xinv(const GridDev& g, const FftPlan& px, const cpx<R>* twx, const cpx<R>* W, cpx<R>* X, int ncomp,
-                        cudaStream_t st, int czc = 0, const Dither& dt = kNoDither);
+cudaError_t launch_xinv(const GridDev& g, const FftPlan& px, const cpx<R>* twx, const void* twq, const cpx<R>* W,
+                        cpx<R>* X, int ncomp, cudaStream_t st, int czc = 0, const Dither& dt = kNoDither);
 template <typename R>
-cudaError_t launch_xfwd(const GridDev& g, const FftPlan& px, const cpx<R>* twx, const cpx<R>* Z, cpx<R>* F, int ncomp,
-                        cudaStream_t st, int czc = 0, const Dither& dt = kNoDither);
+cudaError_t launch_xfwd(const GridDev& g, const FftPlan& px, const cpx<R>* twx, const void* twq, const cpx<R>* Z,
+                        cpx<R>* F, int ncomp, cudaStream_t st, int czc = 0, const Dither& dt = kNoDither);
+
+// The FP64 passes on 64-bit integers (xz_fx.cu): fx_twiddles splits a plan's twiddle table (four ints per entry).
+std::vector<int> fx_twiddles(const std::vector<std::complex<long double>>& tw);
+cudaError_t launch_xinv_fx(const GridDev& g, const FftPlan& px, const void* tw, const cpx<double>* W, cpx<double>* X,
+                           int ncomp, int czc, cudaStream_t st);
+cudaError_t launch_xfwd_fx(const GridDev& g, const FftPlan& px, const void* tw, const cpx<double>* Z, cpx<double>* F,
+                           int ncomp, int czc, cudaStream_t st);
+cudaError_t launch_zphys_fx(const GridDev& g, int form, const FftPlan& pz, const void* tw, int RP, const cpx<double>* X,
+                            cpx<double>* Z, cudaStream_t st);
 
 // Fused x/z pass of the rotational form (xz_fused.cu, xz_fused.cuh): one thread-block cluster of C CTAs per
 // plane of gp, RC x rows per z chunk; W = u, v, w, ox, oy, oz at the Gauss-Lobatto points ([c][plane][mode]),

@@ -650,39 +650,47 @@ size_t xfft_smem_bytes(const GridDev& g, int czc) {
 }
 
 template <typename R>
-cudaError_t launch_xinv(const GridDev& g, const FftPlan& px, const cpx<R>* twx, const cpx<R>* W, cpx<R>* X, int ncomp,
-                        cudaStream_t st, int czc, const Dither& dt) {
-  // kernel attributes set once per process (thread-safe static initialisation)
-  static const bool attr_set = [] {
-    cudaFuncSetAttribute(k_xinv<R>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
-    return true;
-  }();
-  (void)attr_set;
+cudaError_t launch_xinv(const GridDev& g, const FftPlan& px, const cpx<R>* twx, const void* twq, const cpx<R>* W,
+                        cpx<R>* X, int ncomp, cudaStream_t st, int czc, const Dither& dt) {
   if (czc <= 0 || czc > g.NKz) czc = xfft_cols<R>(g);
-  return launch_pdl(k_xinv<R>, dim3(g.Ny, ncomp, (g.NKz + czc - 1) / czc), dim3(256), xfft_smem_bytes<R>(g, czc), st,
-                    g, px, twx, W, X, czc, dt);
+  if constexpr (sizeof(R) == 8) {
+    return launch_xinv_fx(g, px, twq, W, X, ncomp, czc, st);
+  } else {
+    // kernel attributes set once per process (thread-safe static initialisation)
+    static const bool attr_set = [] {
+      cudaFuncSetAttribute(k_xinv<R>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
+      return true;
+    }();
+    (void)attr_set;
+    return launch_pdl(k_xinv<R>, dim3(g.Ny, ncomp, (g.NKz + czc - 1) / czc), dim3(256), xfft_smem_bytes<R>(g, czc), st,
+                      g, px, twx, W, X, czc, dt);
+  }
 }
 
 template <typename R>
-cudaError_t launch_xfwd(const GridDev& g, const FftPlan& px, const cpx<R>* twx, const cpx<R>* Z, cpx<R>* F, int ncomp,
-                        cudaStream_t st, int czc, const Dither& dt) {
-  // kernel attributes set once per process (thread-safe static initialisation)
-  static const bool attr_set = [] {
-    cudaFuncSetAttribute(k_xfwd<R>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
-    return true;
-  }();
-  (void)attr_set;
-  const double scale = 1.0 / ((double)g.Nx * (double)g.Nz);
+cudaError_t launch_xfwd(const GridDev& g, const FftPlan& px, const cpx<R>* twx, const void* twq, const cpx<R>* Z,
+                        cpx<R>* F, int ncomp, cudaStream_t st, int czc, const Dither& dt) {
   if (czc <= 0 || czc > g.NKz) czc = xfft_cols<R>(g);
-  return launch_pdl(k_xfwd<R>, dim3(g.Ny, ncomp, (g.NKz + czc - 1) / czc), dim3(256), xfft_smem_bytes<R>(g, czc), st,
-                    g, px, twx, Z, F, scale, czc, dt);
+  if constexpr (sizeof(R) == 8) {
+    return launch_xfwd_fx(g, px, twq, Z, F, ncomp, czc, st);
+  } else {
+    // kernel attributes set once per process (thread-safe static initialisation)
+    static const bool attr_set = [] {
+      cudaFuncSetAttribute(k_xfwd<R>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
+      return true;
+    }();
+    (void)attr_set;
+    const double scale = 1.0 / ((double)g.Nx * (double)g.Nz);
+    return launch_pdl(k_xfwd<R>, dim3(g.Ny, ncomp, (g.NKz + czc - 1) / czc), dim3(256), xfft_smem_bytes<R>(g, czc), st,
+                      g, px, twx, Z, F, scale, czc, dt);
+  }
 }
 
 #define INST_R(R)                                                                                                   \
-  template cudaError_t launch_xinv<R>(const GridDev&, const FftPlan&, const cpx<R>*, const cpx<R>*, cpx<R>*, int,   \
-                                      cudaStream_t, int, const Dither&);                                            \
-  template cudaError_t launch_xfwd<R>(const GridDev&, const FftPlan&, const cpx<R>*, const cpx<R>*, cpx<R>*, int,   \
-                                      cudaStream_t, int, const Dither&);                                            \
+  template cudaError_t launch_xinv<R>(const GridDev&, const FftPlan&, const cpx<R>*, const void*, const cpx<R>*,    \
+                                      cpx<R>*, int, cudaStream_t, int, const Dither&);                              \
+  template cudaError_t launch_xfwd<R>(const GridDev&, const FftPlan&, const cpx<R>*, const void*, const cpx<R>*,    \
+                                      cpx<R>*, int, cudaStream_t, int, const Dither&);                              \
   template size_t xfft_smem_bytes<R>(const GridDev&, int);
 
 INST_R(float)

@@ -1,0 +1,427 @@
+// x and z passes of the FP64 path on 64-bit integers (fx.cuh): the x inverse and forward FFTs of the solved
+// columns of one y-plane and component, and the z pass (c2r, the nonlinear form's products, r2c).  Arrays in and
+// out are the FP64 arrays of the generic passes (k_xinv, k_zphys, k_xfwd), in the same layout.
+//
+// Every line is scaled on its own: a column of the x passes, each real row of the z pass (two rows share a complex
+// sequence, with a scale each).
+//
+// Measured at 128x97x128 against the same passes in FP64 arithmetic, which the FP64 pipe bounds (one warp instruction
+// per 64 cycles): z pass 340 -> 123 us, x inverse 134 -> 55 us, x forward 76 -> 29 us; bound here by integer issue.
+// Relative error of N(u) against extended precision: 1.5e-16 ... 2.5e-16 at 32x9x32 (FP64 arithmetic 2.7e-16 ...
+// 8.8e-16), for spectra from 0.5^(|kx|+|kz|) to flat.
+#include "fx.cuh"
+#include "kernels.h"
+
+namespace {
+
+constexpr int FX_THREADS = 256;
+
+__device__ __forceinline__ double fx_raw(long long v) { return __longlong_as_double(v); }
+
+// Scales the raw doubles of one complex column (elements pos(i), i < n, all others zero) to integers in place; one
+// warp.  Returns K.
+template <class POS>
+__device__ __forceinline__ int fx_scale_column(fxc* col, int n, POS pos, int lane) {
+  unsigned key = 0;
+  for (int i = lane; i < n; i += 32) {
+    const fxc v = col[pos(i)];
+    key = max(key, max(fx_key(fx_raw(v.x)), fx_key(fx_raw(v.y))));
+  }
+  key = __reduce_max_sync(0xffffffffu, key);
+  const int emax = fx_exp_of_key(key);
+  unsigned S = 0;
+  for (int i = lane; i < n; i += 32) {
+    const fxc v = col[pos(i)];
+    S += fx_mag(fx_raw(v.x), emax) + fx_mag(fx_raw(v.y), emax);
+  }
+  S = __reduce_add_sync(0xffffffffu, S);
+  const int K = fx_line_K(emax, S, 61);
+  for (int i = lane; i < n; i += 32) {
+    const fxc v = col[pos(i)];
+    col[pos(i)] = key == 0 ? fxc{0, 0} : fxc{fx_quant(fx_raw(v.x), K), fx_quant(fx_raw(v.y), K)};
+  }
+  return key == 0 ? FX_ZERO : (emax == 2047 ? FX_NAN : K);
+}
+
+__global__ void __launch_bounds__(FX_THREADS) k_xinv_fx(GridDev g, FftPlan px, const fxtw* __restrict__ tw,
+                                                        const double2* __restrict__ W, double2* __restrict__ X, int czc) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  pdl_wait();  // launched with launch_pdl: the previous kernel's output is read from here on
+  const int ss = g.Nx + 1;
+  const int iz0 = blockIdx.z * czc, nc = min(czc, g.NKz - iz0);
+  const float invc = 1.0f / nc;
+  fxc* a = reinterpret_cast<fxc*>(smem_raw);
+  fxc* b = a + (size_t)czc * ss;
+  int* sK = reinterpret_cast<int*>(b + (size_t)czc * ss);
+  const int ny = blockIdx.x, c = blockIdx.y;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const double2* src = W + ((size_t)c * g.Ny + ny) * g.Md;
+  const int Kx = g.Kx, NKx = g.NKx, Nx = g.Nx;
+#pragma unroll 4
+  for (int i = tid; i < NKx * nc; i += FX_THREADS) {
+    int ix, jz;
+    divmod_small(i, nc, invc, ix, jz);
+    const double2 v = src[ix * g.NKz + iz0 + jz];
+    a[jz * ss + (ix <= Kx ? ix : Nx + ix - NKx)] = fxc{__double_as_longlong(v.x), __double_as_longlong(v.y)};
+  }
+  {
+    const int G = Nx - NKx;  // the unsolved wavenumbers
+    const float invg = 1.0f / G;
+    for (int i = tid; i < nc * G; i += FX_THREADS) {
+      int jz, p;
+      divmod_small(i, G, invg, jz, p);
+      a[jz * ss + Kx + 1 + p] = fxc{0, 0};
+    }
+  }
+  __syncthreads();
+  for (int jz = warp; jz < nc; jz += FX_THREADS / 32) {
+    const int K = fx_scale_column(a + jz * ss, NKx, [=](int i) { return i <= Kx ? i : Nx + i - NKx; }, lane);
+    if (lane == 0) sK[jz] = K;
+  }
+  __syncthreads();
+  const fxc* r = fx_fft(a, b, nc, ss, px, tw, +1, tid, FX_THREADS);
+  double2* dst = X + ((size_t)c * g.Ny + ny) * (size_t)Nx * g.NKz;
+  for (int i = tid; i < Nx * nc; i += FX_THREADS) {
+    int x, jz;
+    divmod_small(i, nc, invc, x, jz);
+    const fxc v = r[jz * ss + x];
+    const int K = sK[jz];
+    dst[x * g.NKz + iz0 + jz] = make_double2(fx_double(v.x, K), fx_double(v.y, K));
+  }
+}
+
+__global__ void __launch_bounds__(FX_THREADS) k_xfwd_fx(GridDev g, FftPlan px, const fxtw* __restrict__ tw,
+                                                        const double2* __restrict__ Z, double2* __restrict__ F,
+                                                        double scale, int czc) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  pdl_wait();  // launched with launch_pdl: the previous kernel's output is read from here on
+  const int ss = g.Nx + 1;
+  const int iz0 = blockIdx.z * czc, nc = min(czc, g.NKz - iz0);
+  const float invc = 1.0f / nc;
+  fxc* a = reinterpret_cast<fxc*>(smem_raw);
+  fxc* b = a + (size_t)czc * ss;
+  int* sK = reinterpret_cast<int*>(b + (size_t)czc * ss);
+  const int ny = blockIdx.x, c = blockIdx.y;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const double2* src = Z + ((size_t)c * g.Ny + ny) * (size_t)g.Nx * g.NKz;
+#pragma unroll 4
+  for (int i = tid; i < g.Nx * nc; i += FX_THREADS) {
+    int x, jz;
+    divmod_small(i, nc, invc, x, jz);
+    const double2 v = src[x * g.NKz + iz0 + jz];
+    a[jz * ss + x] = fxc{__double_as_longlong(v.x), __double_as_longlong(v.y)};
+  }
+  __syncthreads();
+  for (int jz = warp; jz < nc; jz += FX_THREADS / 32) {
+    const int K = fx_scale_column(a + jz * ss, g.Nx, [](int i) { return i; }, lane);
+    if (lane == 0) sK[jz] = K;
+  }
+  __syncthreads();
+  const fxc* r = fx_fft(a, b, nc, ss, px, tw, -1, tid, FX_THREADS);
+  double2* dst = F + ((size_t)c * g.Ny + ny) * g.Md;
+#pragma unroll 4
+  for (int i = tid; i < g.NKx * nc; i += FX_THREADS) {
+    int ix, jz;
+    divmod_small(i, nc, invc, ix, jz);
+    const fxc v = r[jz * ss + (ix <= g.Kx ? ix : g.Nx + ix - g.NKx)];
+    const int K = sK[jz];
+    dst[ix * g.NKz + iz0 + jz] = make_double2(fx_double(v.x, K) * scale, fx_double(v.y, K) * scale);
+  }
+}
+
+// ---------------------------------------------------------------------------
+// z pass.  Real sequence k of the block (row r = k / NC, component c = k % NC) is half of complex sequence k / 2.
+// ---------------------------------------------------------------------------
+template <int FORM>
+struct FxForm;
+template <>
+struct FxForm<NL_ROTATIONAL> { static constexpr int NC = 6, NO = 3; };
+template <>
+struct FxForm<NL_CONVECTION> { static constexpr int NC = 12, NO = 3; };
+template <>
+struct FxForm<NL_DIVERGENCE> { static constexpr int NC = 3, NO = 6; };
+template <>
+struct FxForm<NL_SKEW> { static constexpr int NC = 12, NO = 9; };
+
+// Products of the form: output o is the sum of its terms c[a] c[b] (sub: minus).
+struct FxTerm {
+  int a, b;
+  bool sub;
+};
+template <int FORM>
+__host__ __device__ constexpr int fx_nterm(int o) {
+  return FORM == NL_ROTATIONAL ? 2 : ((FORM == NL_CONVECTION || (FORM == NL_SKEW && o < 3)) ? 3 : 1);
+}
+template <int FORM>
+__host__ __device__ constexpr FxTerm fx_term(int o, int t) {
+  if (FORM == NL_ROTATIONAL) {  // omega x u, c = u, v, w, ox, oy, oz
+    const int j = (o + 1) % 3, k = (o + 2) % 3;
+    return t == 0 ? FxTerm{3 + j, k, false} : FxTerm{3 + k, j, true};
+  }
+  if (FORM == NL_CONVECTION || (FORM == NL_SKEW && o < 3)) return FxTerm{t, 3 + 3 * o + t, false};  // u_j d u_o / d x_j
+  const int q = FORM == NL_SKEW ? o - 3 : o;  // uu, uv, uw, vv, vw, ww
+  return FxTerm{q < 3 ? 0 : (q < 5 ? 1 : 2), q < 3 ? q : (q < 5 ? q - 2 : 2), false};
+}
+
+__device__ __forceinline__ unsigned fx_absbits(long long v) {
+  const int h = (int)(v >> 32);
+  return (unsigned)(h ^ (h >> 31));
+}
+__device__ __forceinline__ long long fx_round_shift(long long v, int s) {  // v 2^s
+  return s >= 0 ? v << s : ((v >> (min(-s, 63) - 1)) + 1) >> 1;
+}
+
+template <int FORM>
+__global__ void __launch_bounds__(FX_THREADS) k_zphys_fx(GridDev g, FftPlan pz, const fxtw* __restrict__ tw, int RP,
+                                                         const double2* __restrict__ X, double2* __restrict__ Z) {
+  constexpr int NC = FxForm<FORM>::NC, NO = FxForm<FORM>::NO;
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  pdl_wait();  // launched with launch_pdl: the previous kernel's output is read from here on
+  const int Nz = g.Nz, ss = Nz + 1, NKz = g.NKz;
+  const int nseq = ((NC > NO ? NC : NO) * RP) / 2;
+  const int ninv = NC * RP / 2, nfwd = NO * RP / 2;
+  fxc* A = reinterpret_cast<fxc*>(smem_raw);
+  fxc* B = A + (size_t)nseq * ss;
+  int* sK = reinterpret_cast<int*>(B + (size_t)nseq * ss);  // exponent K of every component's row (normalised)
+  int* sN = sK + 2 * nseq;                                  // left shift that normalises it
+  int* sF = sN + 2 * nseq;                                  // exponent K of every output's row
+  const int ny = blockIdx.y, x0 = blockIdx.x * RP;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const size_t plane = (size_t)g.Nx * NKz;
+  const float invk = 1.0f / NKz;
+  {
+    // the pack below writes bins 0..NKz-1 and Nz-NKz+1..Nz-1 of every inverse sequence: zero the gap
+    const int G = Nz - 2 * NKz + 1;
+    const float invg = 1.0f / G;
+    for (int i = tid; i < ninv * G; i += FX_THREADS) {
+      int sq, z;
+      divmod_small(i, G, invg, sq, z);
+      A[(size_t)sq * ss + NKz + z] = fxc{0, 0};
+    }
+  }
+  // raw doubles of the two rows a, b of a sequence: bin iz holds a's coefficient, bin Nz - iz b's, bin 0 both
+#pragma unroll 4
+  for (int i = tid; i < ninv * NKz; i += FX_THREADS) {
+    int s, iz;
+    divmod_small(i, NKz, invk, s, iz);
+    const int k0 = 2 * s, k1 = 2 * s + 1;
+    const int r0 = k0 / NC, c0 = k0 % NC, r1 = k1 / NC, c1 = k1 % NC;
+    double2 ca = make_double2(0, 0), cb = make_double2(0, 0);
+    if (x0 + r0 < g.Nx) ca = X[((size_t)c0 * g.Ny + ny) * plane + (size_t)(x0 + r0) * NKz + iz];
+    if (x0 + r1 < g.Nx) cb = X[((size_t)c1 * g.Ny + ny) * plane + (size_t)(x0 + r1) * NKz + iz];
+    fxc* sq = A + (size_t)s * ss;
+    if (iz == 0) {
+      sq[0] = fxc{__double_as_longlong(ca.x), __double_as_longlong(cb.x)};
+    } else {
+      sq[iz] = fxc{__double_as_longlong(ca.x), __double_as_longlong(ca.y)};
+      sq[Nz - iz] = fxc{__double_as_longlong(cb.x), __double_as_longlong(cb.y)};
+    }
+  }
+  __syncthreads();
+  for (int s = warp; s < ninv; s += FX_THREADS / 32) {
+    fxc* sq = A + (size_t)s * ss;
+    unsigned ka = 0, kb = 0;
+    for (int iz = lane; iz < NKz; iz += 32) {
+      const fxc p = sq[iz];
+      if (iz == 0) {
+        ka = fx_key(fx_raw(p.x));
+        kb = fx_key(fx_raw(p.y));
+      } else {
+        const fxc q = sq[Nz - iz];
+        ka = max(ka, max(fx_key(fx_raw(p.x)), fx_key(fx_raw(p.y))));
+        kb = max(kb, max(fx_key(fx_raw(q.x)), fx_key(fx_raw(q.y))));
+      }
+    }
+    ka = __reduce_max_sync(0xffffffffu, ka);
+    kb = __reduce_max_sync(0xffffffffu, kb);
+    const int ea = fx_exp_of_key(ka), eb = fx_exp_of_key(kb);
+    unsigned Sa = 0, Sb = 0;  // every coefficient but the mean appears twice in the sequence
+    for (int iz = lane; iz < NKz; iz += 32) {
+      const fxc p = sq[iz];
+      if (iz == 0) {
+        Sa = fx_mag(fx_raw(p.x), ea);
+        Sb = fx_mag(fx_raw(p.y), eb);
+      } else {
+        const fxc q = sq[Nz - iz];
+        Sa += 2 * (fx_mag(fx_raw(p.x), ea) + fx_mag(fx_raw(p.y), ea));
+        Sb += 2 * (fx_mag(fx_raw(q.x), eb) + fx_mag(fx_raw(q.y), eb));
+      }
+    }
+    Sa = __reduce_add_sync(0xffffffffu, Sa);
+    Sb = __reduce_add_sync(0xffffffffu, Sb);
+    const int Ka = fx_line_K(ea, Sa, 60), Kb = fx_line_K(eb, Sb, 60);
+    for (int iz = lane; iz < NKz; iz += 32) {
+      const fxc p = sq[iz];
+      if (iz == 0) {
+        sq[0] = fxc{ka ? fx_quant(fx_raw(p.x), Ka) : 0, kb ? fx_quant(fx_raw(p.y), Kb) : 0};
+      } else {
+        const fxc q = sq[Nz - iz];
+        const long long ax = ka ? fx_quant(fx_raw(p.x), Ka) : 0, ay = ka ? fx_quant(fx_raw(p.y), Ka) : 0;
+        const long long bx = kb ? fx_quant(fx_raw(q.x), Kb) : 0, by = kb ? fx_quant(fx_raw(q.y), Kb) : 0;
+        sq[iz] = fxc{ax - by, ay + bx};       // A_k + i B_k
+        sq[Nz - iz] = fxc{ax + by, bx - ay};  // conj(A_k) + i conj(B_k)
+      }
+    }
+    if (lane == 0) {
+      sK[2 * s] = ka == 0 ? FX_ZERO : (ea == 2047 ? FX_NAN : Ka);
+      sK[2 * s + 1] = kb == 0 ? FX_ZERO : (eb == 2047 ? FX_NAN : Kb);
+    }
+  }
+  __syncthreads();
+  fxc* P = fx_fft(A, B, ninv, ss, pz, tw, +1, tid, FX_THREADS);
+  fxc* Q = P == A ? B : A;
+  // normalise every component by its largest value: the scale above allows for the sum of magnitudes
+  for (int s = warp; s < ninv; s += FX_THREADS / 32) {
+    const fxc* sq = P + (size_t)s * ss;
+    unsigned mx = 0, my = 0;
+    for (int z = lane; z < Nz; z += 32) {
+      const fxc v = sq[z];
+      mx |= fx_absbits(v.x);
+      my |= fx_absbits(v.y);
+    }
+    mx = __reduce_or_sync(0xffffffffu, mx);
+    my = __reduce_or_sync(0xffffffffu, my);
+    if (lane < 2) {
+      const int n = max(__clz(lane == 0 ? mx : my) - 3, 0);  // |v| < 2^61 after the shift
+      sN[2 * s + lane] = n;
+      sK[2 * s + lane] += n;
+    }
+  }
+  __syncthreads();
+  for (int i = tid; i < RP * Nz; i += FX_THREADS) {
+    const int r = i / Nz, z = i - r * Nz;
+    long long c[NC];
+#pragma unroll
+    for (int q = 0; q < NC; ++q) {
+      const int k = r * NC + q;
+      const fxc* v = P + (size_t)(k >> 1) * ss + z;
+      c[q] = ((k & 1) ? v->y : v->x) << sN[k];
+    }
+    const int* Kr = sK + r * NC;
+#pragma unroll
+    for (int o = 0; o < NO; ++o) {
+      constexpr int MT = 3;
+      int kt[MT], km = INT32_MAX;
+#pragma unroll
+      for (int t = 0; t < MT; ++t)
+        if (t < fx_nterm<FORM>(o)) {
+          kt[t] = Kr[fx_term<FORM>(o, t).a] + Kr[fx_term<FORM>(o, t).b];
+          km = min(km, kt[t]);
+        }
+      long long f = 0;
+#pragma unroll
+      for (int t = 0; t < MT; ++t)
+        if (t < fx_nterm<FORM>(o)) {
+          const long long p = __mul64hi(c[fx_term<FORM>(o, t).a], c[fx_term<FORM>(o, t).b]) >> min(kt[t] - km, 63);
+          f = fx_term<FORM>(o, t).sub ? f - p : f + p;
+        }
+      const int k = r * NO + o;
+      long long* q = reinterpret_cast<long long*>(Q + (size_t)(k >> 1) * ss + z);
+      q[k & 1] = f;
+      if (z == 0) sF[k] = km - 64;
+    }
+  }
+  __syncthreads();
+  // scale every output row to the sum of its magnitudes (2^60 per half)
+  for (int s = warp; s < nfwd; s += FX_THREADS / 32) {
+    fxc* sq = Q + (size_t)s * ss;
+    unsigned Sx = 0, Sy = 0;
+    for (int z = lane; z < Nz; z += 32) {
+      const fxc v = sq[z];
+      Sx += (fx_absbits(v.x) >> 8) + 1;  // units 2^40
+      Sy += (fx_absbits(v.y) >> 8) + 1;
+    }
+    Sx = __reduce_add_sync(0xffffffffu, Sx);
+    Sy = __reduce_add_sync(0xffffffffu, Sy);
+    const int sx = 20 - (32 - __clz(Sx)), sy = 20 - (32 - __clz(Sy));
+    for (int z = lane; z < Nz; z += 32) {
+      const fxc v = sq[z];
+      sq[z] = fxc{fx_round_shift(v.x, sx), fx_round_shift(v.y, sy)};
+    }
+    if (lane == 0) {
+      sF[2 * s] += sx;
+      sF[2 * s + 1] += sy;
+    }
+  }
+  __syncthreads();
+  const fxc* G = fx_fft(Q, P, nfwd, ss, pz, tw, -1, tid, FX_THREADS);
+#pragma unroll 2
+  for (int i = tid; i < nfwd * NKz; i += FX_THREADS) {
+    int s, iz;
+    divmod_small(i, NKz, invk, s, iz);
+    const fxc* sq = G + (size_t)s * ss;
+    const fxc zk = sq[iz], zm = sq[iz == 0 ? 0 : Nz - iz];
+    const int k0 = 2 * s, k1 = 2 * s + 1;
+    const int r0 = k0 / NO, o0 = k0 % NO, r1 = k1 / NO, o1 = k1 % NO;
+    const int K0 = sF[k0] + 1, K1 = sF[k1] + 1;  // + 1: half the sum
+    if (x0 + r0 < g.Nx)
+      Z[((size_t)o0 * g.Ny + ny) * plane + (size_t)(x0 + r0) * NKz + iz] =
+          make_double2(fx_double(zk.x + zm.x, K0), fx_double(zk.y - zm.y, K0));
+    if (x0 + r1 < g.Nx)
+      Z[((size_t)o1 * g.Ny + ny) * plane + (size_t)(x0 + r1) * NKz + iz] =
+          make_double2(fx_double(zk.y + zm.y, K1), fx_double(zm.x - zk.x, K1));
+  }
+}
+
+template <int FORM>
+cudaError_t run_zphys_fx(const GridDev& g, const FftPlan& pz, const fxtw* tw, int RP, const double2* X, double2* Z,
+                         cudaStream_t st) {
+  static const bool attr = [] {
+    cudaFuncSetAttribute(k_zphys_fx<FORM>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
+    return true;
+  }();
+  (void)attr;
+  return launch_pdl(k_zphys_fx<FORM>, dim3((g.Nx + RP - 1) / RP, g.Ny), dim3(FX_THREADS),
+                    zphys_smem_bytes<double>(g, FORM, RP), st, g, pz, tw, RP, X, Z);
+}
+
+size_t xfx_smem(const GridDev& g, int czc) { return xfft_smem_bytes<double>(g, czc) + sizeof(int) * czc; }
+
+}  // namespace
+
+std::vector<int> fx_twiddles(const std::vector<std::complex<long double>>& tw) {
+  std::vector<int> t(4 * (tw.empty() ? 1 : tw.size()), 0);
+  for (size_t i = 0; i < tw.size(); ++i) {
+    fx_split(tw[i].real(), t[4 * i], t[4 * i + 1]);
+    fx_split(tw[i].imag(), t[4 * i + 2], t[4 * i + 3]);
+  }
+  return t;
+}
+
+cudaError_t launch_xinv_fx(const GridDev& g, const FftPlan& px, const void* tw, const cpx<double>* W, cpx<double>* X,
+                           int ncomp, int czc, cudaStream_t st) {
+  static const bool attr = [] {
+    cudaFuncSetAttribute(k_xinv_fx, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
+    return true;
+  }();
+  (void)attr;
+  return launch_pdl(k_xinv_fx, dim3(g.Ny, ncomp, (g.NKz + czc - 1) / czc), dim3(FX_THREADS), xfx_smem(g, czc), st, g, px,
+                    (const fxtw*)tw, (const double2*)W, (double2*)X, czc);
+}
+
+cudaError_t launch_xfwd_fx(const GridDev& g, const FftPlan& px, const void* tw, const cpx<double>* Z, cpx<double>* F,
+                           int ncomp, int czc, cudaStream_t st) {
+  static const bool attr = [] {
+    cudaFuncSetAttribute(k_xfwd_fx, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
+    return true;
+  }();
+  (void)attr;
+  const double scale = 1.0 / ((double)g.Nx * (double)g.Nz);
+  return launch_pdl(k_xfwd_fx, dim3(g.Ny, ncomp, (g.NKz + czc - 1) / czc), dim3(FX_THREADS), xfx_smem(g, czc), st, g, px,
+                    (const fxtw*)tw, (const double2*)Z, (double2*)F, scale, czc);
+}
+
+cudaError_t launch_zphys_fx(const GridDev& g, int form, const FftPlan& pz, const void* tw, int RP, const cpx<double>* X,
+                            cpx<double>* Z, cudaStream_t st) {
+  const fxtw* t = (const fxtw*)tw;
+  const double2* x = (const double2*)X;
+  double2* z = (double2*)Z;
+  if (RP < 2 || RP % 2) return cudaErrorInvalidValue;  // whole pairs of output rows
+  switch (form) {
+    case NL_ROTATIONAL: return run_zphys_fx<NL_ROTATIONAL>(g, pz, t, RP, x, z, st);
+    case NL_CONVECTION: return run_zphys_fx<NL_CONVECTION>(g, pz, t, RP, x, z, st);
+    case NL_DIVERGENCE: return run_zphys_fx<NL_DIVERGENCE>(g, pz, t, RP, x, z, st);
+    case NL_SKEW: return run_zphys_fx<NL_SKEW>(g, pz, t, RP, x, z, st);
+    default: return cudaErrorInvalidValue;
+  }
+}

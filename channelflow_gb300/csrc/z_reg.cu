@@ -13,8 +13,8 @@
 // thread transforms 8 or N1 points in registers, so a transform costs two shared-memory round trips, against
 // one per radix stage for the generic Stockham FFT; sequences are padded by one slot per N1 points.  Twiddles:
 // the full-circle table exp(-2 pi i e / Nz), e < Nz, in the field's dithered version on the mixed path.  One
-// CTA takes RC x rows of one plane (the DNS's tuned z-pass row count).  FP32 (mixed path) only: in FP64 the
-// Stockham kernel's radix-4 stages take fewer FP64-pipe slots and were faster.
+// CTA takes RC x rows of one plane (the DNS's tuned z-pass row count).  FP32 (mixed path) only: the
+// FP64 path's z pass runs on integers (xz_fx.cu).
 #include "fft_steps.cuh"
 #include "kernels.h"
 
