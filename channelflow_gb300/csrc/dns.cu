@@ -623,6 +623,10 @@ struct cfgpu_dns_s {
   FftPlan px{}, pz{};
   void *twx = nullptr, *twz = nullptr;  // R-typed complex
   void *twxq = nullptr, *twzq = nullptr;  // FP64: the same as fixed-point splits (fx_twiddles)
+  // FP64 Chebyshev transforms on the tensor cores (cheb_oz.cu): tables in one block, off where Ny is not covered
+  bool oz = false;
+  OzTables ozt{};
+  void* ozblock = nullptr;
   // fused x/z pass (rotational form): full-circle twiddle tables exp(-2 pi i e/L), cluster shape
   void *twxf = nullptr, *twzf = nullptr;
   bool xzf = false;
@@ -792,6 +796,77 @@ Dither dither_of(cfgpu_dns d) {
   return dt;
 }
 
+// FP64 Chebyshev transforms on the tensor cores (d->oz).
+int oz_run(cfgpu_dns d, bool inverse, const OzJob* jobs, int n) {
+  CK(launch_cheb_oz(d->gm, d->N, inverse, (int)d->rowc(), d->rowc(), d->ozt, jobs, n, d->dtcerr, d->st));
+  d->launches++;
+  return CFGPU_OK;
+}
+
+// Component c of U, with the base flow unless bare, at the Gauss-Lobatto points (or its d/dy).
+OzJob oz_component(cfgpu_dns d, const double* U, double* W, int c, int slot, bool deriv, bool bare, double Vsuck) {
+  OzJob j{};
+  j.in = U + c * d->compc();
+  j.out = W + slot * d->compc();
+  j.deriv = deriv;
+  if (bare) return j;
+  if (c != 1) {
+    j.base = d->hetero ? d->dbaseS + (c == 2 ? (size_t)d->nb * d->N : 0) : (c == 2 ? d->dWbase : d->dUbase);
+    j.bstride = d->hetero ? d->N : 0;
+  } else if (!deriv) {
+    j.shift = Vsuck;
+  }
+  return j;
+}
+
+// W = u, v, w, dw/dy, -, du/dy at the Gauss-Lobatto points (the x pass forms the curl).
+int oz_curl(cfgpu_dns d, const double* U, double* W, double Vsuck) {
+  const OzJob j[5] = {oz_component(d, U, W, 0, 0, false, false, Vsuck), oz_component(d, U, W, 1, 1, false, false, Vsuck),
+                      oz_component(d, U, W, 2, 2, false, false, Vsuck), oz_component(d, U, W, 2, 3, true, false, Vsuck),
+                      oz_component(d, U, W, 0, 5, true, false, Vsuck)};
+  return oz_run(d, true, j, 5);
+}
+
+// W = u, v, w and, with gradient, the nine derivatives d u_i / d x_j at the Gauss-Lobatto points.
+int oz_grad(cfgpu_dns d, const double* U, double* W, bool gradient, bool bare, double Vsuck) {
+  OzJob j[6];
+  for (int c = 0; c < 3; ++c) {
+    j[c] = oz_component(d, U, W, c, c, false, bare, Vsuck);
+    if (gradient) {
+      j[c].gx = W + (3 + 3 * c) * d->compc();
+      j[c].gz = W + (5 + 3 * c) * d->compc();
+      j[3 + c] = oz_component(d, U, W, c, 4 + 3 * c, true, bare, Vsuck);
+    }
+  }
+  return oz_run(d, true, j, gradient ? 6 : 3);
+}
+
+int oz_forward(cfgpu_dns d, const double* in, double* out) {
+  OzJob j[3] = {};
+  for (int c = 0; c < 3; ++c) {
+    j[c].in = in + c * d->compc();
+    j[c].out = out + c * d->compc();
+  }
+  return oz_run(d, false, j, 3);
+}
+
+// out_i = F (w conv_i + w d/dx p_i0 + w d/dz p_i2) + w DF p_i1 of the products p_ij (uu, uv, uw, vv, vw, ww)
+int oz_divergence(cfgpu_dns d, const double* conv, const double* p, double w, double* out) {
+  const int pij[3][3] = {{0, 1, 2}, {1, 3, 4}, {2, 4, 5}};
+  const size_t comp = d->compc();
+  OzJob j[3] = {};
+  for (int i = 0; i < 3; ++i) {
+    j[i].in = conv ? conv + i * comp : nullptr;
+    j[i].out = out + i * comp;
+    j[i].pkx = p + pij[i][0] * comp;
+    j[i].pkz = p + pij[i][2] * comp;
+    j[i].pd = p + pij[i][1] * comp;
+    j[i].wF = j[i].wK = w;
+    j[i].wD = w * 2.0 / (d->gm.b - d->gm.a);
+  }
+  return oz_run(d, false, j, 3);
+}
+
 // Nonlinear term N(u) of the fields in U (solved-mode layout) into Nout (R-typed):
 // navierstokesNL (nse.cpp:12-91) for the form selected by the flags; `which`
 // selects the NSE (0 main, 1 init) whose Alternating state is advanced.
@@ -804,6 +879,7 @@ int nonlinear_impl(cfgpu_dns d, const double* U, void* Nout, int form) {
   R* W = (R*)d->W6;
   const size_t row = d->rowc(), comp = d->compc();
   int nin = 6, nout = 3;
+  bool curl = false;  // the x pass forms the vorticity (FP64)
   const void* by = d->hetero ? d->baseyS : d->basey;
   const int bstride = d->hetero ? 4 * N : 0;
   const Dither dt = dither_of(d);
@@ -812,6 +888,12 @@ int nonlinear_impl(cfgpu_dns d, const double* U, void* Nout, int form) {
   if (form == CFGPU_LinearAboutProfile) {
     // linearizedNL: u, v, w at the points (no base flow), (U d/dx + W d/dz) u + v (U', 0, W'), forward y
     if ((N + 1) / 2 > 56) return fail(CFGPU_ENOTSUP, "Ny > 111 with LinearAboutProfile");
+    if constexpr (sizeof(R) == 8) {
+      CKS(oz_grad(d, U, W, false, true, 0.0));
+      CK(launch_linprof<R>(g, N, W, (const R*)by, bstride, (R*)d->F3, d->st, dt));
+      d->launches += 1;
+      return oz_forward(d, (const double*)d->F3, (double*)Nout);
+    } else {
     CK(launch_grad_cheb<R>(g, N, false, U, W, (const R*)d->cinvA, (const R*)d->cinvB, (const R*)d->cderA,
                            (const R*)d->cderB, (const R*)d->zbasey, 0.0, d->st, bstride, dt0));
     CK(launch_linprof<R>(g, N, W, (const R*)by, bstride, (R*)d->F3, d->st, dt));
@@ -819,6 +901,7 @@ int nonlinear_impl(cfgpu_dns d, const double* U, void* Nout, int form) {
                              (const R*)d->cfwdA, (const R*)d->cfwdB, d->st, dt)));
     d->launches += 3;
     return CFGPU_OK;
+    }
   }
   const double* bU = d->hetero ? d->dbaseS : d->dUbase;
   const double* bW = d->hetero ? d->dbaseS + (size_t)d->nb * N : d->dWbase;
@@ -829,12 +912,26 @@ int nonlinear_impl(cfgpu_dns d, const double* U, void* Nout, int form) {
                      (const cpx<R>*)d->cdct, d->st, dt));
     d->launches += 2;
   } else if (form == NL_ROTATIONAL) {
-    if ((N + 1) / 2 <= 56) {
+    bool done = false;
+    if constexpr (sizeof(R) == 8) {
+      if (d->oz) {
+        CKS(oz_curl(d, U, W, d->fl.Vsuck));
+        done = true;
+        if (d->xzf) {
+          CK(launch_curl_points(gp, (cpx<double>*)W, d->st));
+          d->launches += 1;
+        } else {
+          curl = true;
+        }
+      }
+    } else if ((N + 1) / 2 <= 56) {
+      done = true;
       CK(launch_curl_cheb<R>(g, N, U, W, (const R*)d->cinvA, (const R*)d->cinvB, (const R*)d->cderA,
                              (const R*)d->cderB, (const R*)(d->hetero ? d->baseyS : d->basey), d->fl.Vsuck, d->st,
                              d->hetero ? 4 * N : 0, dt));
       d->launches += 1;
-    } else {
+    }
+    if (!done) {
       CK(launch_curl_base<R>(g, U, C6, bU, bW, d->hetero ? N : 0, d->fl.Vsuck, d->st));
       CK((launch_cheb<R, R, R>(N, true, (int)row, 6, C6, row, comp, W, row, comp, (const R*)d->cinvA,
                                (const R*)d->cinvB, d->st, dt)));
@@ -843,10 +940,14 @@ int nonlinear_impl(cfgpu_dns d, const double* U, void* Nout, int form) {
   } else {
     if ((N + 1) / 2 > 56) return fail(CFGPU_ENOTSUP, "Ny > 111 with a gradient nonlinear form");
     const bool gradient = form != NL_DIVERGENCE;
-    CK(launch_grad_cheb<R>(g, N, gradient, U, W, (const R*)d->cinvA, (const R*)d->cinvB, (const R*)d->cderA,
-                           (const R*)d->cderB, (const R*)(d->hetero ? d->baseyS : d->basey), d->fl.Vsuck, d->st,
-                           d->hetero ? 4 * N : 0, dt));
-    d->launches += 1;
+    if constexpr (sizeof(R) == 8) {
+      CKS(oz_grad(d, U, W, gradient, false, d->fl.Vsuck));
+    } else {
+      CK(launch_grad_cheb<R>(g, N, gradient, U, W, (const R*)d->cinvA, (const R*)d->cinvB, (const R*)d->cderA,
+                             (const R*)d->cderB, (const R*)(d->hetero ? d->baseyS : d->basey), d->fl.Vsuck, d->st,
+                             d->hetero ? 4 * N : 0, dt));
+      d->launches += 1;
+    }
     nin = gradient ? 12 : 3;
     nout = form == NL_CONVECTION ? 3 : (form == NL_DIVERGENCE ? 6 : 9);
   }
@@ -856,7 +957,7 @@ int nonlinear_impl(cfgpu_dns d, const double* U, void* Nout, int form) {
     d->launches += 1;
   } else {
     CK(launch_xinv<R>(gp, d->px, (const cpx<R>*)d->twx, d->twxq, (const cpx<R>*)W, (cpx<R>*)d->X6, nin, d->st, d->xcols,
-                      dt));
+                      dt, curl));
     CK(launch_zphys<R>(gp, form, d->pz, (const cpx<R>*)d->twz, d->twzq, d->RP, (const cpx<R>*)d->X6, (cpx<R>*)d->Z3, d->st,
                        dt, (const cpx<R>*)d->twzf));
     CK(launch_xfwd<R>(gp, d->px, (const cpx<R>*)d->twx, d->twxq, (const cpx<R>*)d->Z3, (cpx<R>*)d->F3, nout, d->st,
@@ -871,6 +972,13 @@ int nonlinear_impl(cfgpu_dns d, const double* U, void* Nout, int form) {
       return CFGPU_OK;
     }
   }
+  if constexpr (sizeof(R) == 8) {
+    if (form == NL_CONVECTION || (form == NL_ROTATIONAL && d->oz && !d->ydct))
+      return oz_forward(d, (const double*)F, (double*)Nout);
+    if (form != NL_ROTATIONAL)
+      return oz_divergence(d, form == NL_SKEW ? (const double*)F : nullptr,
+                           (const double*)(form == NL_SKEW ? F + 3 * comp : F), form == NL_SKEW ? 0.5 : 1.0, (double*)Nout);
+  }
   if (form == NL_ROTATIONAL && d->ydct) {
     CK(launch_dct<R>(N, false, g.Md, 3, (const cpx<R>*)F, row / 2, comp / 2, (cpx<R>*)Nout, row / 2, comp / 2,
                      (const cpx<R>*)d->cdct, d->st, dt));
@@ -879,7 +987,7 @@ int nonlinear_impl(cfgpu_dns d, const double* U, void* Nout, int form) {
     CK((launch_cheb<R, R, R>(N, false, (int)row, 3, F, row, comp, (R*)Nout, row, comp, (const R*)d->cfwdA,
                              (const R*)d->cfwdB, d->st, dt)));
     d->launches += 1;
-  } else {
+  } else if constexpr (sizeof(R) == 4) {
     // products p_ij (ij = uu, uv, uw, vv, vw, ww) follow the convection term for the skew form
     const R* p = form == NL_SKEW ? F + 3 * comp : F;
     const int pij[3][3] = {{0, 1, 2}, {1, 3, 4}, {2, 4, 5}};
@@ -1433,6 +1541,31 @@ int upload_ints(const std::vector<int>& t, void** dst, long long& bytes, cudaStr
   return CFGPU_OK;
 }
 
+// Tables of the FP64 Chebyshev transforms (cheb_oz.cu), the derivative's only for the forms with a divergence.
+int oz_upload(cfgpu_dns d, bool with_df) {
+  const int N = d->N, nm = with_df ? 3 : 2;
+  const size_t mb = oz_matrix_bytes(N), rb = 2 * 4 * (size_t)((((N + 1) / 2) + 7) & ~7);
+  std::vector<unsigned char> h((mb + rb) * nm);
+  for (int k = 0; k < nm; ++k) {
+    std::vector<uint16_t> dg;
+    std::vector<int> re;
+    if (!oz_matrix(N, k, dg, re)) return CFGPU_OK;
+    std::memcpy(h.data() + k * mb, dg.data(), mb);
+    std::memcpy(h.data() + nm * mb + k * rb, re.data(), rb);
+  }
+  unsigned char* p;
+  CKS(dalloc(&p, h.size(), d->bytes));
+  d->ozblock = p;
+  CK(cudaMemcpyAsync(p, h.data(), h.size(), cudaMemcpyHostToDevice, d->st));
+  CKS(dalloc(&d->dtcerr, 1, d->bytes));
+  CK(cudaMemsetAsync(d->dtcerr, 0, sizeof(int), d->st));
+  OzMatrix* m[3] = {&d->ozt.T, &d->ozt.F, &d->ozt.DF};
+  for (int k = 0; k < nm; ++k) *m[k] = OzMatrix{p + k * mb, (const int*)(p + nm * mb + k * rb)};
+  d->ozt.N = N;
+  d->oz = true;
+  return CFGPU_OK;
+}
+
 template <typename R>
 int upload_tw(const std::vector<std::complex<long double>>& tw, void** dst, long long& bytes, cudaStream_t st) {
   std::vector<cpx<R>> t(tw.size() ? tw.size() : 1);
@@ -1557,8 +1690,12 @@ int tune_xz(cfgpu_dns d) {
       return CFGPU_OK;
     }
   }
-  const std::vector<XzShape> cand = xz_fused_candidates(gp, sizeof(R) == 8);
   d->xzC = d->xzRC = 0;
+  d->xzf = false;
+  // FP64: the three kernels run on integers and are the faster form (32x35x32: 20 us, fused 21.5; at 128x97x128 the
+  // fused kernel was behind them even in FP64 arithmetic), the fused kernel only when it is asked for
+  if (sizeof(R) == 8 && g_fused_xz.load() != 2) return CFGPU_OK;
+  const std::vector<XzShape> cand = xz_fused_candidates(gp, sizeof(R) == 8);
   if (!cand.empty()) {
     d->xzC = cand[0].C;
     d->xzRC = cand[0].RC;
@@ -1608,6 +1745,7 @@ int tune_cheb(cfgpu_dns d) {
   d->ydct = false;
   const int mode = g_cheb_fft.load();
   if (mode == 0 || !d->cdct || !dct_supported(d->N)) return CFGPU_OK;
+  if (sizeof(R) == 8 && d->oz && mode == 1) return CFGPU_OK;  // FP64 matrix products on the tensor cores
   if (mode == 2) {
     d->ydct = true;
     return CFGPU_OK;
@@ -1630,11 +1768,13 @@ int tune_cheb(cfgpu_dns d) {
   R* C6 = (R*)d->C6;
   R* W = (R*)d->W6;
   const float tdense = time_ms<R>(d, [&]() {
-    cudaError_t e;
-    if ((N + 1) / 2 <= 56) {
-      e = launch_curl_cheb<R>(g, N, d->Ucur, W, (const R*)d->cinvA, (const R*)d->cinvB, (const R*)d->cderA,
-                              (const R*)d->cderB, (const R*)d->basey, 0.0, d->st);
-    } else {
+    cudaError_t e = cudaErrorNotSupported;
+    if constexpr (sizeof(R) == 4) {
+      if ((N + 1) / 2 <= 56)
+        e = launch_curl_cheb<R>(g, N, d->Ucur, W, (const R*)d->cinvA, (const R*)d->cinvB, (const R*)d->cderA,
+                                (const R*)d->cderB, (const R*)d->basey, 0.0, d->st);
+    }
+    if (e == cudaErrorNotSupported) {
       e = launch_curl_base<R>(g, d->Ucur, C6, d->dUbase, d->dWbase, 0, 0.0, d->st);
       if (e == cudaSuccess)
         e = launch_cheb<R, R, R>(N, true, nl1, 6, C6, row, comp, W, row, comp, (const R*)d->cinvA,
@@ -1864,6 +2004,7 @@ int dns_create_impl(cfgpu_dns d, const cfgpu_grid* grid, const cfgpu_flags* flag
     CKS(upload_as<double>(cm.dfA, &d->cdfA, B, d->st));
     CKS(upload_as<double>(cm.dfB, &d->cdfB, B, d->st));
     if (dct_supported(Ny)) CKS(upload_as<double>(dct_table(Ny), &d->cdct, B, d->st));
+    CKS(oz_upload(d, f.nonlinearity != CFGPU_Rotational && f.nonlinearity != CFGPU_Convection));
   } else {
     // DITHER_V dithered versions of every FP32 constant table in one block (16-byte aligned tables)
     std::vector<std::vector<double>> tabs = {cm.invA, cm.invB, cm.fwdA, cm.fwdB, cm.derA, cm.derB, cm.dfA, cm.dfB};
@@ -2046,7 +2187,7 @@ void dns_free(cfgpu_dns d) {
     d->twx = d->twz = d->cinvA = d->cinvB = d->cfwdA = d->cfwdB = d->cderA = d->cderB = d->cdfA = d->cdfB = nullptr;
     d->twxf = d->twzf = d->cdct = nullptr;
   }
-  F(d->twxf); F(d->twzf); F(d->cdct); F(d->ctc); F(d->dtcerr);
+  F(d->twxf); F(d->twzf); F(d->cdct); F(d->ctc); F(d->dtcerr); F(d->ozblock);
   F(d->dUbase); F(d->dWbase); F(d->dUbaseyy); F(d->dWbaseyy); F(d->ddPdx);
   F(d->hb_lo); F(d->hb_di); F(d->hb_up);
   F(d->twx); F(d->twz); F(d->twxq); F(d->twzq); F(d->cinvA); F(d->cinvB); F(d->cfwdA); F(d->cfwdB);
@@ -2081,7 +2222,19 @@ template <typename R>
 int cfl_enqueue(cfgpu_dns d) {
   const GridDev& g = d->gm;
   R* W = (R*)d->W6;
-  if ((d->N + 1) / 2 > 56 || d->ydct) {
+  bool done = false;
+  if constexpr (sizeof(R) == 8) {
+    if (d->oz && !d->ydct) {
+      CKS(oz_grad(d, d->Ucur, W, false, false, 0.0));
+      done = true;
+    }
+  } else if ((d->N + 1) / 2 <= 56 && !d->ydct) {
+    CK(launch_grad_cheb<R>(g, d->N, false, d->Ucur, W, (const R*)d->cinvA, (const R*)d->cinvB, (const R*)d->cderA,
+                           (const R*)d->cderB, (const R*)(d->hetero ? d->baseyS : d->basey), 0.0, d->st,
+                           d->hetero ? 4 * d->N : 0));
+    done = true;
+  }
+  if (!done) {
     // tall grids, or transforms through the FFT: u + base flow as Chebyshev coefficients (the curl pass's
     // first three components), then the inverse transform to the Gauss-Lobatto points
     const size_t row = d->rowc(), comp = d->compc(), nN = (size_t)d->nb * d->N;
@@ -2094,10 +2247,6 @@ int cfl_enqueue(cfgpu_dns d) {
       CK((launch_cheb<R, R, R>(d->N, true, (int)row, 3, (const R*)d->C6, row, comp, W, row, comp,
                                (const R*)d->cinvA, (const R*)d->cinvB, d->st)));
     d->launches += 2;
-  } else {
-    CK(launch_grad_cheb<R>(g, d->N, false, d->Ucur, W, (const R*)d->cinvA, (const R*)d->cinvB, (const R*)d->cderA,
-                           (const R*)d->cderB, (const R*)(d->hetero ? d->baseyS : d->basey), 0.0, d->st,
-                           d->hetero ? 4 * d->N : 0));
   }
   CK(launch_xinv<R>(d->gp, d->px, (const cpx<R>*)d->twx, d->twxq, (const cpx<R>*)W, (cpx<R>*)d->X6, 3, d->st, d->xcols));
   CK(cudaMemsetAsync(d->dred, 0, d->nb * sizeof(unsigned long long), d->st));

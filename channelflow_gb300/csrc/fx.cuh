@@ -251,7 +251,7 @@ __device__ __forceinline__ unsigned fx_mag(double x, int emax) {
 // K of a line (value = v 2^-K) from its magnitude sum S > 0 (units 2^(emax - 1039)): the magnitudes of its integers
 // sum to less than 2^lim.
 __device__ __forceinline__ int fx_line_K(int emax, unsigned S, int lim) {
-  return lim - (32 - __clz(S)) - (emax - 1039);
+  return min(lim - (32 - __clz(S)) - (emax - 1039), 1083 - emax);  // the bound holds for lines of subnormals only
 }
 // round(x 2^K), K from fx_line_K of the line (lim <= 61, so the shift is at least 2)
 __device__ __forceinline__ long long fx_quant(double x, int K) {
@@ -262,6 +262,21 @@ __device__ __forceinline__ long long fx_quant(double x, int K) {
   m = ((m << 10) >> (r - 1)) + 1 >> 1;
   const long long s = (long long)hi >> 63;  // sign
   return ((long long)m ^ s) - s;
+}
+// v 2^-K, rounded to nearest even, without the conversion instruction
+__device__ __forceinline__ double fx_to_double(long long v, int K) {
+  if (v == 0) return K <= FX_NAN / 2 ? __longlong_as_double(0x7ff8000000000000ll) : 0.0;
+  unsigned long long u = (unsigned long long)(v < 0 ? -v : v);
+  const int lz = __clzll((long long)u);
+  const int E = 1085 - lz - K;  // biased exponent - 1
+  if (E < 0 || E > 2044) {      // rare: results near the ends of the exponent range
+    if (K <= FX_NAN / 2) return __longlong_as_double(0x7ff8000000000000ll);
+    return scalbn(__ll2double_rn(v), -K);
+  }
+  u <<= lz;
+  const unsigned r = (((unsigned)u & 0x7ffu) + ((unsigned)(u >> 11) & 1u) + 0x3ffu) >> 11;
+  const unsigned long long b = ((unsigned long long)(unsigned)E << 52) + (u >> 11) + r;
+  return __longlong_as_double((long long)(b | ((unsigned long long)v & 0x8000000000000000ull)));
 }
 // v 2^-K
 __device__ __forceinline__ double fx_double(long long v, int K) {

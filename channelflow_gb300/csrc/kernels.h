@@ -37,8 +37,6 @@ cudaError_t launch_dct(int N, bool inverse, int nmodes, int ncomp, const cpx<R>*
 size_t cheb_smem_bytes(int N, size_t rsize);
 
 template <typename R>
-size_t curl_cheb_smem_bytes(int N);
-template <typename R>
 cudaError_t launch_curl_cheb(const GridDev& g, int N, const double* U, R* W6, const R* CA, const R* CB, const R* DA,
                              const R* DB, const R* basey, double Vsuck, cudaStream_t st,
                              int bstride = 0, const Dither& dt = kNoDither);
@@ -56,11 +54,42 @@ std::vector<uint16_t> cheb_tc_matrix(const std::vector<double>& F, int N);
 cudaError_t launch_cheb_tc(int N, int nlines, int ncomp, const float* in, size_t ld, size_t cs, float* out,
                            const void* Ag, int* err, cudaStream_t st);
 
+// Chebyshev transforms of FP64 lines on the tensor cores by exact integer products (cheb_oz.cu).  Matrix tables:
+// digits and row exponents of oz_matrix, uploaded; false where N is too large for exact accumulation.
+enum { OZ_T = 0, OZ_F = 1, OZ_DF = 2 };  // inverse, forward, derivative of forward (for b - a = 2)
+constexpr int OZ_MAX_JOBS = 6;
+struct OzMatrix {
+  const void* digits;
+  const int* rexp;
+};
+struct OzTables {
+  int N;
+  OzMatrix T, F, DF;
+};
+// One transform: element (n, line) of in / out at [n ld + line]; modes are pairs of lines (re, im).
+struct OzJob {
+  const double* in;
+  double* out;
+  // inverse: i kx and i kz times the result (both or none); Chebyshev coefficients added to the real part of each
+  // field's (0,0) mode, shift subtracted from the first of them; deriv: d/dy
+  double *gx, *gz;
+  const double* base;
+  int bstride;
+  double shift;
+  int deriv;
+  // forward: out = F (wF in + wK (i kx pkx + i kz pkz)) + wD DF pd (pkx null: F in; in may be null beside pkx)
+  const double *pkx, *pkz, *pd;
+  double wF, wK, wD;
+  int inplace;  // forward: out == in
+};
+size_t oz_matrix_bytes(int N);
+bool oz_matrix(int N, int kind, std::vector<uint16_t>& digits, std::vector<int>& rexp);
+cudaError_t launch_cheb_oz(const GridDev& g, int N, bool inverse, int nlines, size_t ld, const OzTables& t, const OzJob* jobs,
+                           int njobs, int* err, cudaStream_t st);
+
 // Nonlinear forms (values of the reference's NonlinearMethod enum, dnsflags.h:28-35)
 enum { NL_ROTATIONAL = 0, NL_CONVECTION = 1, NL_DIVERGENCE = 2, NL_SKEW = 3 };
 
-template <typename R>
-size_t grad_cheb_smem_bytes(int N);
 template <typename R>
 cudaError_t launch_grad_cheb(const GridDev& g, int N, bool gradient, const double* U, R* W, const R* CA, const R* CB,
                              const R* DA, const R* DB, const R* basey, double Vsuck, cudaStream_t st,
@@ -81,8 +110,6 @@ cudaError_t launch_zrot(const GridDev& g, int RC, const cpx<float>* X, cpx<float
                         cudaStream_t st, const Dither& dt);
 void set_zpass_register(int enable);
 template <typename R>
-size_t cheb_fwd_div_smem_bytes(int N);
-template <typename R>
 cudaError_t launch_cheb_fwd_div(const GridDev& g, int N, const R* pF, const R* pKx, const R* pKz, const R* pD, R wF,
                                 R wK, R wD, R* out, const R* FA, const R* FB, const R* DFA, const R* DFB,
                                 cudaStream_t st, const Dither& dt = kNoDither);
@@ -102,15 +129,18 @@ size_t xfft_smem_bytes(const GridDev& g, int czc = 0);  // czc <= 0: all solved 
 // x passes: czc kz columns per block (0: as many as fit in shared memory); FP64 on 64-bit integers, as the z pass
 template <typename R>
 cudaError_t launch_xinv(const GridDev& g, const FftPlan& px, const cpx<R>* twx, const void* twq, const cpx<R>* W,
-                        cpx<R>* X, int ncomp, cudaStream_t st, int czc = 0, const Dither& dt = kNoDither);
+                        cpx<R>* X, int ncomp, cudaStream_t st, int czc = 0, const Dither& dt = kNoDither,
+                        bool curl = false);
 template <typename R>
 cudaError_t launch_xfwd(const GridDev& g, const FftPlan& px, const cpx<R>* twx, const void* twq, const cpx<R>* Z,
                         cpx<R>* F, int ncomp, cudaStream_t st, int czc = 0, const Dither& dt = kNoDither);
 
 // The FP64 passes on 64-bit integers (xz_fx.cu): fx_twiddles splits a plan's twiddle table (four ints per entry).
 std::vector<int> fx_twiddles(const std::vector<std::complex<long double>>& tw);
+// curl: W holds u, v, w, dw/dy, -, du/dy; components 3, 4, 5 transformed are the vorticity (launch_curl_points: in place)
 cudaError_t launch_xinv_fx(const GridDev& g, const FftPlan& px, const void* tw, const cpx<double>* W, cpx<double>* X,
-                           int ncomp, int czc, cudaStream_t st);
+                           int ncomp, int czc, bool curl, cudaStream_t st);
+cudaError_t launch_curl_points(const GridDev& g, cpx<double>* W, cudaStream_t st);
 cudaError_t launch_xfwd_fx(const GridDev& g, const FftPlan& px, const void* tw, const cpx<double>* Z, cpx<double>* F,
                            int ncomp, int czc, cudaStream_t st);
 cudaError_t launch_zphys_fx(const GridDev& g, int form, const FftPlan& pz, const void* tw, int RP, const cpx<double>* X,

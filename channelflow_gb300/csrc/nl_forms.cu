@@ -634,18 +634,19 @@ cudaError_t launch_rotation(const GridDev& g, int N, const double* U, const doub
                                          const Dither&);                                                          \
   template cudaError_t launch_rotation<R>(const GridDev&, int, const double*, const double*, int, double, double,   \
                                           R*, cudaStream_t);                                                       \
-  template size_t grad_cheb_smem_bytes<R>(int);                                                                    \
-  template cudaError_t launch_grad_cheb<R>(const GridDev&, int, bool, const double*, R*, const R*, const R*,      \
-                                           const R*, const R*, const R*, double, cudaStream_t, int, const Dither&); \
   template size_t zphys_smem_bytes<R>(const GridDev&, int, int);                                                   \
   template cudaError_t launch_zphys<R>(const GridDev&, int, const FftPlan&, const cpx<R>*, const void*, int, const cpx<R>*, \
-                                       cpx<R>*, cudaStream_t, const Dither&, const cpx<R>*);                       \
-  template size_t cheb_fwd_div_smem_bytes<R>(int);                                                                 \
-  template cudaError_t launch_cheb_fwd_div<R>(const GridDev&, int, const R*, const R*, const R*, const R*, R, R, R, \
-                                              R*, const R*, const R*, const R*, const R*, cudaStream_t, const Dither&);
+                                       cpx<R>*, cudaStream_t, const Dither&, const cpx<R>*);
 
 INST_FORMS(float)
 INST_FORMS(double)
+// FP64 takes cheb_oz.cu
+template cudaError_t launch_grad_cheb<float>(const GridDev&, int, bool, const double*, float*, const float*, const float*,
+                                             const float*, const float*, const float*, double, cudaStream_t, int,
+                                             const Dither&);
+template cudaError_t launch_cheb_fwd_div<float>(const GridDev&, int, const float*, const float*, const float*, const float*,
+                                                float, float, float, float*, const float*, const float*, const float*,
+                                                const float*, cudaStream_t, const Dither&);
 
 // Advance every field's constant version after a nonlinear evaluation (one thread per field).
 __global__ void k_dither_bump(int* ver, int nb) {

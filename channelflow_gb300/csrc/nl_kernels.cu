@@ -463,11 +463,6 @@ cudaError_t launch_curl_cheb(const GridDev& g, int N, const double* U, R* W6, co
 template cudaError_t launch_curl_cheb<float>(const GridDev&, int, const double*, float*, const float*, const float*,
                                              const float*, const float*, const float*, double, cudaStream_t, int,
                                              const Dither&);
-template cudaError_t launch_curl_cheb<double>(const GridDev&, int, const double*, double*, const double*,
-                                              const double*, const double*, const double*, const double*, double,
-                                              cudaStream_t, int, const Dither&);
-template size_t curl_cheb_smem_bytes<float>(int);
-template size_t curl_cheb_smem_bytes<double>(int);
 
 // ---------------------------------------------------------------------------
 // x-direction inverse FFT of the solved (kx, kz) block of one y-plane and
@@ -651,10 +646,10 @@ size_t xfft_smem_bytes(const GridDev& g, int czc) {
 
 template <typename R>
 cudaError_t launch_xinv(const GridDev& g, const FftPlan& px, const cpx<R>* twx, const void* twq, const cpx<R>* W,
-                        cpx<R>* X, int ncomp, cudaStream_t st, int czc, const Dither& dt) {
+                        cpx<R>* X, int ncomp, cudaStream_t st, int czc, const Dither& dt, bool curl) {
   if (czc <= 0 || czc > g.NKz) czc = xfft_cols<R>(g);
   if constexpr (sizeof(R) == 8) {
-    return launch_xinv_fx(g, px, twq, W, X, ncomp, czc, st);
+    return launch_xinv_fx(g, px, twq, W, X, ncomp, czc, curl, st);
   } else {
     // kernel attributes set once per process (thread-safe static initialisation)
     static const bool attr_set = [] {
@@ -688,7 +683,7 @@ cudaError_t launch_xfwd(const GridDev& g, const FftPlan& px, const cpx<R>* twx, 
 
 #define INST_R(R)                                                                                                   \
   template cudaError_t launch_xinv<R>(const GridDev&, const FftPlan&, const cpx<R>*, const void*, const cpx<R>*,    \
-                                      cpx<R>*, int, cudaStream_t, int, const Dither&);                              \
+                                      cpx<R>*, int, cudaStream_t, int, const Dither&, bool);                        \
   template cudaError_t launch_xfwd<R>(const GridDev&, const FftPlan&, const cpx<R>*, const void*, const cpx<R>*,    \
                                       cpx<R>*, int, cudaStream_t, int, const Dither&);                              \
   template size_t xfft_smem_bytes<R>(const GridDev&, int);

@@ -18,6 +18,7 @@
 //
 // Kernels (not on the DNS step's hot path, which keeps only solved modes and fuses its transforms into the
 // nonlinear pass):
+//   launch_cheb_oz (cheb_oz.cu)  y-lines on the tensor cores, in place; where Ny is not covered:
 //   k_cheb_full   dense Ny x Ny FP64 product per y-line, 32 x 32 output tiles staged through shared memory
 //   k_xcols       complex FFT along x of kz columns of one (y, component) plane, in place
 //   k_zrows       z transform of x rows: c2r (Hermitian completion, FFTW's convention of taking only the
@@ -26,8 +27,10 @@
 #include "../../include/cfgpu.h"
 #include "kernels.h"
 
+#include <algorithm>
 #include <cmath>
 #include <complex>
+#include <cstring>
 #include <string>
 #include <vector>
 
@@ -165,6 +168,8 @@ struct cfgpu_flowfield_s {
   size_t n = 0;  // doubles
   double* data = nullptr;
   double* work = nullptr;
+  OzTables oz{};  // N = 0: Ny not covered, dense products with Mfwd, Minv
+  unsigned char* ozblock = nullptr;
   double* Mfwd = nullptr;  // [n][j] chebyfft
   double* Minv = nullptr;  // [j][n] ichebyfft
   cpx<double>* twx = nullptr;
@@ -186,6 +191,21 @@ int y_transform(cfgpu_flowfield f, bool to_spectral) {
   if (f->Ny < 2) return CFGPU_OK;
   const int nl = f->Nx * 2 * (f->Nz / 2 + 1);
   const size_t cs = (size_t)f->Ny * nl;
+  if (f->oz.N) {
+    GridDev g{};
+    g.b = 1;
+    g.a = -1;
+    for (int c0 = 0; c0 < f->Nd; c0 += OZ_MAX_JOBS) {
+      OzJob job[OZ_MAX_JOBS] = {};
+      const int nj = std::min(OZ_MAX_JOBS, f->Nd - c0);
+      for (int c = 0; c < nj; ++c) {
+        job[c].in = job[c].out = f->data + (c0 + c) * cs;
+        job[c].inplace = 1;
+      }
+      TF_CK(launch_cheb_oz(g, f->Ny, !to_spectral, nl, nl, f->oz, job, nj, nullptr, f->st));
+    }
+    return CFGPU_OK;
+  }
   dim3 grid((nl + CT - 1) / CT, (f->Ny + CT - 1) / CT, f->Nd);
   k_cheb_full<<<grid, 256, 0, f->st>>>(f->Ny, nl, cs, to_spectral ? f->Mfwd : f->Minv, f->data, f->work);
   TF_CK(cudaGetLastError());
@@ -260,25 +280,44 @@ cfgpu_status cfgpu_flowfield_create(const cfgpu_grid* g, int Nd, cfgpu_flowfield
     st = tf_fail(CFGPU_ECUDA, "cudaStreamCreate failed");
   if (st == CFGPU_OK) {
     cudaError_t e = cudaMalloc((void**)&f->data, f->n * sizeof(double));
-    if (e == cudaSuccess) e = cudaMalloc((void**)&f->work, f->n * sizeof(double));
     if (e == cudaSuccess) e = cudaMemsetAsync(f->data, 0, f->n * sizeof(double), f->st);
     if (e != cudaSuccess) st = tf_fail(CFGPU_ENOMEM, std::string("cudaMalloc: ") + cudaGetErrorString(e));
   }
   if (st == CFGPU_OK) {
     const int N = g->Ny;
-    std::vector<double> Mf((size_t)N * N), Mi((size_t)N * N);
-    for (int n = 0; n < N; ++n)
-      for (int j = 0; j < N; ++j) {
-        const long double cn = (n == 0 || n == N - 1) ? 0.5L : 1.0L;
-        const long double w = (j == 0 || j == N - 1) ? 1.0L : 2.0L;
-        Mf[(size_t)n * N + j] = (double)(w * cn * cospi_frac((long long)n * j, N - 1) / (N - 1));
-        Mi[(size_t)j * N + n] = (double)cospi_frac((long long)n * j, N - 1);
+    std::vector<uint16_t> dg[2];
+    std::vector<int> re[2];
+    std::vector<unsigned char> oz;
+    std::vector<double> Mf, Mi;
+    if (f->n / Nd < (1ull << 32) && oz_matrix(N, OZ_T, dg[0], re[0]) && oz_matrix(N, OZ_F, dg[1], re[1])) {
+      const size_t mb = oz_matrix_bytes(N), rb = re[0].size() * sizeof(int);
+      oz.resize(2 * (mb + rb));
+      for (int k = 0; k < 2; ++k) {
+        std::memcpy(oz.data() + k * mb, dg[k].data(), mb);
+        std::memcpy(oz.data() + 2 * mb + k * rb, re[k].data(), rb);
       }
+      st = tf_upload(oz, &f->ozblock, f->st);
+      f->oz.N = N;
+      f->oz.T = OzMatrix{f->ozblock, (const int*)(f->ozblock + 2 * mb)};
+      f->oz.F = OzMatrix{f->ozblock + mb, (const int*)(f->ozblock + 2 * mb + rb)};
+    } else {
+      Mf.resize((size_t)N * N);
+      Mi.resize((size_t)N * N);
+      for (int n = 0; n < N; ++n)
+        for (int j = 0; j < N; ++j) {
+          const long double cn = (n == 0 || n == N - 1) ? 0.5L : 1.0L;
+          const long double w = (j == 0 || j == N - 1) ? 1.0L : 2.0L;
+          Mf[(size_t)n * N + j] = (double)(w * cn * cospi_frac((long long)n * j, N - 1) / (N - 1));
+          Mi[(size_t)j * N + n] = (double)cospi_frac((long long)n * j, N - 1);
+        }
+      if (cudaMalloc((void**)&f->work, f->n * sizeof(double)) != cudaSuccess)
+        st = tf_fail(CFGPU_ENOMEM, "cudaMalloc: work array");
+      if (st == CFGPU_OK) st = tf_upload(Mf, &f->Mfwd, f->st);
+      if (st == CFGPU_OK) st = tf_upload(Mi, &f->Minv, f->st);
+    }
     std::vector<cpx<double>> tx(twx.size() ? twx.size() : 1), tz(twz.size() ? twz.size() : 1);
     for (size_t i = 0; i < twx.size(); ++i) tx[i] = cmk<double>((double)twx[i].real(), (double)twx[i].imag());
     for (size_t i = 0; i < twz.size(); ++i) tz[i] = cmk<double>((double)twz[i].real(), (double)twz[i].imag());
-    st = tf_upload(Mf, &f->Mfwd, f->st);
-    if (st == CFGPU_OK) st = tf_upload(Mi, &f->Minv, f->st);
     if (st == CFGPU_OK) st = tf_upload(tx, &f->twx, f->st);
     if (st == CFGPU_OK) st = tf_upload(tz, &f->twz, f->st);
     // the host vectors go out of scope: wait for the copies
@@ -297,6 +336,7 @@ cfgpu_status cfgpu_flowfield_destroy(cfgpu_flowfield f) {
   if (f->st) cudaStreamSynchronize(f->st);
   cudaFree(f->data);
   cudaFree(f->work);
+  cudaFree(f->ozblock);
   cudaFree(f->Mfwd);
   cudaFree(f->Minv);
   cudaFree(f->twx);

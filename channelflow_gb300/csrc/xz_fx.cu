@@ -43,8 +43,31 @@ __device__ __forceinline__ int fx_scale_column(fxc* col, int n, POS pos, int lan
   return key == 0 ? FX_ZERO : (emax == 2047 ? FX_NAN : K);
 }
 
+// Vorticity component c - 3 of a mode (wavenumbers kx, kz) at one point, W (component stride cs) = u, v, w, dw/dy, -,
+// du/dy:  omega = (dw/dy - i kz v, i kz u - i kx w, i kx v - du/dy).
+__device__ __forceinline__ double2 fx_vorticity(int c, const double2* W, size_t cs, double kx, double kz) {
+  if (c == 4) {
+    const double2 u = W[0], w = W[2 * cs];
+    return make_double2(kx * w.y - kz * u.y, kz * u.x - kx * w.x);
+  }
+  const double2 v = W[cs], d = W[c * cs];
+  if (c == 3) return make_double2(fma(kz, v.y, d.x), fma(-kz, v.x, d.y));
+  return make_double2(fma(-kx, v.y, -d.x), fma(kx, v.x, -d.y));
+}
+
+__global__ void k_curl_points(GridDev g, double2* W) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x, ny = blockIdx.y;
+  if (i >= g.Md) return;
+  const int ix = i / g.NKz, iz = i - ix * g.NKz;
+  const size_t cs = (size_t)g.Ny * g.Md;
+  double2* w = W + (size_t)ny * g.Md + i;
+  const double kx = 2.0 * M_PI / g.Lx * (ix <= g.Kx ? ix : ix - g.NKx), kz = 2.0 * M_PI / g.Lz * iz;
+  for (int c = 3; c < 6; ++c) w[c * cs] = fx_vorticity(c, w, cs, kx, kz);
+}
+
 __global__ void __launch_bounds__(FX_THREADS) k_xinv_fx(GridDev g, FftPlan px, const fxtw* __restrict__ tw,
-                                                        const double2* __restrict__ W, double2* __restrict__ X, int czc) {
+                                                        const double2* __restrict__ W, double2* __restrict__ X, int czc,
+                                                        int curl) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   pdl_wait();  // launched with launch_pdl: the previous kernel's output is read from here on
   const int ss = g.Nx + 1;
@@ -52,16 +75,25 @@ __global__ void __launch_bounds__(FX_THREADS) k_xinv_fx(GridDev g, FftPlan px, c
   const float invc = 1.0f / nc;
   fxc* a = reinterpret_cast<fxc*>(smem_raw);
   fxc* b = a + (size_t)czc * ss;
-  int* sK = reinterpret_cast<int*>(b + (size_t)czc * ss);
+  double* skx = reinterpret_cast<double*>(b + (size_t)czc * ss);  // wavenumbers (curl)
+  double* skz = skx + (curl ? g.NKx : 0);
+  int* sK = reinterpret_cast<int*>(skz + (curl ? czc : 0));
   const int ny = blockIdx.x, c = blockIdx.y;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const double2* src = W + ((size_t)c * g.Ny + ny) * g.Md;
   const int Kx = g.Kx, NKx = g.NKx, Nx = g.Nx;
+  if (curl && c >= 3) {
+    for (int i = tid; i < NKx; i += FX_THREADS) skx[i] = 2.0 * M_PI * (i <= Kx ? i : i - NKx) / g.Lx;
+    for (int i = tid; i < nc; i += FX_THREADS) skz[i] = 2.0 * M_PI * (iz0 + i) / g.Lz;
+    __syncthreads();
+  }
 #pragma unroll 4
   for (int i = tid; i < NKx * nc; i += FX_THREADS) {
     int ix, jz;
     divmod_small(i, nc, invc, ix, jz);
-    const double2 v = src[ix * g.NKz + iz0 + jz];
+    double2 v = src[ix * g.NKz + iz0 + jz];
+    if (curl && c >= 3) v = fx_vorticity(c, W + (size_t)ny * g.Md + ix * g.NKz + iz0 + jz, (size_t)g.Ny * g.Md,
+                                         skx[ix], skz[jz]);
     a[jz * ss + (ix <= Kx ? ix : Nx + ix - NKx)] = fxc{__double_as_longlong(v.x), __double_as_longlong(v.y)};
   }
   {
@@ -375,7 +407,9 @@ cudaError_t run_zphys_fx(const GridDev& g, const FftPlan& pz, const fxtw* tw, in
                     zphys_smem_bytes<double>(g, FORM, RP), st, g, pz, tw, RP, X, Z);
 }
 
-size_t xfx_smem(const GridDev& g, int czc) { return xfft_smem_bytes<double>(g, czc) + sizeof(int) * czc; }
+size_t xfx_smem(const GridDev& g, int czc, bool curl) {
+  return xfft_smem_bytes<double>(g, czc) + sizeof(int) * czc + (curl ? sizeof(double) * (g.NKx + czc) : 0);
+}
 
 }  // namespace
 
@@ -389,14 +423,24 @@ std::vector<int> fx_twiddles(const std::vector<std::complex<long double>>& tw) {
 }
 
 cudaError_t launch_xinv_fx(const GridDev& g, const FftPlan& px, const void* tw, const cpx<double>* W, cpx<double>* X,
-                           int ncomp, int czc, cudaStream_t st) {
+                           int ncomp, int czc, bool curl, cudaStream_t st) {
   static const bool attr = [] {
     cudaFuncSetAttribute(k_xinv_fx, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
     return true;
   }();
   (void)attr;
-  return launch_pdl(k_xinv_fx, dim3(g.Ny, ncomp, (g.NKz + czc - 1) / czc), dim3(FX_THREADS), xfx_smem(g, czc), st, g, px,
-                    (const fxtw*)tw, (const double2*)W, (double2*)X, czc);
+  if (curl && xfx_smem(g, czc, true) > 227 * 1024) {  // no room for the wavenumbers beside one very long column
+    const cudaError_t e = launch_curl_points(g, const_cast<cpx<double>*>(W), st);
+    if (e != cudaSuccess) return e;
+    curl = false;
+  }
+  return launch_pdl(k_xinv_fx, dim3(g.Ny, ncomp, (g.NKz + czc - 1) / czc), dim3(FX_THREADS), xfx_smem(g, czc, curl), st, g, px,
+                    (const fxtw*)tw, (const double2*)W, (double2*)X, czc, (int)curl);
+}
+
+cudaError_t launch_curl_points(const GridDev& g, cpx<double>* W, cudaStream_t st) {
+  k_curl_points<<<dim3((g.Md + 127) / 128, g.Ny), 128, 0, st>>>(g, (double2*)W);
+  return cudaGetLastError();
 }
 
 cudaError_t launch_xfwd_fx(const GridDev& g, const FftPlan& px, const void* tw, const cpx<double>* Z, cpx<double>* F,
@@ -407,7 +451,7 @@ cudaError_t launch_xfwd_fx(const GridDev& g, const FftPlan& px, const void* tw, 
   }();
   (void)attr;
   const double scale = 1.0 / ((double)g.Nx * (double)g.Nz);
-  return launch_pdl(k_xfwd_fx, dim3(g.Ny, ncomp, (g.NKz + czc - 1) / czc), dim3(FX_THREADS), xfx_smem(g, czc), st, g, px,
+  return launch_pdl(k_xfwd_fx, dim3(g.Ny, ncomp, (g.NKz + czc - 1) / czc), dim3(FX_THREADS), xfx_smem(g, czc, false), st, g, px,
                     (const fxtw*)tw, (const double2*)Z, (double2*)F, scale, czc);
 }
 
