@@ -175,134 +175,6 @@ __device__ __forceinline__ int n_func(int k, int Nb) {
   return 2 * Nb;
 }
 
-// One thread per mode: the TauSolver constructor for lambda = lambda_t + nu kappa^2,
-// for modes m0 .. m0+mcount-1.
-// blockIdx.y selects one of tb's tables (its lambda_t; 4 scratch lines of its own).
-__global__ void k_tau_setup(GridDev g, int N, TauSetupBatch tb, double nu, HelmB hb, double* scratch, int m0,
-                            int mcount) {
-  const int m = m0 + blockIdx.x * blockDim.x + threadIdx.x;
-  if (m >= m0 + mcount || m >= g.Md) return;
-  const size_t Md = g.Md;
-  const size_t FN = (size_t)N * Md;
-  const double lambda_t = tb.lambda_t[blockIdx.y];
-  const TauTable tt = tb.tab[blockIdx.y];
-  scratch += (size_t)blockIdx.y * 4 * FN;
-  auto T = [&](int f) { return Ln{tt.f + f * FN + m, Md}; };
-  auto S = [&](int k) { return Ln{scratch + k * FN + m, Md}; };
-  const int kx = mode_kx(g, m), kz = mode_kz(g, m);
-  const double Lx = g.Lx, Lz = g.Lz, a = g.a, b = g.b;
-  const double kappa2 = 4 * (M_PI * M_PI) * ((kx / Lx) * (kx / Lx) + (kz / Lz) * (kz / Lz));
-  const double c4 = 4.0 * (M_PI * M_PI) * nu;
-  const double lambda = lambda_t + c4 * ((kx / Lx) * (kx / Lx) + (kz / Lz) * (kz / Lz));
-  const double scale = 4.0 / (b - a);
-  const int Nb = N - 1;
-  HelmFac PH{T(TF_PBAND), T(TF_PUP), T(TF_PLO), T(TF_PINV)};
-  HelmFac VH{T(TF_VBAND), T(TF_VUP), T(TF_VLO), T(TF_VINV)};
-  helm_build(N, a, b, kappa2, 1.0, PH);
-  helm_build(N, a, b, lambda, nu, VH);
-  Ln z = S(0), d = S(1), d2 = S(2);
-  for (int n = 0; n < N; ++n) z[n] = 0.0;
-  Ln Pp = T(TF_PP), Vp = T(TF_VP), Pm = T(TF_PM), Vm = T(TF_VM), P0 = T(TF_P0), V0 = T(TF_V0);
-  helm_solve(PH, hb, N, z, Pp, 0.0, 1.0);
-  cheb_diff(N, scale, Pp, d);
-  helm_solve(VH, hb, N, d, Vp, 0.0, 0.0);
-  helm_solve(PH, hb, N, z, Pm, 1.0, 0.0);
-  cheb_diff(N, scale, Pm, d);
-  helm_solve(VH, hb, N, d, Vm, 0.0, 0.0);
-  cheb_diff(N, scale, Vp, d);
-  const double A = eval_b(N, d), C = eval_a(N, d);
-  cheb_diff(N, scale, Vm, d);
-  const double B = eval_b(N, d), D = eval_a(N, d);
-  const bool zero = (kx == 0 && kz == 0);
-  const double disc = A * D - B * C;
-  double i00 = 0, i01 = 0, i10 = 0, i11 = 0;
-  if (!zero) {
-    i00 = D / disc;
-    i01 = -B / disc;
-    i10 = -C / disc;
-    i11 = A / disc;
-  }
-  const double c = 2 / (b - a);
-  for (int n = 0; n < N; ++n) z[n] = c * n_func(n, Nb);
-  helm_solve(PH, hb, N, z, P0, 0.0, 0.0);
-  cheb_diff(N, scale, P0, d2);  // dP0dy (before the influence correction, as the reference)
-  helm_solve(VH, hb, N, d2, V0, 0.0, 0.0);
-  if (!zero) {
-    cheb_diff(N, scale, V0, d);
-    const double plus = eval_b(N, d), minus = eval_a(N, d);
-    const double dp = -i00 * plus - i01 * minus;
-    const double dm = -i10 * plus - i11 * minus;
-    for (int n = 0; n < N; ++n) {
-      P0[n] += dp * Pp[n] + dm * Pm[n];
-      V0[n] += dp * Vp[n] + dm * Vm[n];
-    }
-  }
-  // v0yy at Nb-1, Nb is identically zero (two downward recurrences from d[Nb] = 0)
-  cheb_diff(N, scale, V0, d);
-  Ln d3 = S(3);
-  cheb_diff(N, scale, d, d3);
-  const double s0Nb1 = lambda * V0[Nb - 1] + d2[Nb - 1] - nu * d3[Nb - 1];
-  const double s0Nb = lambda * V0[Nb] + d2[Nb] - nu * d3[Nb];
-  // segment products of the UL sweeps of both factorisations (four segments of L rows per parity)
-  {
-    const int L = tau_seg_rows(N);
-    const HelmFac* fac[2] = {&PH, &VH};
-    Ln Hs[2] = {T(TF_PH), T(TF_VH)}, Gs[2] = {T(TF_PG), T(TF_VG)};
-    for (int f = 0; f < 2; ++f)
-      for (int q = 0; q < 2; ++q) {
-        const int M = q == 0 ? nE_of(N) : nO_of(N);
-        Hs[f][q] = 1.0;
-        Gs[f][q] = 1.0;
-        for (int i0 = 0; i0 < M; i0 += L) {
-          const int ia = i0 > 1 ? i0 : 1, ib = i0 + L < M ? i0 + L : M;
-          double h = 1.0;
-          for (int i = ib - 1; i >= ia; --i) {
-            h = -fac[f]->up[2 * i + q] * h;
-            Hs[f][2 * i + q] = h;
-          }
-          double gg = 1.0;
-          for (int i = ia; i < ib; ++i) {
-            gg = (-fac[f]->lo[2 * i + q] * gg) * fac[f]->inv[2 * i + q];
-            Gs[f][2 * i + q] = gg;
-          }
-        }
-      }
-  }
-  // mean-constrained helper (helmholtz.cpp:193-205): mean of the solution of nu u'' - lambda u = nu
-  for (int n = 0; n < N; ++n) z[n] = 0.0;
-  z[0] = nu;
-  helm_solve(VH, hb, N, z, d, 0.0, 0.0);
-  const double ucmean = cheb_mean(N, d);
-  double* s = tt.s + m;
-  s[TS_I00 * Md] = i00;
-  s[TS_I01 * Md] = i01;
-  s[TS_I10 * Md] = i10;
-  s[TS_I11 * Md] = i11;
-  s[TS_S0NB1 * Md] = s0Nb1;
-  s[TS_S0NB * Md] = s0Nb;
-  s[TS_UCMEAN * Md] = ucmean;
-  s[TS_LAMBDA * Md] = lambda;
-  s[TS_KXL * Md] = 2 * M_PI * kx / Lx;
-  s[TS_KZL * Md] = 2 * M_PI * kz / Lz;
-  s[TS_DX * Md] = 2 * M_PI * kx / Lx * (kx == g.kxmax ? 0.0 : 1.0);
-  s[TS_DZ * Md] = 2 * M_PI * kz / Lz * (kz == g.kzmax ? 0.0 : 1.0);
-  s[TS_KAPPA2 * Md] = kappa2;
-  s[TS_RS0NB1 * Md] = zero ? 0.0 : 1.0 / (1.0 - s0Nb1);
-  s[TS_RS0NB * Md] = zero ? 0.0 : 1.0 / (1.0 - s0Nb);
-}
-
-cudaError_t launch_tau_setup_batch(const GridDev& g, int N, const TauSetupBatch& tb, int ntab, double nu,
-                                   const HelmB& hb, double* scratch, cudaStream_t st, int m0, int mcount) {
-  const int T = 64;
-  if (mcount <= 0) {
-    m0 = 0;
-    mcount = g.Md;
-  }
-  if (ntab < 1 || ntab > 4) return cudaErrorInvalidValue;
-  k_tau_setup<<<dim3((mcount + T - 1) / T, ntab), T, 0, st>>>(g, N, tb, nu, hb, scratch, m0, mcount);
-  return cudaGetLastError();
-}
-
 // ---------------------------------------------------------------------------
 // Batched HelmholtzSolver (helmholtz.cpp:18-95, 158-213): one thread per system
 // nu u'' - lambda_s u = f_s (+ mu_s), u(a) = ua_s, u(b) = ub_s, with the
@@ -346,14 +218,6 @@ cudaError_t launch_helmholtz(int N, int nsys, double a, double b, const double* 
   if (nsys <= 0) return cudaSuccess;
   k_helmholtz<<<(nsys + 127) / 128, 128, 0, st>>>(N, nsys, a, b, lambda, nu, hb, f, ua, ub, umean, u, mu, W);
   return cudaGetLastError();
-}
-
-cudaError_t launch_tau_setup(const GridDev& g, int N, double lambda_t, double nu, const HelmB& hb, TauTable tt,
-                             double* scratch, cudaStream_t st, int m0, int mcount) {
-  TauSetupBatch tb{};
-  tb.lambda_t[0] = lambda_t;
-  tb.tab[0] = tt;
-  return launch_tau_setup_batch(g, N, tb, 1, nu, hb, scratch, st, m0, mcount);
 }
 
 // ---------------------------------------------------------------------------
@@ -460,6 +324,187 @@ __device__ double diff_par(int M, int q, int N, double scale, PLn xo, PLn* dst) 
       }
   }
   return sum;
+}
+
+// ---------------------------------------------------------------------------
+// The TauSolver constructor (tausolver.cpp:81-176) for lambda = lambda_t + nu kappa^2, modes m0 .. m0 + mcount - 1;
+// blockIdx.y selects one of tb's tables (its lambda_t; 4 scratch lines of its own).  Four lanes a mode: two systems
+// (pressure, velocity) or right-hand sides (P+, P0) by two Chebyshev parities.  Bound by the chain of dependent FP64
+// operations of a lane (64 cycles each), so independent chains stand side by side and divisions are few:
+//   A = nu I - lambda B row by row, so its rows come from B's (no divisions), and one reciprocal per row serves the
+//   factorisation;
+//   P- is P+ mirrored: P-_n = (-1)^n P+_n, v-_n = (-1)^(n+1) v+_n and the walls change places, exactly;
+//   the mean of the constrained solve is needed for the (0,0) mode only.
+// 48x49x48: 631 us (one thread a mode) -> 89 us.
+// ---------------------------------------------------------------------------
+__global__ void __launch_bounds__(128) k_tau_setup(GridDev g, int N, TauSetupBatch tb, double nu, HelmB hb,
+                                                   double* scratch, int m0, int mcount) {
+  const int t = blockIdx.x * 128 + threadIdx.x;
+  const int mend = min(m0 + mcount, g.Md);
+  const int m = m0 + (t >> 2);
+  if (m >= mend) return;  // a mode's four lanes together
+  const int r = (t >> 1) & 1, q = t & 1;
+  const unsigned gmask = 0xFu << (threadIdx.x & 28);
+  const int Md = g.Md;
+  const size_t FN = (size_t)N * Md;
+  const double lambda_t = tb.lambda_t[blockIdx.y];
+  const TauTable tt = tb.tab[blockIdx.y];
+  scratch += (size_t)blockIdx.y * 4 * FN;
+  const int M = q ? N / 2 : (N + 1) / 2, Nb = N - 1;
+  auto T = [&](int f) { return PLn{tt.f + f * FN + m + (size_t)q * Md, 2 * Md}; };         // own parity
+  auto To = [&](int f) { return PLn{tt.f + f * FN + m + (size_t)(1 - q) * Md, 2 * Md}; };  // the other
+  auto S = [&](int k) { return PLn{scratch + k * FN + m + (size_t)q * Md, 2 * Md}; };
+  const int kx = mode_kx(g, m), kz = mode_kz(g, m);
+  const bool zero = kx == 0 && kz == 0;
+  const double rx = kx / g.Lx, rz = kz / g.Lz;
+  const double k2 = rx * rx + rz * rz;
+  const double kappa2 = 4 * (M_PI * M_PI) * k2;
+  const double lambda = lambda_t + 4.0 * (M_PI * M_PI) * nu * k2;
+  const double scale = 4.0 / (g.b - g.a);
+  {
+    // UL factors of system r (BandedTridiag::ULdecomp, bandedtridiag.cpp:212-229) and their segment products (four
+    // segments of L rows per parity)
+    const double lam = r ? lambda : kappa2, h = (g.b - g.a) / 2, nus = (r ? nu : 1.0) / (h * h);
+    const int f0 = r ? TF_VBAND : TF_PBAND, h0 = r ? TF_VH : TF_PH, g0 = r ? TF_VG : TF_PG;
+    PLn band = T(f0), up = T(f0 + 1), lo = T(f0 + 2), inv = T(f0 + 3);
+    PLn H = T(h0), G = T(g0);
+    const int L = tau_seg_rows(N);
+    double diag = nus - lam * __ldg(hb.di + 2 * (M - 1) + q), bk = 1.0, u = 0.0, hp = 1.0;
+    int top = (M - 1) / L * L;  // first row of the segment
+    for (int k = M - 1; k > 0; --k) {
+      const int n = 2 * k + q;
+      const double iv = 1.0 / diag, w = -(lam * __ldg(hb.lo + n));
+      hp = -u * hp;
+      bk *= iv;
+      inv[k] = iv;
+      lo[k] = w;
+      band[k] = bk;
+      up[k] = u;
+      H[k] = hp;
+      if (k == top) {
+        hp = 1.0;
+        top -= L;
+      }
+      bk = 1.0 - w * bk;
+      if (k > 1) {
+        u = -(lam * __ldg(hb.up + n - 2)) * iv;
+        diag = (nus - lam * __ldg(hb.di + n - 2)) - w * u;
+      }
+    }
+    band[0] = bk;
+    inv[0] = 1.0 / bk;
+    up[0] = lo[0] = 0.0;
+    H[0] = G[0] = 1.0;
+    double gp = 1.0;
+    for (int i0 = 1; i0 < M; i0 += TCH) {
+      double lv[TCH], iv[TCH];
+#pragma unroll
+      for (int k = 0; k < TCH; ++k)
+        if (i0 + k < M) {
+          lv[k] = lo[i0 + k];
+          iv[k] = inv[i0 + k];
+        }
+#pragma unroll
+      for (int k = 0; k < TCH; ++k)
+        if (i0 + k < M) {
+          if ((i0 + k) % L == 0) gp = 1.0;
+          gp = (-lv[k] * gp) * iv[k];
+          G[i0 + k] = gp;
+        }
+    }
+    // right-hand sides of the pressure solves: zero (P+) and n_func (P0)
+    const double c = r ? 2 / (g.b - g.a) : 0.0;
+    PLn z = S(r ? 0 : 3);
+    for (int i = 0; i < M; ++i) z[i] = c * n_func(2 * i + q, Nb);
+  }
+  __syncwarp(gmask);
+  PLn Pr = T(r ? TF_P0 : TF_PP), Vr = T(r ? TF_V0 : TF_VP), d = S(r ? 2 : 1);
+  helm_par(M, q, hb.lo, hb.di, hb.up, T(TF_PBAND), T(TF_PUP), T(TF_PLO), T(TF_PINV), S(r ? 0 : 3), Pr, r ? 0.0 : 0.5);
+  __syncwarp(gmask);
+  diff_par(M, q, N, scale, To(r ? TF_P0 : TF_PP), &d);  // of P0 before the influence correction, as the reference
+  helm_par(M, q, hb.lo, hb.di, hb.up, T(TF_VBAND), T(TF_VUP), T(TF_VLO), T(TF_VINV), d, Vr, 0.0);
+  __syncwarp(gmask);
+  const double sq = diff_par(M, q, N, scale, To(r ? TF_V0 : TF_VP), nullptr);
+  const double so = __shfl_xor_sync(gmask, sq, 1);
+  const double wb = q ? so + sq : sq + so, wa = q ? so - sq : sq - so;  // v' at b and a
+  const double A = __shfl_sync(gmask, wb, threadIdx.x & 28), C = __shfl_sync(gmask, wa, threadIdx.x & 28);
+  const double plus = __shfl_sync(gmask, wb, (threadIdx.x & 28) | 2), minus = __shfl_sync(gmask, wa, (threadIdx.x & 28) | 2);
+  double i00 = 0, i01 = 0;
+  if (!zero) {  // influence matrix A C / C A
+    const double disc = A * A - C * C;
+    i00 = A / disc;
+    i01 = -C / disc;
+  }
+  const double dp = -i00 * plus - i01 * minus, dm = -i01 * plus - i00 * minus;
+  {
+    // r = 0: the pressure lines, r = 1: the velocity lines; own parity
+    PLn p = T(r ? TF_VP : TF_PP), mm = T(r ? TF_VM : TF_PM), x = T(r ? TF_V0 : TF_P0);
+    const bool neg = r != q;
+    const double cm = zero ? 0.0 : (neg ? dp - dm : dp + dm);
+    for (int i = 0; i < M; ++i) {
+      const double v = p[i];
+      mm[i] = neg ? -v : v;
+      x[i] = fma(cm, v, x[i]);
+    }
+  }
+  __syncwarp(gmask);
+  double ucmean = 0.0;
+  if (zero) {
+    // mean-constrained helper (helmholtz.cpp:193-205): mean of the solution of nu u'' - lambda u = nu
+    if (r == 1 && q == 0) {
+      PLn z = S(0), u = S(1);
+      for (int i = 0; i < M; ++i) z[i] = 0.0;
+      z[0] = nu;
+      helm_par(M, 0, hb.lo, hb.di, hb.up, T(TF_VBAND), T(TF_VUP), T(TF_VLO), T(TF_VINV), z, u, 0.0);
+      ucmean = u[0];
+      for (int i = 1; i < M; ++i) ucmean -= u[i] / (double)(4 * i * i - 1);
+    }
+    ucmean = __shfl_sync(gmask, ucmean, (threadIdx.x & 28) | 2);
+  }
+  if (r == 0 && q == 0) {
+    // sigma0 at Nb - 1, Nb; v0'' is identically zero there (two downward recurrences from zero)
+    const double* V0 = tt.f + TF_V0 * FN + m;
+    const double* dP0 = scratch + 2 * FN + m;
+    const double s0Nb1 = lambda * V0[(size_t)(Nb - 1) * Md] + dP0[(size_t)(Nb - 1) * Md];
+    const double s0Nb = lambda * V0[(size_t)Nb * Md] + dP0[(size_t)Nb * Md];
+    double* s = tt.s + m;
+    const size_t Ms = Md;
+    s[TS_I00 * Ms] = i00;
+    s[TS_I01 * Ms] = i01;
+    s[TS_I10 * Ms] = i01;
+    s[TS_I11 * Ms] = i00;
+    s[TS_S0NB1 * Ms] = s0Nb1;
+    s[TS_S0NB * Ms] = s0Nb;
+    s[TS_UCMEAN * Ms] = ucmean;
+    s[TS_LAMBDA * Ms] = lambda;
+    s[TS_KXL * Ms] = 2 * M_PI * kx / g.Lx;
+    s[TS_KZL * Ms] = 2 * M_PI * kz / g.Lz;
+    s[TS_DX * Ms] = 2 * M_PI * kx / g.Lx * (kx == g.kxmax ? 0.0 : 1.0);
+    s[TS_DZ * Ms] = 2 * M_PI * kz / g.Lz * (kz == g.kzmax ? 0.0 : 1.0);
+    s[TS_KAPPA2 * Ms] = kappa2;
+    s[TS_RS0NB1 * Ms] = zero ? 0.0 : 1.0 / (1.0 - s0Nb1);
+    s[TS_RS0NB * Ms] = zero ? 0.0 : 1.0 / (1.0 - s0Nb);
+  }
+}
+
+cudaError_t launch_tau_setup_batch(const GridDev& g, int N, const TauSetupBatch& tb, int ntab, double nu,
+                                   const HelmB& hb, double* scratch, cudaStream_t st, int m0, int mcount) {
+  const int T = 128;
+  if (mcount <= 0) {
+    m0 = 0;
+    mcount = g.Md;
+  }
+  if (ntab < 1 || ntab > 4) return cudaErrorInvalidValue;
+  k_tau_setup<<<dim3((4 * mcount + T - 1) / T, ntab), T, 0, st>>>(g, N, tb, nu, hb, scratch, m0, mcount);
+  return cudaGetLastError();
+}
+
+cudaError_t launch_tau_setup(const GridDev& g, int N, double lambda_t, double nu, const HelmB& hb, TauTable tt,
+                             double* scratch, cudaStream_t st, int m0, int mcount) {
+  TauSetupBatch tb{};
+  tb.lambda_t[0] = lambda_t;
+  tb.tab[0] = tt;
+  return launch_tau_setup_batch(g, N, tb, 1, nu, hb, scratch, st, m0, mcount);
 }
 
 template <typename R>
@@ -782,7 +827,69 @@ __device__ void helm_t(int M, int q, const double* __restrict__ hlo, const doubl
 }
 
 // ---------------------------------------------------------------------------
-// Right-hand side of the step solve (NSE::linear and the scheme's combination,
+// Right-hand side of a multistep scheme, sum_j a_j u_j + b_j N_j (dnsalgo.cpp:217-224), elementwise: one thread per
+// (component, n, mode), one component a grid layer (blockIdx.z), into the scratch lines 0, 2 and 1.  Bound by its 4
+// ORDER FP64 multiply-adds a mode and coefficient (64 cycles a warp instruction); the FP32 history is widened on
+// integers.  The (0,0) modes' base-flow and pressure-gradient terms run in a layer of their own: a predicated FP64
+// instruction takes the whole warp's slot.  Against four lanes a mode walking the rows, SBDF3: 64 x 48x49x48 mixed 303
+// -> 119 us, 128x97x128 FP64 64 -> 29 us, 32x35x32 FP64 16 -> 4.5 us.
+// ---------------------------------------------------------------------------
+template <typename R, int ORDER>
+__global__ void __launch_bounds__(128) k_tau_rhs_ms(GridDev g, int N, SolveParams sp, SolvePtrs P) {
+  pdl_wait();
+  pdl_trigger();
+  const int m = blockIdx.x * 128 + threadIdx.x, n = blockIdx.y;
+  if (m >= g.Md) return;
+  const bool m00 = mode_kx(g, m) == 0 && mode_kz(g, m) == 0;
+  if (m00 != (blockIdx.z == 3)) return;
+  const int fld = mode_field(g, m);
+  if (P.slot) apply_slot(sp, P.slot[fld]);
+  const size_t comp = (size_t)g.Md * N, o = (size_t)n * g.Md + m;
+  auto combine = [&](int c) {
+    double2 u[ORDER], acc = make_double2(0.0, 0.0);
+    cpx<R> f[ORDER];
+#pragma unroll
+    for (int j = 0; j < ORDER; ++j) {
+      u[j] = __ldg(reinterpret_cast<const double2*>(P.uin[j]) + c * comp + o);
+      f[j] = static_cast<const cpx<R>*>(P.nin[j])[c * comp + o];
+    }
+#pragma unroll
+    for (int j = 0; j < ORDER; ++j) {
+      acc.x = fma(sp.b[j], widen(f[j].x), fma(sp.a[j], u[j].x, acc.x));
+      acc.y = fma(sp.b[j], widen(f[j].y), fma(sp.a[j], u[j].y, acc.y));
+    }
+    return acc;
+  };
+  double2* out = reinterpret_cast<double2*>(P.scratch) + o;
+  if (blockIdx.z < 3) {
+    const int c = blockIdx.z;
+    out[(c == 0 ? 0 : 3 - c) * comp] = combine(c);
+    return;
+  }
+  for (int c = 0; c < 3; ++c) {
+    double2 a = combine(c);
+    if (c != 1) {
+      a.x += sp.nu * (c == 0 ? P.Ubaseyy : P.Wbaseyy)[(size_t)P.base_stride * fld + n];
+      if (n == 0 && sp.constraint == 0) a.x -= c == 0 ? sp.dPdxRef : sp.dPdzRef;
+    }
+    out[(c == 0 ? 0 : 3 - c) * comp] = a;
+  }
+}
+
+template <typename R>
+static cudaError_t launch_rhs_ms(const GridDev& g, int N, const SolveParams& sp, const SolvePtrs& p, cudaStream_t st) {
+  const dim3 grid((g.Md + 127) / 128, N, 4);
+  switch (sp.order) {
+    case 1: return launch_pdl(k_tau_rhs_ms<R, 1>, grid, dim3(128), 0, st, g, N, sp, p);
+    case 2: return launch_pdl(k_tau_rhs_ms<R, 2>, grid, dim3(128), 0, st, g, N, sp, p);
+    case 3: return launch_pdl(k_tau_rhs_ms<R, 3>, grid, dim3(128), 0, st, g, N, sp, p);
+    case 4: return launch_pdl(k_tau_rhs_ms<R, 4>, grid, dim3(128), 0, st, g, N, sp, p);
+    default: return cudaErrorInvalidValue;
+  }
+}
+
+// ---------------------------------------------------------------------------
+// Right-hand side of the CNAB and RK substeps (NSE::linear and the scheme's combination,
 // nse.cpp:393-477, dnsalgo.cpp:202-253, 641-697, 419-470) for the table-staged
 // solve: one group of four lanes (re/im part, Chebyshev parity) per (mode,
 // component), one component per grid row (blockIdx.y), writing Rx, Ry, Rz to
@@ -829,44 +936,7 @@ __global__ void __launch_bounds__(32, 10) k_tau_rhs(GridDev g, int N, SolveParam
   const size_t fb = (size_t)P.base_stride * fld;
   const double nu = sp.nu;
 
-  // ---- A: right-hand side -------------------------------------------------
-  if (sp.kind == 0) {
-    PLn outx = G(Rxg), outz = G(Rzg);
-    PLn outy = G(Ryg);
-    for (int c = cc; c <= cc; ++c) {
-      for (int i0 = 0; i0 < M; i0 += TCH) {
-        double acc[TCH];
-#pragma unroll
-        for (int k = 0; k < TCH; ++k) acc[k] = 0.0;
-        for (int j = 0; j < sp.order; ++j) {
-          const double* uj = P.uin[j] + c * comp;
-          const R* nj = static_cast<const R*>(P.nin[j]) + c * comp;
-          double uv[TCH], nv[TCH];
-#pragma unroll
-          for (int k = 0; k < TCH; ++k)
-            if (i0 + k < M) {
-              const size_t o = (size_t)(2 * (i0 + k) + q) * row + off;
-              uv[k] = __ldg(uj + o);
-              nv[k] = (double)__ldg(nj + o);
-            }
-#pragma unroll
-          for (int k = 0; k < TCH; ++k)
-            if (i0 + k < M) acc[k] += sp.a[j] * uv[k] + sp.b[j] * nv[k];
-        }
-#pragma unroll
-        for (int k = 0; k < TCH; ++k)
-          if (i0 + k < M) {
-            const int i = i0 + k, n = 2 * i + q;
-            double a = acc[k];
-            if (m00 && part == 0 && c != 1) {
-              a += nu * (c == 0 ? P.Ubaseyy[fb + n] : P.Wbaseyy[fb + n]);
-              if (n == 0 && sp.constraint == 0) a -= (c == 0 ? sp.dPdxRef : sp.dPdzRef);
-            }
-            if (act) (c == 0 ? outx : (c == 1 ? outy : outz))[i] = a;
-          }
-      }
-    }
-  } else {
+  {
     // rows per batch of the streamed lines (two batches in registers: 6 rows when the nonlinear terms are FP64)
     constexpr int RB = sizeof(R) == 8 ? 6 : TCH;
     // per-mode constants from the tables (no FP64 divisions here)
@@ -1358,7 +1428,9 @@ cudaError_t launch_tau_solve(const GridDev& g, int N, const SolveParams& sp, con
     }();
     (void)attr;
     const size_t smem_r = sizeof(double) * (((N + 1) & ~1) + (size_t)M0 * 32);
-    cudaError_t e = launch_pdl(k_tau_rhs<R>, dim3((4 * g.Md + 31) / 32, 3), dim3(32), smem_r, st, g, N, sp, p, tt);
+    const cudaError_t e = sp.kind == 0 ? launch_rhs_ms<R>(g, N, sp, p, st)
+                                       : launch_pdl(k_tau_rhs<R>, dim3((4 * g.Md + 31) / 32, 3), dim3(32), smem_r, st, g,
+                                                    N, sp, p, tt);
     if (e != cudaSuccess) return e;
     return launch_tau_pvuw_seg(g, N, sp, p, hb, tt, st);
   }
@@ -1373,7 +1445,12 @@ cudaError_t launch_tau_solve(const GridDev& g, int N, const SolveParams& sp, con
     }();
     (void)attr;
     const size_t smem_r = sizeof(double) * (((N + 1) & ~1) + (size_t)M0 * 32);
-    k_tau_rhs<R><<<dim3((4 * g.Md + 31) / 32, 3), 32, smem_r, st>>>(g, N, sp, p, tt);
+    if (sp.kind == 0) {
+      const cudaError_t e = launch_rhs_ms<R>(g, N, sp, p, st);
+      if (e != cudaSuccess) return e;
+    } else {
+      k_tau_rhs<R><<<dim3((4 * g.Md + 31) / 32, 3), 32, smem_r, st>>>(g, N, sp, p, tt);
+    }
     k_tau_solve_t<R><<<(4 * g.Md + 31) / 32, 32, smem_t, st>>>(g, N, sp, p, hb, tt);
     const size_t smem_u = sizeof(double) * ((size_t)M0 * 32 + (size_t)4 * N * 4);
     k_tau_uw<R><<<(8 * g.Md + 31) / 32, 32, smem_u, st>>>(g, N, sp, p, hb, tt);
