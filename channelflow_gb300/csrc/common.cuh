@@ -26,7 +26,7 @@
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;\n" ::: "memory"); }
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory"); }
 
-// cfgpu_set_pdl: programmatic dependent launch on (the default) or off for launches made afterwards
+// cfgpu_set_pdl: programmatic dependent launch on or off (the default) for launches made afterwards
 int pdl_enabled();
 
 inline bool pdl_stream(cudaStream_t st) {

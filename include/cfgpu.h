@@ -263,12 +263,12 @@ cfgpu_status cfgpu_set_autotune(int enable);
  * x and z transforms and product as one fused kernel per step (a thread-block cluster per y-plane,
  * distributed shared memory) when the grid allows (Nx, Nz in {32, 48, 64, 96, 128}); otherwise as three
  * kernels. Both give the same results to rounding.  With enable == 1 the fused kernel's launch shapes are
- * timed against the three kernels and the faster kept; enable == 2 keeps the fused kernel wherever the grid
+ * timed against the three kernels and the faster kept (FP64: the three kernels); enable == 2 keeps the fused kernel wherever the grid
  * allows (its shapes still timed), e.g. for profiling runs, whose timings can favour the other form. */
 cfgpu_status cfgpu_set_fused_xz(int enable);
 /* No reference counterpart: programmatic dependent launch between the kernels of a step (a kernel's launch
  * and set-up overlap the previous kernel's tail; it waits for that kernel's results before reading them).
- * On by default; applies to launches made afterwards (a DNS captures its step graphs on its first steps). */
+ * Off by default; applies to launches made afterwards (a DNS captures its step graphs on its first steps). */
 cfgpu_status cfgpu_set_pdl(int enable);
 /* No reference counterpart: the mixed path's rotational z pass in the three-kernel x/z path with
  * register-resident four-step FFTs (enable != 0, the default; Nz in {32, 48, 64, 96, 128}) or with the generic
