@@ -143,6 +143,12 @@ cudaError_t launch_xinv_fx(const GridDev& g, const FftPlan& px, const void* tw, 
 cudaError_t launch_curl_points(const GridDev& g, cpx<double>* W, cudaStream_t st);
 cudaError_t launch_xfwd_fx(const GridDev& g, const FftPlan& px, const void* tw, const cpx<double>* Z, cpx<double>* F,
                            int ncomp, int czc, cudaStream_t st);
+// Whole-FlowField passes, in place: FFT along x of the Mz columns of nplanes planes [x][Mz] (times scale); c2r (inverse)
+// or r2c of nrows rows of Nz + 2 doubles.  One sequence with its copy fits in shared memory: lengths up to 7200.
+cudaError_t launch_field_x(int Nx, int Mz, int nplanes, const FftPlan& px, const void* tw, int sign, double scale,
+                           cpx<double>* data, cudaStream_t st);
+cudaError_t launch_field_z(long long nrows, int Nz, bool inverse, const FftPlan& pz, const void* tw, double* data,
+                           cudaStream_t st);
 cudaError_t launch_zphys_fx(const GridDev& g, int form, const FftPlan& pz, const void* tw, int RP, const cpx<double>* X,
                             cpx<double>* Z, cudaStream_t st);
 

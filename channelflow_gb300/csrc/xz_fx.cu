@@ -395,6 +395,166 @@ __global__ void __launch_bounds__(FX_THREADS) k_zphys_fx(GridDev g, FftPlan pz, 
   }
 }
 
+// ---------------------------------------------------------------------------
+// Whole-FlowField passes (transforms.cu), in place: every mode, Nyquist included.
+// ---------------------------------------------------------------------------
+
+// Complex FFT along x of columns [z0, z0 + cols) of one plane [x][Mz]; plane blockIdx.x, column chunk blockIdx.y.
+__global__ void __launch_bounds__(FX_THREADS) k_field_x(int Nx, int Mz, int cols, FftPlan px, const fxtw* __restrict__ tw,
+                                                        int sign, double scale, double2* __restrict__ data) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  const int ss = Nx + 1, z0 = blockIdx.y * cols, nc = min(cols, Mz - z0);
+  const float invc = 1.0f / nc;
+  fxc* a = reinterpret_cast<fxc*>(smem_raw);
+  fxc* b = a + (size_t)cols * ss;
+  int* sK = reinterpret_cast<int*>(b + (size_t)cols * ss);
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  double2* plane = data + blockIdx.x * (size_t)Nx * Mz + z0;
+#pragma unroll 4
+  for (int i = tid; i < Nx * nc; i += FX_THREADS) {
+    int x, c;
+    divmod_small(i, nc, invc, x, c);
+    const double2 v = plane[(size_t)x * Mz + c];
+    a[c * ss + x] = fxc{__double_as_longlong(v.x), __double_as_longlong(v.y)};
+  }
+  __syncthreads();
+  for (int c = warp; c < nc; c += FX_THREADS / 32) {
+    const int K = fx_scale_column(a + c * ss, Nx, [](int i) { return i; }, lane);
+    if (lane == 0) sK[c] = K;
+  }
+  __syncthreads();
+  const fxc* r = fx_fft(a, b, nc, ss, px, tw, sign, tid, FX_THREADS);
+#pragma unroll 2
+  for (int i = tid; i < Nx * nc; i += FX_THREADS) {
+    int x, c;
+    divmod_small(i, nc, invc, x, c);
+    const fxc v = r[c * ss + x];
+    plane[(size_t)x * Mz + c] = make_double2(fx_double(v.x, sK[c]) * scale, fx_double(v.y, sK[c]) * scale);
+  }
+}
+
+// z transform of x rows, two real rows per complex sequence, with a scale each.  Rows of Nzpad = Nz + 2 doubles;
+// c2r (INV): Nz / 2 + 1 complex in (the imaginary parts of the first and last are not used), Nz reals out, the padding
+// zero; r2c: the reverse.
+template <bool INV>
+__global__ void __launch_bounds__(FX_THREADS) k_field_z(long long nrows, int Nz, int seqs, FftPlan pz,
+                                                        const fxtw* __restrict__ tw, double* __restrict__ data) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  const int ss = Nz + 1, Mz = Nz / 2 + 1, Nzpad = 2 * Mz;
+  fxc* a = reinterpret_cast<fxc*>(smem_raw);
+  fxc* b = a + (size_t)seqs * ss;
+  int* sK = reinterpret_cast<int*>(b + (size_t)seqs * ss);
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const long long row0 = 2ll * seqs * blockIdx.x;
+  const int nr = (int)min((long long)(2 * seqs), nrows - row0), ns = (nr + 1) / 2;  // an odd last row pairs with zeros
+  double* rows = data + row0 * Nzpad;
+  const float invz = 1.0f / Nz, invm = 1.0f / Mz;
+  if (INV) {
+    // bin k < Mz of row 2 s at k, of row 2 s + 1 at Nz - k (the ends: both real parts in one element)
+#pragma unroll 2
+    for (int i = tid; i < ns * Mz; i += FX_THREADS) {
+      int s, k;
+      divmod_small(i, Mz, invm, s, k);
+      const double2 p = reinterpret_cast<const double2*>(rows + (size_t)(2 * s) * Nzpad)[k];
+      const double2 q = 2 * s + 1 < nr ? reinterpret_cast<const double2*>(rows + (size_t)(2 * s + 1) * Nzpad)[k]
+                                       : make_double2(0, 0);
+      fxc* sq = a + (size_t)s * ss;
+      if (k == 0 || 2 * k == Nz) {
+        sq[k] = fxc{__double_as_longlong(p.x), __double_as_longlong(q.x)};
+      } else {
+        sq[k] = fxc{__double_as_longlong(p.x), __double_as_longlong(p.y)};
+        sq[Nz - k] = fxc{__double_as_longlong(q.x), __double_as_longlong(q.y)};
+      }
+    }
+  } else {
+#pragma unroll 2
+    for (int i = tid; i < ns * Nz; i += FX_THREADS) {
+      int s, z;
+      divmod_small(i, Nz, invz, s, z);
+      const double p = rows[(size_t)(2 * s) * Nzpad + z];
+      const double q = 2 * s + 1 < nr ? rows[(size_t)(2 * s + 1) * Nzpad + z] : 0.0;
+      a[(size_t)s * ss + z] = fxc{__double_as_longlong(p), __double_as_longlong(q)};
+    }
+  }
+  __syncthreads();
+  for (int s = warp; s < ns; s += FX_THREADS / 32) {
+    fxc* sq = a + (size_t)s * ss;
+    const int n = INV ? Mz : Nz;
+    // raw values of element i: row 0's in p, row 1's in q; ends: real values only
+    auto get = [&](int i, double (&p)[2], double (&q)[2]) {
+      const fxc v = sq[i];
+      const bool real = !INV || i == 0 || 2 * i == Nz;
+      const fxc w = real ? fxc{v.y, 0} : sq[Nz - i];
+      p[0] = fx_raw(v.x);
+      p[1] = real ? 0.0 : fx_raw(v.y);
+      q[0] = fx_raw(w.x);
+      q[1] = real ? 0.0 : fx_raw(w.y);
+    };
+    unsigned ka = 0, kb = 0;
+    for (int i = lane; i < n; i += 32) {
+      double p[2], q[2];
+      get(i, p, q);
+      ka = max(ka, max(fx_key(p[0]), fx_key(p[1])));
+      kb = max(kb, max(fx_key(q[0]), fx_key(q[1])));
+    }
+    ka = __reduce_max_sync(0xffffffffu, ka);
+    kb = __reduce_max_sync(0xffffffffu, kb);
+    const int ea = fx_exp_of_key(ka), eb = fx_exp_of_key(kb);
+    unsigned Sa = 0, Sb = 0;  // a c2r coefficient appears twice in the sequence
+    for (int i = lane; i < n; i += 32) {
+      double p[2], q[2];
+      get(i, p, q);
+      Sa += fx_mag(p[0], ea) + fx_mag(p[1], ea);
+      Sb += fx_mag(q[0], eb) + fx_mag(q[1], eb);
+    }
+    Sa = __reduce_add_sync(0xffffffffu, Sa) * (INV ? 2 : 1);
+    Sb = __reduce_add_sync(0xffffffffu, Sb) * (INV ? 2 : 1);
+    const int Ka = fx_line_K(ea, Sa, 60), Kb = fx_line_K(eb, Sb, 60);
+    for (int i = lane; i < n; i += 32) {
+      double p[2], q[2];
+      get(i, p, q);
+      const long long ax = ka ? fx_quant(p[0], Ka) : 0, ay = ka ? fx_quant(p[1], Ka) : 0;
+      const long long bx = kb ? fx_quant(q[0], Kb) : 0, by = kb ? fx_quant(q[1], Kb) : 0;
+      if (!INV || i == 0 || 2 * i == Nz) {
+        sq[i] = fxc{ax, bx};
+      } else {
+        sq[i] = fxc{ax - by, ay + bx};       // A_k + i B_k
+        sq[Nz - i] = fxc{ax + by, bx - ay};  // conj(A_k) + i conj(B_k)
+      }
+    }
+    if (lane == 0) {
+      sK[2 * s] = ka == 0 ? FX_ZERO : (ea == 2047 ? FX_NAN : Ka);
+      sK[2 * s + 1] = kb == 0 ? FX_ZERO : (eb == 2047 ? FX_NAN : Kb);
+    }
+  }
+  __syncthreads();
+  const fxc* G = fx_fft(a, b, ns, ss, pz, tw, INV ? +1 : -1, tid, FX_THREADS);
+  if (INV) {
+#pragma unroll 2
+    for (int i = tid; i < ns * Nz; i += FX_THREADS) {
+      int s, z;
+      divmod_small(i, Nz, invz, s, z);
+      const fxc v = G[(size_t)s * ss + z];
+      rows[(size_t)(2 * s) * Nzpad + z] = fx_double(v.x, sK[2 * s]);
+      if (2 * s + 1 < nr) rows[(size_t)(2 * s + 1) * Nzpad + z] = fx_double(v.y, sK[2 * s + 1]);
+    }
+    for (int i = tid; i < 2 * nr; i += FX_THREADS) rows[(size_t)(i >> 1) * Nzpad + Nz + (i & 1)] = 0.0;
+  } else {
+#pragma unroll 2
+    for (int i = tid; i < ns * Mz; i += FX_THREADS) {
+      int s, k;
+      divmod_small(i, Mz, invm, s, k);
+      const fxc zk = G[(size_t)s * ss + k], zm = G[(size_t)s * ss + (k == 0 ? 0 : Nz - k)];
+      const int K0 = sK[2 * s] + 1, K1 = sK[2 * s + 1] + 1;  // + 1: half the sum
+      reinterpret_cast<double2*>(rows + (size_t)(2 * s) * Nzpad)[k] =
+          make_double2(fx_double(zk.x + zm.x, K0), fx_double(zk.y - zm.y, K0));
+      if (2 * s + 1 < nr)
+        reinterpret_cast<double2*>(rows + (size_t)(2 * s + 1) * Nzpad)[k] =
+            make_double2(fx_double(zk.y + zm.y, K1), fx_double(zm.x - zk.x, K1));
+    }
+  }
+}
+
 template <int FORM>
 cudaError_t run_zphys_fx(const GridDev& g, const FftPlan& pz, const fxtw* tw, int RP, const double2* X, double2* Z,
                          cudaStream_t st) {
@@ -420,6 +580,41 @@ std::vector<int> fx_twiddles(const std::vector<std::complex<long double>>& tw) {
     fx_split(tw[i].imag(), t[4 * i + 2], t[4 * i + 3]);
   }
   return t;
+}
+
+// Shared memory of n sequences of length L with their exponents (two per sequence).
+static size_t field_smem(int L, int n) { return (2 * sizeof(fxc) * (size_t)(L + 1) + 2 * sizeof(int)) * n; }
+
+cudaError_t launch_field_x(int Nx, int Mz, int nplanes, const FftPlan& px, const void* tw, int sign, double scale,
+                           cpx<double>* data, cudaStream_t st) {
+  static const bool attr = [] {
+    cudaFuncSetAttribute(k_field_x, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
+    return true;
+  }();
+  (void)attr;
+  int cols = 1;  // about 64 KB of columns: three blocks an SM
+  while (cols < Mz && cols < 16 && field_smem(Nx, cols + 1) <= 64 * 1024) ++cols;
+  k_field_x<<<dim3(nplanes, (Mz + cols - 1) / cols), FX_THREADS, field_smem(Nx, cols), st>>>(Nx, Mz, cols, px, (const fxtw*)tw,
+                                                                                             sign, scale, (double2*)data);
+  return cudaGetLastError();
+}
+
+cudaError_t launch_field_z(long long nrows, int Nz, bool inverse, const FftPlan& pz, const void* tw, double* data,
+                           cudaStream_t st) {
+  static const bool attr = [] {
+    cudaFuncSetAttribute(k_field_z<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
+    cudaFuncSetAttribute(k_field_z<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
+    return true;
+  }();
+  (void)attr;
+  int seqs = 1;
+  while (seqs < 16 && field_smem(Nz, seqs + 1) <= 64 * 1024) ++seqs;
+  const unsigned nb = (unsigned)((nrows + 2 * seqs - 1) / (2 * seqs));
+  if (inverse)
+    k_field_z<true><<<nb, FX_THREADS, field_smem(Nz, seqs), st>>>(nrows, Nz, seqs, pz, (const fxtw*)tw, data);
+  else
+    k_field_z<false><<<nb, FX_THREADS, field_smem(Nz, seqs), st>>>(nrows, Nz, seqs, pz, (const fxtw*)tw, data);
+  return cudaGetLastError();
 }
 
 cudaError_t launch_xinv_fx(const GridDev& g, const FftPlan& px, const void* tw, const cpx<double>* W, cpx<double>* X,
