@@ -625,7 +625,7 @@ struct cfgpu_dns_s {
   // transforms
   FftPlan px{}, pz{};
   void *twx = nullptr, *twz = nullptr;  // R-typed complex
-  void *twxq = nullptr, *twzq = nullptr;  // FP64: the same as fixed-point splits (fx_twiddles)
+  void *twxq = nullptr, *twzq = nullptr;  // FP64: fixed-point tables (fx_twiddles)
   // FP64 Chebyshev transforms on the tensor cores (cheb_oz.cu): tables in one block, off where Ny is not covered
   bool oz = false;
   OzTables ozt{};
@@ -1993,8 +1993,8 @@ int dns_create_impl(cfgpu_dns d, const cfgpu_grid* grid, const cfgpu_flags* flag
   if (fp64) {
     CKS(upload_tw<double>(twx, &d->twx, B, d->st));
     CKS(upload_tw<double>(twz, &d->twz, B, d->st));
-    CKS(upload_ints(fx_twiddles(twx), &d->twxq, B, d->st));
-    CKS(upload_ints(fx_twiddles(twz), &d->twzq, B, d->st));
+    CKS(upload_ints(fx_twiddles(Nx), &d->twxq, B, d->st));
+    CKS(upload_ints(fx_twiddles(Nz), &d->twzq, B, d->st));
     CKS(upload_as<double>(circx, &d->twxf, B, d->st));
     CKS(upload_as<double>(circz, &d->twzf, B, d->st));
     CKS(upload_as<double>(cm.invA, &d->cinvA, B, d->st));

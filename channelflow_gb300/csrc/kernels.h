@@ -99,7 +99,7 @@ size_t zphys_smem_bytes(const GridDev& g, int form, int RP);
 // z pass of the x/z path (c2r, the form's products, r2c).  With twzf (the full-circle twiddle table
 // exp(-2 pi i e / Nz), e < Nz) the FP32 rotational form runs with register-resident FFTs where Nz allows
 // (launch_zrot, csrc/z_reg.cu), else the generic Stockham kernel.  FP64 runs on 64-bit integers (csrc/xz_fx.cu) with
-// the twiddles twq = fx_twiddles of the plan's table; twz is unused there.
+// the twiddles twq = fx_twiddles(Nz); twz is unused there.
 template <typename R>
 cudaError_t launch_zphys(const GridDev& g, int form, const FftPlan& pz, const cpx<R>* twz, const void* twq, int RP,
                          const cpx<R>* X, cpx<R>* Z, cudaStream_t st, const Dither& dt = kNoDither,
@@ -135,8 +135,8 @@ template <typename R>
 cudaError_t launch_xfwd(const GridDev& g, const FftPlan& px, const cpx<R>* twx, const void* twq, const cpx<R>* Z,
                         cpx<R>* F, int ncomp, cudaStream_t st, int czc = 0, const Dither& dt = kNoDither);
 
-// The FP64 passes on 64-bit integers (xz_fx.cu): fx_twiddles splits a plan's twiddle table (four ints per entry).
-std::vector<int> fx_twiddles(const std::vector<std::complex<long double>>& tw);
+// The FP64 passes on 64-bit integers (xz_fx.cu): fx_twiddles is the table of a length (four ints per entry).
+std::vector<int> fx_twiddles(int L);
 // curl: W holds u, v, w, dw/dy, -, du/dy; components 3, 4, 5 transformed are the vorticity (launch_curl_points: in place)
 cudaError_t launch_xinv_fx(const GridDev& g, const FftPlan& px, const void* tw, const cpx<double>* W, cpx<double>* X,
                            int ncomp, int czc, bool curl, cudaStream_t st);
@@ -145,9 +145,9 @@ cudaError_t launch_xfwd_fx(const GridDev& g, const FftPlan& px, const void* tw, 
                            int ncomp, int czc, cudaStream_t st);
 // Whole-FlowField passes, in place: FFT along x of the Mz columns of nplanes planes [x][Mz] (times scale); c2r (inverse)
 // or r2c of nrows rows of Nz + 2 doubles.  One sequence with its copy fits in shared memory: lengths up to 7200.
-cudaError_t launch_field_x(int Nx, int Mz, int nplanes, const FftPlan& px, const void* tw, int sign, double scale,
+cudaError_t launch_field_x(int Nx, int Mz, int nplanes, const void* tw, int sign, double scale,
                            cpx<double>* data, cudaStream_t st);
-cudaError_t launch_field_z(long long nrows, int Nz, bool inverse, const FftPlan& pz, const void* tw, double* data,
+cudaError_t launch_field_z(long long nrows, int Nz, bool inverse, const void* tw, double* data,
                            cudaStream_t st);
 cudaError_t launch_zphys_fx(const GridDev& g, int form, const FftPlan& pz, const void* tw, int RP, const cpx<double>* X,
                             cpx<double>* Z, cudaStream_t st);

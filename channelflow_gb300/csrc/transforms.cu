@@ -106,7 +106,6 @@ struct cfgpu_flowfield_s {
   double* Minv = nullptr;  // [j][n] ichebyfft
   int* twx = nullptr;  // fx_twiddles
   int* twz = nullptr;
-  FftPlan px{}, pz{};
   cudaStream_t st = nullptr;
 };
 
@@ -151,11 +150,11 @@ int xz_transform(cfgpu_flowfield f, bool to_spectral) {
   if (f->Nx > TF_MAX || f->Nz > TF_MAX) return tf_fail(CFGPU_ENOTSUP, "Nx or Nz too large for the shared-memory FFT");
   cpx<double>* cd = reinterpret_cast<cpx<double>*>(f->data);
   if (to_spectral) {
-    TF_CK(launch_field_z(rows, f->Nz, false, f->pz, f->twz, f->data, f->st));
-    TF_CK(launch_field_x(f->Nx, Mz, planes, f->px, f->twx, -1, 1.0 / ((double)f->Nx * f->Nz), cd, f->st));
+    TF_CK(launch_field_z(rows, f->Nz, false, f->twz, f->data, f->st));
+    TF_CK(launch_field_x(f->Nx, Mz, planes, f->twx, -1, 1.0 / ((double)f->Nx * f->Nz), cd, f->st));
   } else {
-    TF_CK(launch_field_x(f->Nx, Mz, planes, f->px, f->twx, +1, 1.0, cd, f->st));
-    TF_CK(launch_field_z(rows, f->Nz, true, f->pz, f->twz, f->data, f->st));
+    TF_CK(launch_field_x(f->Nx, Mz, planes, f->twx, +1, 1.0, cd, f->st));
+    TF_CK(launch_field_z(rows, f->Nz, true, f->twz, f->data, f->st));
   }
   return CFGPU_OK;
 }
@@ -188,9 +187,10 @@ cfgpu_status cfgpu_flowfield_create(const cfgpu_grid* g, int Nd, cfgpu_flowfield
   f->a = g->a;
   f->b = g->b;
   f->n = (size_t)Nd * g->Ny * g->Nx * 2 * (g->Nz / 2 + 1);
-  std::vector<std::complex<long double>> twx, twz;
+  std::vector<std::complex<long double>> tw;
+  FftPlan plan{};
   int st = CFGPU_OK;
-  if (!cfgpu_fft_plan(g->Nx, f->px, twx) || !cfgpu_fft_plan(g->Nz, f->pz, twz))
+  if (!cfgpu_fft_plan(g->Nx, plan, tw) || !cfgpu_fft_plan(g->Nz, plan, tw))
     st = tf_fail(CFGPU_ENOTSUP, "Nx and Nz must factor into primes <= " + std::to_string(FFT_MAX_RADIX));
   if (st == CFGPU_OK && cudaStreamCreateWithFlags(&f->st, cudaStreamNonBlocking) != cudaSuccess)
     st = tf_fail(CFGPU_ECUDA, "cudaStreamCreate failed");
@@ -231,7 +231,7 @@ cfgpu_status cfgpu_flowfield_create(const cfgpu_grid* g, int Nd, cfgpu_flowfield
       if (st == CFGPU_OK) st = tf_upload(Mf, &f->Mfwd, f->st);
       if (st == CFGPU_OK) st = tf_upload(Mi, &f->Minv, f->st);
     }
-    const std::vector<int> tx = fx_twiddles(twx), tz = fx_twiddles(twz);
+    const std::vector<int> tx = fx_twiddles(f->Nx), tz = fx_twiddles(f->Nz);
     if (st == CFGPU_OK) st = tf_upload(tx, &f->twx, f->st);
     if (st == CFGPU_OK) st = tf_upload(tz, &f->twz, f->st);
     // the host vectors go out of scope: wait for the copies

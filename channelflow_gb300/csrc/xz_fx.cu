@@ -5,12 +5,51 @@
 // Every line is scaled on its own: a column of the x passes, each real row of the z pass (two rows share a complex
 // sequence, with a scale each).
 //
-// Measured at 128x97x128 against the same passes in FP64 arithmetic, which the FP64 pipe bounds (one warp instruction
-// per 64 cycles): z pass 340 -> 123 us, x inverse 134 -> 55 us, x forward 76 -> 29 us; bound here by integer issue.
+// Measured against the same passes in FP64 arithmetic, which the FP64 pipe bounds (one warp instruction per 64 cycles),
+// at 128x97x128: z pass 340 -> 116 us, x inverse 134 -> 55 us (65 us with the vorticity formed in it), x forward 76 -> 29
+// us; 192x129x160: z pass 1138 -> 353 us; bound here by integer issue.  Against radices 4, 2, 3, 5 alone: z pass 123 ->
+// 116 us at 128x97x128, 402 -> 353 us at 192x129x160, 170 -> 143 us at 72x57x90 (skew-symmetric form).
 // Relative error of N(u) against extended precision: 1.5e-16 ... 2.5e-16 at 32x9x32 (FP64 arithmetic 2.7e-16 ...
 // 8.8e-16), for spectra from 0.5^(|kx|+|kz|) to flat.
-#include "fx.cuh"
+#include <algorithm>
+#include <atomic>
+#include <cmath>
+
+#include "fx_fft.cuh"
 #include "kernels.h"
+
+// Fewest stages, then the smallest radices, largest first; primes above 5 last.
+static void fx_search(int m, int maxr, unsigned long long cur, int n, int sum, int& bn, int& bsum, unsigned long long& best) {
+  if (m == 1) {
+    if (n < bn || (n == bn && sum < bsum)) {
+      bn = n;
+      bsum = sum;
+      best = cur;
+    }
+    return;
+  }
+  if (n + 1 > bn) return;
+  for (int r = std::min(maxr, m); r >= 2; --r)
+    if (m % r == 0 && fx_composite(r)) fx_search(m / r, r, cur | (unsigned long long)r << (8 * n), n + 1, sum + r, bn, bsum, best);
+}
+
+static FxPlan fx_plan(int L) {
+  static std::atomic<unsigned long long> known[8192];  // a function of L alone
+  if (L < 8192)
+    if (const unsigned long long k = known[L].load(std::memory_order_relaxed)) return FxPlan{L, k};
+  int m = L, np = 0, primes[8];
+  for (int p = 7; p <= m; p += 2)
+    while (m % p == 0 && p % 3 && p % 5) {
+      primes[np++] = p;
+      m /= p;
+    }
+  int bn = 8, bsum = 0;
+  unsigned long long best = 0;
+  fx_search(m, 8, 0, 0, 0, bn, bsum, best);
+  for (int i = 0; i < np; ++i) best |= (unsigned long long)primes[i] << (8 * (bn + i));
+  if (L < 8192) known[L].store(best, std::memory_order_relaxed);
+  return FxPlan{L, best};
+}
 
 namespace {
 
@@ -65,7 +104,7 @@ __global__ void k_curl_points(GridDev g, double2* W) {
   for (int c = 3; c < 6; ++c) w[c * cs] = fx_vorticity(c, w, cs, kx, kz);
 }
 
-__global__ void __launch_bounds__(FX_THREADS) k_xinv_fx(GridDev g, FftPlan px, const fxtw* __restrict__ tw,
+__global__ void __launch_bounds__(FX_THREADS, 4) k_xinv_fx(GridDev g, FxPlan px, const fxtw* __restrict__ tw,
                                                         const double2* __restrict__ W, double2* __restrict__ X, int czc,
                                                         int curl) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -111,7 +150,7 @@ __global__ void __launch_bounds__(FX_THREADS) k_xinv_fx(GridDev g, FftPlan px, c
     if (lane == 0) sK[jz] = K;
   }
   __syncthreads();
-  const fxc* r = fx_fft(a, b, nc, ss, px, tw, +1, tid, FX_THREADS);
+  const fxc* r = a + fx_fft(0, czc * ss, nc, ss, px.L, px.rad, tw, true);
   double2* dst = X + ((size_t)c * g.Ny + ny) * (size_t)Nx * g.NKz;
   for (int i = tid; i < Nx * nc; i += FX_THREADS) {
     int x, jz;
@@ -122,7 +161,7 @@ __global__ void __launch_bounds__(FX_THREADS) k_xinv_fx(GridDev g, FftPlan px, c
   }
 }
 
-__global__ void __launch_bounds__(FX_THREADS) k_xfwd_fx(GridDev g, FftPlan px, const fxtw* __restrict__ tw,
+__global__ void __launch_bounds__(FX_THREADS, 4) k_xfwd_fx(GridDev g, FxPlan px, const fxtw* __restrict__ tw,
                                                         const double2* __restrict__ Z, double2* __restrict__ F,
                                                         double scale, int czc) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -149,7 +188,7 @@ __global__ void __launch_bounds__(FX_THREADS) k_xfwd_fx(GridDev g, FftPlan px, c
     if (lane == 0) sK[jz] = K;
   }
   __syncthreads();
-  const fxc* r = fx_fft(a, b, nc, ss, px, tw, -1, tid, FX_THREADS);
+  const fxc* r = a + fx_fft(0, czc * ss, nc, ss, px.L, px.rad, tw, false);
   double2* dst = F + ((size_t)c * g.Ny + ny) * g.Md;
 #pragma unroll 4
   for (int i = tid; i < g.NKx * nc; i += FX_THREADS) {
@@ -204,7 +243,7 @@ __device__ __forceinline__ long long fx_round_shift(long long v, int s) {  // v 
 }
 
 template <int FORM>
-__global__ void __launch_bounds__(FX_THREADS) k_zphys_fx(GridDev g, FftPlan pz, const fxtw* __restrict__ tw, int RP,
+__global__ void __launch_bounds__(FX_THREADS, 4) k_zphys_fx(GridDev g, FxPlan pz, const fxtw* __restrict__ tw, int RP,
                                                          const double2* __restrict__ X, double2* __restrict__ Z) {
   constexpr int NC = FxForm<FORM>::NC, NO = FxForm<FORM>::NO;
   extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -300,7 +339,7 @@ __global__ void __launch_bounds__(FX_THREADS) k_zphys_fx(GridDev g, FftPlan pz, 
     }
   }
   __syncthreads();
-  fxc* P = fx_fft(A, B, ninv, ss, pz, tw, +1, tid, FX_THREADS);
+  fxc* P = A + fx_fft(0, nseq * ss, ninv, ss, pz.L, pz.rad, tw, true);
   fxc* Q = P == A ? B : A;
   // normalise every component by its largest value: the scale above allows for the sum of magnitudes
   for (int s = warp; s < ninv; s += FX_THREADS / 32) {
@@ -344,7 +383,7 @@ __global__ void __launch_bounds__(FX_THREADS) k_zphys_fx(GridDev g, FftPlan pz, 
 #pragma unroll
       for (int t = 0; t < MT; ++t)
         if (t < fx_nterm<FORM>(o)) {
-          const long long p = __mul64hi(c[fx_term<FORM>(o, t).a], c[fx_term<FORM>(o, t).b]) >> min(kt[t] - km, 63);
+          const long long p = fx_mulhi(c[fx_term<FORM>(o, t).a], c[fx_term<FORM>(o, t).b]) >> min(kt[t] - km, 63);
           f = fx_term<FORM>(o, t).sub ? f - p : f + p;
         }
       const int k = r * NO + o;
@@ -376,7 +415,7 @@ __global__ void __launch_bounds__(FX_THREADS) k_zphys_fx(GridDev g, FftPlan pz, 
     }
   }
   __syncthreads();
-  const fxc* G = fx_fft(Q, P, nfwd, ss, pz, tw, -1, tid, FX_THREADS);
+  const fxc* G = A + fx_fft((int)(Q - A), (int)(P - A), nfwd, ss, pz.L, pz.rad, tw, false);
 #pragma unroll 2
   for (int i = tid; i < nfwd * NKz; i += FX_THREADS) {
     int s, iz;
@@ -400,7 +439,7 @@ __global__ void __launch_bounds__(FX_THREADS) k_zphys_fx(GridDev g, FftPlan pz, 
 // ---------------------------------------------------------------------------
 
 // Complex FFT along x of columns [z0, z0 + cols) of one plane [x][Mz]; plane blockIdx.x, column chunk blockIdx.y.
-__global__ void __launch_bounds__(FX_THREADS) k_field_x(int Nx, int Mz, int cols, FftPlan px, const fxtw* __restrict__ tw,
+__global__ void __launch_bounds__(FX_THREADS, 4) k_field_x(int Nx, int Mz, int cols, FxPlan px, const fxtw* __restrict__ tw,
                                                         int sign, double scale, double2* __restrict__ data) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const int ss = Nx + 1, z0 = blockIdx.y * cols, nc = min(cols, Mz - z0);
@@ -423,7 +462,7 @@ __global__ void __launch_bounds__(FX_THREADS) k_field_x(int Nx, int Mz, int cols
     if (lane == 0) sK[c] = K;
   }
   __syncthreads();
-  const fxc* r = fx_fft(a, b, nc, ss, px, tw, sign, tid, FX_THREADS);
+  const fxc* r = a + fx_fft(0, cols * ss, nc, ss, px.L, px.rad, tw, sign > 0);
 #pragma unroll 2
   for (int i = tid; i < Nx * nc; i += FX_THREADS) {
     int x, c;
@@ -437,7 +476,7 @@ __global__ void __launch_bounds__(FX_THREADS) k_field_x(int Nx, int Mz, int cols
 // c2r (INV): Nz / 2 + 1 complex in (the imaginary parts of the first and last are not used), Nz reals out, the padding
 // zero; r2c: the reverse.
 template <bool INV>
-__global__ void __launch_bounds__(FX_THREADS) k_field_z(long long nrows, int Nz, int seqs, FftPlan pz,
+__global__ void __launch_bounds__(FX_THREADS, 4) k_field_z(long long nrows, int Nz, int seqs, FxPlan pz,
                                                         const fxtw* __restrict__ tw, double* __restrict__ data) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const int ss = Nz + 1, Mz = Nz / 2 + 1, Nzpad = 2 * Mz;
@@ -528,7 +567,7 @@ __global__ void __launch_bounds__(FX_THREADS) k_field_z(long long nrows, int Nz,
     }
   }
   __syncthreads();
-  const fxc* G = fx_fft(a, b, ns, ss, pz, tw, INV ? +1 : -1, tid, FX_THREADS);
+  const fxc* G = a + fx_fft(0, seqs * ss, ns, ss, pz.L, pz.rad, tw, INV);
   if (INV) {
 #pragma unroll 2
     for (int i = tid; i < ns * Nz; i += FX_THREADS) {
@@ -564,7 +603,7 @@ cudaError_t run_zphys_fx(const GridDev& g, const FftPlan& pz, const fxtw* tw, in
   }();
   (void)attr;
   return launch_pdl(k_zphys_fx<FORM>, dim3((g.Nx + RP - 1) / RP, g.Ny), dim3(FX_THREADS),
-                    zphys_smem_bytes<double>(g, FORM, RP), st, g, pz, tw, RP, X, Z);
+                    zphys_smem_bytes<double>(g, FORM, RP), st, g, fx_plan(pz.L), tw, RP, X, Z);
 }
 
 size_t xfx_smem(const GridDev& g, int czc, bool curl) {
@@ -573,19 +612,34 @@ size_t xfx_smem(const GridDev& g, int czc, bool curl) {
 
 }  // namespace
 
-std::vector<int> fx_twiddles(const std::vector<std::complex<long double>>& tw) {
-  std::vector<int> t(4 * (tw.empty() ? 1 : tw.size()), 0);
-  for (size_t i = 0; i < tw.size(); ++i) {
-    fx_split(tw[i].real(), t[4 * i], t[4 * i + 1]);
-    fx_split(tw[i].imag(), t[4 * i + 2], t[4 * i + 3]);
+// Per stage: exp(-2 pi i k r / (Ns R)) at [k (R - 1) + r - 1], then a prime's roots exp(-2 pi i e / R).
+std::vector<int> fx_twiddles(int L) {
+  std::vector<int> t;
+  auto push = [&](long long m, long long n) {
+    const long double x = 2 * 3.14159265358979323846264338327950288L * (long double)(m % n) / (long double)n;
+    const bool cz = 4 * (m % n) == n || 4 * (m % n) == 3 * n, sz = 2 * (m % n) % n == 0;
+    int v[4];
+    fx_split(cz ? 0.0L : cosl(x), v[0], v[1]);
+    fx_split(sz ? 0.0L : -sinl(x), v[2], v[3]);
+    t.insert(t.end(), v, v + 4);
+  };
+  unsigned long long rad = fx_plan(L).rad;
+  for (int Ns = 1; Ns < L; rad >>= 8) {
+    const int R = (int)(rad & 255);
+    for (int k = 0; k < Ns; ++k)
+      for (int r = 1; r < R; ++r) push((long long)k * r, (long long)Ns * R);
+    if (!fx_composite(R))
+      for (int e = 0; e < R; ++e) push(e, R);
+    Ns *= R;
   }
+  if (t.empty()) t.resize(4);
   return t;
 }
 
 // Shared memory of n sequences of length L with their exponents (two per sequence).
 static size_t field_smem(int L, int n) { return (2 * sizeof(fxc) * (size_t)(L + 1) + 2 * sizeof(int)) * n; }
 
-cudaError_t launch_field_x(int Nx, int Mz, int nplanes, const FftPlan& px, const void* tw, int sign, double scale,
+cudaError_t launch_field_x(int Nx, int Mz, int nplanes, const void* tw, int sign, double scale,
                            cpx<double>* data, cudaStream_t st) {
   static const bool attr = [] {
     cudaFuncSetAttribute(k_field_x, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
@@ -594,12 +648,12 @@ cudaError_t launch_field_x(int Nx, int Mz, int nplanes, const FftPlan& px, const
   (void)attr;
   int cols = 1;  // about 64 KB of columns: three blocks an SM
   while (cols < Mz && cols < 16 && field_smem(Nx, cols + 1) <= 64 * 1024) ++cols;
-  k_field_x<<<dim3(nplanes, (Mz + cols - 1) / cols), FX_THREADS, field_smem(Nx, cols), st>>>(Nx, Mz, cols, px, (const fxtw*)tw,
+  k_field_x<<<dim3(nplanes, (Mz + cols - 1) / cols), FX_THREADS, field_smem(Nx, cols), st>>>(Nx, Mz, cols, fx_plan(Nx), (const fxtw*)tw,
                                                                                              sign, scale, (double2*)data);
   return cudaGetLastError();
 }
 
-cudaError_t launch_field_z(long long nrows, int Nz, bool inverse, const FftPlan& pz, const void* tw, double* data,
+cudaError_t launch_field_z(long long nrows, int Nz, bool inverse, const void* tw, double* data,
                            cudaStream_t st) {
   static const bool attr = [] {
     cudaFuncSetAttribute(k_field_z<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
@@ -611,9 +665,9 @@ cudaError_t launch_field_z(long long nrows, int Nz, bool inverse, const FftPlan&
   while (seqs < 16 && field_smem(Nz, seqs + 1) <= 64 * 1024) ++seqs;
   const unsigned nb = (unsigned)((nrows + 2 * seqs - 1) / (2 * seqs));
   if (inverse)
-    k_field_z<true><<<nb, FX_THREADS, field_smem(Nz, seqs), st>>>(nrows, Nz, seqs, pz, (const fxtw*)tw, data);
+    k_field_z<true><<<nb, FX_THREADS, field_smem(Nz, seqs), st>>>(nrows, Nz, seqs, fx_plan(Nz), (const fxtw*)tw, data);
   else
-    k_field_z<false><<<nb, FX_THREADS, field_smem(Nz, seqs), st>>>(nrows, Nz, seqs, pz, (const fxtw*)tw, data);
+    k_field_z<false><<<nb, FX_THREADS, field_smem(Nz, seqs), st>>>(nrows, Nz, seqs, fx_plan(Nz), (const fxtw*)tw, data);
   return cudaGetLastError();
 }
 
@@ -629,7 +683,7 @@ cudaError_t launch_xinv_fx(const GridDev& g, const FftPlan& px, const void* tw, 
     if (e != cudaSuccess) return e;
     curl = false;
   }
-  return launch_pdl(k_xinv_fx, dim3(g.Ny, ncomp, (g.NKz + czc - 1) / czc), dim3(FX_THREADS), xfx_smem(g, czc, curl), st, g, px,
+  return launch_pdl(k_xinv_fx, dim3(g.Ny, ncomp, (g.NKz + czc - 1) / czc), dim3(FX_THREADS), xfx_smem(g, czc, curl), st, g, fx_plan(px.L),
                     (const fxtw*)tw, (const double2*)W, (double2*)X, czc, (int)curl);
 }
 
@@ -646,7 +700,7 @@ cudaError_t launch_xfwd_fx(const GridDev& g, const FftPlan& px, const void* tw, 
   }();
   (void)attr;
   const double scale = 1.0 / ((double)g.Nx * (double)g.Nz);
-  return launch_pdl(k_xfwd_fx, dim3(g.Ny, ncomp, (g.NKz + czc - 1) / czc), dim3(FX_THREADS), xfx_smem(g, czc, false), st, g, px,
+  return launch_pdl(k_xfwd_fx, dim3(g.Ny, ncomp, (g.NKz + czc - 1) / czc), dim3(FX_THREADS), xfx_smem(g, czc, false), st, g, fx_plan(px.L),
                     (const fxtw*)tw, (const double2*)Z, (double2*)F, scale, czc);
 }
 

@@ -14,7 +14,9 @@ TOL = 1000 * np.finfo(float).eps
 # lengths around the compile-time ones, every radix (2, 3, 4, 5, 7, 11, 13), single solved wavenumbers, row counts
 # that leave the last block of the z pass ragged
 GRIDS = [(4, 9, 6), (6, 9, 4), (10, 9, 32), (30, 9, 22), (34, 9, 26), (50, 9, 28), (64, 17, 96), (128, 9, 10), (14, 9, 128),
-         (160, 9, 48)]
+         (160, 9, 48),
+         # radices 6, 8, 9, 10, 12, 15, 16, single stages, three stages, a prime behind a composite
+         (144, 9, 8), (8, 9, 192), (90, 9, 72), (36, 9, 150), (256, 9, 12), (16, 9, 270), (224, 9, 14)]
 
 
 @pytest.fixture(autouse=True)
