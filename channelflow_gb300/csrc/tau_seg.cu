@@ -176,8 +176,8 @@ __device__ __forceinline__ void store_lines(double* dst, int Md, int mbase, int 
 // right-hand sides Rx, Rz, Ry in scratch lines 0, 1, 2; writes q and v.  One warp: two modes (lanes 16 ml +
 // 8 part + 4 q + s).
 // ---------------------------------------------------------------------------
-template <int L>
-__global__ void __launch_bounds__(32, 12) k_tau_pv_seg(GridDev g, int N, SolveParams sp, SolvePtrs P, HelmB hb,
+template <int L, int WARPS>  // at least WARPS warps an SM
+__global__ void __launch_bounds__(32, WARPS) k_tau_pv_seg(GridDev g, int N, SolveParams sp, SolvePtrs P, HelmB hb,
                                                    TauTable tt) {
   extern __shared__ double sm[];
   pdl_wait();
@@ -313,8 +313,9 @@ __global__ void __launch_bounds__(32, 12) k_tau_pv_seg(GridDev g, int N, SolvePa
 // solve of the (0,0) mode's real part under the bulk-velocity constraint) from q and Rx, Rz.  One warp: one
 // mode, u (lanes 0-15) and w (16-31).
 // ---------------------------------------------------------------------------
+// Warps an SM against registers: beyond 12 rows a lane, 16 warps spill (97 rows: 52 us, 12 warps 44, 10 warps 41).
 template <int L>
-__global__ void __launch_bounds__(32, 16) k_tau_uw_seg(GridDev g, int N, SolveParams sp, SolvePtrs P, HelmB hb,
+__global__ void __launch_bounds__(32, L >= 10 ? 10 : (L == 9 ? 12 : 16)) k_tau_uw_seg(GridDev g, int N, SolveParams sp, SolvePtrs P, HelmB hb,
                                                    TauTable tt) {
   extern __shared__ double sm[];
   pdl_wait();
@@ -402,12 +403,22 @@ cudaError_t run_seg(const GridDev& g, int N, const SolveParams& sp, const SolveP
   const size_t smem_pv = sizeof(double) * (13 * NL + 16);
   const size_t smem_uw = sizeof(double) * (10 * NL);
   static const bool attr = [] {
-    cudaFuncSetAttribute(k_tau_pv_seg<L>, cudaFuncAttributeMaxDynamicSharedMemorySize, 64 * 1024);
+    cudaFuncSetAttribute(k_tau_pv_seg<L, 12>, cudaFuncAttributeMaxDynamicSharedMemorySize, 64 * 1024);
+    if constexpr (L <= 8) cudaFuncSetAttribute(k_tau_pv_seg<L, 20>, cudaFuncAttributeMaxDynamicSharedMemorySize, 64 * 1024);
     cudaFuncSetAttribute(k_tau_uw_seg<L>, cudaFuncAttributeMaxDynamicSharedMemorySize, 64 * 1024);
     return true;
   }();
   (void)attr;
-  cudaError_t e = launch_pdl(k_tau_pv_seg<L>, dim3((g.Md + 1) / 2), dim3(32), smem_pv, st, g, N, sp, p, hb, tt);
+  // More warps in flight than 12 an SM hide more of the table loads; with fewer modes than that the registers are the
+  // better use (Ny = 49: 31744 modes 340 us with 12, 304 with 20; 33 rows, 190 modes 17.0 and 18.3)
+  const dim3 grid((g.Md + 1) / 2);
+  cudaError_t e;
+  if (L <= 8 && grid.x > 12 * 152) {
+    constexpr int W = L <= 8 ? 20 : 12;
+    e = launch_pdl(k_tau_pv_seg<L, W>, grid, dim3(32), smem_pv, st, g, N, sp, p, hb, tt);
+  } else {
+    e = launch_pdl(k_tau_pv_seg<L, 12>, grid, dim3(32), smem_pv, st, g, N, sp, p, hb, tt);
+  }
   if (e != cudaSuccess) return e;
   return launch_pdl(k_tau_uw_seg<L>, dim3(g.Md), dim3(32), smem_uw, st, g, N, sp, p, hb, tt);
 }
