@@ -229,6 +229,9 @@ cudaError_t launch_helmholtz(int N, int nsys, double a, double b, const double* 
                              const double* f, const double* ua, const double* ub, const double* umean, double* u,
                              double* mu, double* W, cudaStream_t st);
 
+// Complex profiles [component][mode][n] of the batched solves' callers <-> lines [component][n][mode] (noalloc.cu).
+cudaError_t launch_profiles(bool to_lines, int N, int nmodes, int ncomp, const double* src, double* dst, cudaStream_t st);
+
 // Tables of modes m0 .. m0+mcount-1 of g (mcount <= 0: all modes) for lambda_t and nu.
 cudaError_t launch_tau_setup(const GridDev& g, int N, double lambda_t, double nu, const HelmB& hb, TauTable tt,
                              double* scratch, cudaStream_t st, int m0 = 0, int mcount = 0);

@@ -99,6 +99,16 @@ int na_fail(int code, const std::string& m) { return cfgpu_record_error(code, m)
 
 }  // namespace
 
+cudaError_t launch_profiles(bool to_lines, int N, int nmodes, int ncomp, const double* src, double* dst, cudaStream_t st) {
+  const size_t per = 2 * (size_t)N * nmodes;
+  const dim3 grid((unsigned)((per + 255) / 256), ncomp);
+  if (to_lines)
+    k_gather<<<grid, 256, 0, st>>>(N, nmodes, src, dst);
+  else
+    k_scatter<<<grid, 256, 0, st>>>(N, nmodes, src, dst);
+  return cudaGetLastError();
+}
+
 extern "C" cfgpu_status cfgpu_tau_solve_batched_noalloc(int N, int nmodes, const int* kx, const int* kz, double Lx,
                                                         double Lz, double a, double b, double lambda_t, double nu,
                                                         int taucorrection, const double* Rx, const double* Ry,
