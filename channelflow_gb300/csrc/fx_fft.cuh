@@ -14,6 +14,9 @@ constexpr long long kC1 = 1425089352415399811ll;  // cos(2 pi/5)
 constexpr long long kC2 = -3730932361629093763ll; // cos(4 pi/5)
 constexpr long long kS1 = 4385974038932618941ll;  // sin(2 pi/5)
 constexpr long long kS2 = 2710681029835013083ll;  // sin(4 pi/5)
+constexpr long long kD1 = 2875339201863983833ll, kE1 = 3605561316464170519ll;  // cos, sin(2 pi/7)
+constexpr long long kD2 = -1026196679933739317ll, kE2 = 4496061421583520199ll;  // cos, sin(4 pi/7)
+constexpr long long kD3 = -4154985531143938469ll, kE3 = 2000935573311439104ll;  // cos, sin(6 pi/7)
 template <long long C>
 __device__ __forceinline__ long long mul(long long a) {
   constexpr int l = (int)(uint32_t)((unsigned long long)C & 0xffffffffull);
@@ -100,6 +103,27 @@ struct FxDft<5> {
     x[3] = fx_sub(m2, t2);
   }
 };
+// X_o and X_{7-o}: x_0 + sum_r cos(2 pi o r / 7) (x_r + x_{7-r}) -+ i sin(2 pi o r / 7) (x_r - x_{7-r})
+template <>
+struct FxDft<7> {
+  template <long long D1, long long D2, long long D3, long long E1, long long E2, long long E3>
+  static __device__ __forceinline__ void pair(fxc x0, const fxc* a, const fxc* b, fxc& p, fxc& m) {
+    const fxc c = fx_add(fx_add(x0, fxk::mul<D1>(a[0])), fx_add(fxk::mul<D2>(a[1]), fxk::mul<D3>(a[2])));
+    const fxc s = fx_rot<4, 1>(fx_add(fxk::mul<E1>(b[0]), fx_add(fxk::mul<E2>(b[1]), fxk::mul<E3>(b[2]))));
+    p = fx_add(c, s);
+    m = fx_sub(c, s);
+  }
+  static __device__ __forceinline__ void run(fxc* x) {
+    using namespace fxk;
+    const fxc a[3] = {fx_add(x[1], x[6]), fx_add(x[2], x[5]), fx_add(x[3], x[4])};
+    const fxc b[3] = {fx_sub(x[1], x[6]), fx_sub(x[2], x[5]), fx_sub(x[3], x[4])};
+    const fxc x0 = x[0];
+    x[0] = fx_add(x0, fx_add(a[0], fx_add(a[1], a[2])));
+    pair<kD1, kD2, kD3, kE1, kE2, kE3>(x0, a, b, x[1], x[6]);
+    pair<kD2, kD3, kD1, kE2, -kE3, -kE1>(x0, a, b, x[2], x[5]);
+    pair<kD3, kD1, kD2, kE3, -kE1, kE2>(x0, a, b, x[3], x[4]);
+  }
+};
 // A B points: X[k1 + A k2] = sum_n2 exp(-2 pi i n2 k1 / (A B)) (sum_n1 x[n1 B + n2] W_A^(n1 k1)) W_B^(n2 k2).
 template <int A, int B>
 struct FxDft2 {
@@ -128,16 +152,17 @@ template <> struct FxDft<6> : FxDft2<2, 3> {};
 template <> struct FxDft<8> : FxDft2<2, 4> {};
 
 // Stages of a transform of length L: up to eight radices, eight bits each, first stage lowest.  Radices with a
-// butterfly in registers, or primes above 5 (direct DFT, roots behind the stage's twiddles).  Fewest stages first: each
+// butterfly in registers, or primes above 7 (direct DFT, roots behind the stage's twiddles).  Fewest stages first: each
 // costs a pass through shared memory and L (1 - 1 / radix) twiddle products (128 = 8 x 4 x 4: 192 and eighth turns,
 // 4 x 4 x 4 x 2: 256).  Radices up to 8 keep a kernel within 64 registers and four blocks an SM; up to 10 in 80
 // registers were level or slower, up to 16 in 128 registers 20-30% slower (z pass 128x97x128 158 us).
 struct FxPlan {
   int L;
+  bool any;  // a radix of 7 or a larger prime
   unsigned long long rad;
 };
 __host__ __device__ constexpr bool fx_composite(int r) {
-  return (r >= 2 && r <= 6) || r == 8;
+  return r >= 2 && r <= 8;
 }
 // twiddle entries of stage (radix R, Ns points before it)
 __host__ __device__ constexpr int fx_stage_tw(int R, int Ns) { return Ns * (R - 1) + (fx_composite(R) ? 0 : R); }
@@ -210,9 +235,11 @@ __device__ inline void fx_stage_prime(int Rr, fxc* src, fxc* dst, int nseq, int 
 
 // nseq sequences (stride ss) at element offset a of the block's shared memory, ping-pong with b; returns the offset of
 // the result.  All threads of the block; the caller has synchronised the inputs, the result is synchronised.  Not
-// inlined: the kernels share one copy of the butterflies.
+// inlined: the kernels share one copy of the butterflies.  ANY: lengths with a factor of 7 or a larger prime, in
+// kernels of their own (in the same kernel they cost the other lengths 3%).
+template <bool ANY>
 __device__ __noinline__ int fx_fft(int a, int b, int nseq, int ss, int L, unsigned long long rad,
-                                   const fxtw* __restrict__ tw, bool inv) {
+                                       const fxtw* __restrict__ tw, bool inv) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const int tid = threadIdx.x, nthr = blockDim.x;
   fxc* const base = reinterpret_cast<fxc*>(smem_raw);
@@ -223,17 +250,19 @@ __device__ __noinline__ int fx_fft(int a, int b, int nseq, int ss, int L, unsign
     a = b;
     b = t;
   };
+  if constexpr (!ANY) {
 #define FX_STAGE(r, l, n) \
   fx_stage<r, l, n>(base + a, base + b, nseq, ss, l, n, tw, inv, inv, tid, nthr); \
   turn(r, n);
-  switch (L) {  // the lengths of the usual grids, indices known at compile time (the radices of fx_plan)
-    case 32: FX_STAGE(8, 32, 1) FX_STAGE(4, 32, 8) return a;
-    case 48: FX_STAGE(8, 48, 1) FX_STAGE(6, 48, 8) return a;
-    case 64: FX_STAGE(8, 64, 1) FX_STAGE(8, 64, 8) return a;
-    case 96: FX_STAGE(6, 96, 1) FX_STAGE(4, 96, 6) FX_STAGE(4, 96, 24) return a;
-    case 128: FX_STAGE(8, 128, 1) FX_STAGE(4, 128, 8) FX_STAGE(4, 128, 32) return a;
-  }
+    switch (L) {  // the lengths of the usual grids, indices known at compile time (the radices of fx_plan)
+      case 32: FX_STAGE(8, 32, 1) FX_STAGE(4, 32, 8) return a;
+      case 48: FX_STAGE(8, 48, 1) FX_STAGE(6, 48, 8) return a;
+      case 64: FX_STAGE(8, 64, 1) FX_STAGE(8, 64, 8) return a;
+      case 96: FX_STAGE(6, 96, 1) FX_STAGE(4, 96, 6) FX_STAGE(4, 96, 24) return a;
+      case 128: FX_STAGE(8, 128, 1) FX_STAGE(4, 128, 8) FX_STAGE(4, 128, 32) return a;
+    }
 #undef FX_STAGE
+  }
   for (int Ns = 1; Ns < L; rad >>= 8) {
     const int R = (int)(rad & 255);
     const bool in = inv && Ns == 1, out = inv && Ns * R == L;
@@ -241,8 +270,14 @@ __device__ __noinline__ int fx_fft(int a, int b, int nseq, int ss, int L, unsign
 #define FX_CASE(r) \
   case r: fx_stage<r, 0, 0>(base + a, base + b, nseq, ss, L, Ns, tw, in, out, tid, nthr); break;
       FX_CASE(2) FX_CASE(3) FX_CASE(4) FX_CASE(5) FX_CASE(6) FX_CASE(8)
+      default:
+        if constexpr (ANY) {
+          if (R == 7)
+            fx_stage<7, 0, 0>(base + a, base + b, nseq, ss, L, Ns, tw, in, out, tid, nthr);
+          else
+            fx_stage_prime(R, base + a, base + b, nseq, ss, L, Ns, tw, in, out, tid, nthr);
+        }
 #undef FX_CASE
-      default: fx_stage_prime(R, base + a, base + b, nseq, ss, L, Ns, tw, in, out, tid, nthr);
     }
     turn(R, Ns);
     Ns *= R;

@@ -18,7 +18,7 @@
 #include "fx_fft.cuh"
 #include "kernels.h"
 
-// Fewest stages, then the smallest radices, largest first; primes above 5 last.
+// Fewest stages, then the smallest radices, largest first; primes above 7 last.
 static void fx_search(int m, int maxr, unsigned long long cur, int n, int sum, int& bn, int& bsum, unsigned long long& best) {
   if (m == 1) {
     if (n < bn || (n == bn && sum < bsum)) {
@@ -36,10 +36,10 @@ static void fx_search(int m, int maxr, unsigned long long cur, int n, int sum, i
 static FxPlan fx_plan(int L) {
   static std::atomic<unsigned long long> known[8192];  // a function of L alone
   if (L < 8192)
-    if (const unsigned long long k = known[L].load(std::memory_order_relaxed)) return FxPlan{L, k};
+    if (const unsigned long long k = known[L].load(std::memory_order_relaxed)) return FxPlan{L, k >> 63 != 0, k & ~(1ull << 63)};
   int m = L, np = 0, primes[8];
-  for (int p = 7; p <= m; p += 2)
-    while (m % p == 0 && p % 3 && p % 5) {
+  for (int p = 11; p <= m; p += 2)
+    while (m % p == 0 && p % 3 && p % 5 && p % 7) {
       primes[np++] = p;
       m /= p;
     }
@@ -47,8 +47,10 @@ static FxPlan fx_plan(int L) {
   unsigned long long best = 0;
   fx_search(m, 8, 0, 0, 0, bn, bsum, best);
   for (int i = 0; i < np; ++i) best |= (unsigned long long)primes[i] << (8 * (bn + i));
-  if (L < 8192) known[L].store(best, std::memory_order_relaxed);
-  return FxPlan{L, best};
+  bool any = false;
+  for (unsigned long long r = best; r; r >>= 8) any = any || (r & 255) == 7 || (r & 255) > 8;
+  if (L < 8192) known[L].store(best | (unsigned long long)any << 63, std::memory_order_relaxed);
+  return FxPlan{L, any, best};
 }
 
 namespace {
@@ -104,6 +106,7 @@ __global__ void k_curl_points(GridDev g, double2* W) {
   for (int c = 3; c < 6; ++c) w[c * cs] = fx_vorticity(c, w, cs, kx, kz);
 }
 
+template <bool ANY>
 __global__ void __launch_bounds__(FX_THREADS, 4) k_xinv_fx(GridDev g, FxPlan px, const fxtw* __restrict__ tw,
                                                         const double2* __restrict__ W, double2* __restrict__ X, int czc,
                                                         int curl) {
@@ -150,7 +153,7 @@ __global__ void __launch_bounds__(FX_THREADS, 4) k_xinv_fx(GridDev g, FxPlan px,
     if (lane == 0) sK[jz] = K;
   }
   __syncthreads();
-  const fxc* r = a + fx_fft(0, czc * ss, nc, ss, px.L, px.rad, tw, true);
+  const fxc* r = a + fx_fft<ANY>(0, czc * ss, nc, ss, px.L, px.rad, tw, true);
   double2* dst = X + ((size_t)c * g.Ny + ny) * (size_t)Nx * g.NKz;
   for (int i = tid; i < Nx * nc; i += FX_THREADS) {
     int x, jz;
@@ -161,6 +164,7 @@ __global__ void __launch_bounds__(FX_THREADS, 4) k_xinv_fx(GridDev g, FxPlan px,
   }
 }
 
+template <bool ANY>
 __global__ void __launch_bounds__(FX_THREADS, 4) k_xfwd_fx(GridDev g, FxPlan px, const fxtw* __restrict__ tw,
                                                         const double2* __restrict__ Z, double2* __restrict__ F,
                                                         double scale, int czc) {
@@ -188,7 +192,7 @@ __global__ void __launch_bounds__(FX_THREADS, 4) k_xfwd_fx(GridDev g, FxPlan px,
     if (lane == 0) sK[jz] = K;
   }
   __syncthreads();
-  const fxc* r = a + fx_fft(0, czc * ss, nc, ss, px.L, px.rad, tw, false);
+  const fxc* r = a + fx_fft<ANY>(0, czc * ss, nc, ss, px.L, px.rad, tw, false);
   double2* dst = F + ((size_t)c * g.Ny + ny) * g.Md;
 #pragma unroll 4
   for (int i = tid; i < g.NKx * nc; i += FX_THREADS) {
@@ -242,7 +246,7 @@ __device__ __forceinline__ long long fx_round_shift(long long v, int s) {  // v 
   return s >= 0 ? v << s : ((v >> (min(-s, 63) - 1)) + 1) >> 1;
 }
 
-template <int FORM>
+template <int FORM, bool ANY>
 __global__ void __launch_bounds__(FX_THREADS, 4) k_zphys_fx(GridDev g, FxPlan pz, const fxtw* __restrict__ tw, int RP,
                                                          const double2* __restrict__ X, double2* __restrict__ Z) {
   constexpr int NC = FxForm<FORM>::NC, NO = FxForm<FORM>::NO;
@@ -339,7 +343,7 @@ __global__ void __launch_bounds__(FX_THREADS, 4) k_zphys_fx(GridDev g, FxPlan pz
     }
   }
   __syncthreads();
-  fxc* P = A + fx_fft(0, nseq * ss, ninv, ss, pz.L, pz.rad, tw, true);
+  fxc* P = A + fx_fft<ANY>(0, nseq * ss, ninv, ss, pz.L, pz.rad, tw, true);
   fxc* Q = P == A ? B : A;
   // normalise every component by its largest value: the scale above allows for the sum of magnitudes
   for (int s = warp; s < ninv; s += FX_THREADS / 32) {
@@ -415,7 +419,7 @@ __global__ void __launch_bounds__(FX_THREADS, 4) k_zphys_fx(GridDev g, FxPlan pz
     }
   }
   __syncthreads();
-  const fxc* G = A + fx_fft((int)(Q - A), (int)(P - A), nfwd, ss, pz.L, pz.rad, tw, false);
+  const fxc* G = A + fx_fft<ANY>((int)(Q - A), (int)(P - A), nfwd, ss, pz.L, pz.rad, tw, false);
 #pragma unroll 2
   for (int i = tid; i < nfwd * NKz; i += FX_THREADS) {
     int s, iz;
@@ -439,6 +443,7 @@ __global__ void __launch_bounds__(FX_THREADS, 4) k_zphys_fx(GridDev g, FxPlan pz
 // ---------------------------------------------------------------------------
 
 // Complex FFT along x of columns [z0, z0 + cols) of one plane [x][Mz]; plane blockIdx.x, column chunk blockIdx.y.
+template <bool ANY>
 __global__ void __launch_bounds__(FX_THREADS, 4) k_field_x(int Nx, int Mz, int cols, FxPlan px, const fxtw* __restrict__ tw,
                                                         int sign, double scale, double2* __restrict__ data) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -462,7 +467,7 @@ __global__ void __launch_bounds__(FX_THREADS, 4) k_field_x(int Nx, int Mz, int c
     if (lane == 0) sK[c] = K;
   }
   __syncthreads();
-  const fxc* r = a + fx_fft(0, cols * ss, nc, ss, px.L, px.rad, tw, sign > 0);
+  const fxc* r = a + fx_fft<ANY>(0, cols * ss, nc, ss, px.L, px.rad, tw, sign > 0);
 #pragma unroll 2
   for (int i = tid; i < Nx * nc; i += FX_THREADS) {
     int x, c;
@@ -475,7 +480,7 @@ __global__ void __launch_bounds__(FX_THREADS, 4) k_field_x(int Nx, int Mz, int c
 // z transform of x rows, two real rows per complex sequence, with a scale each.  Rows of Nzpad = Nz + 2 doubles;
 // c2r (INV): Nz / 2 + 1 complex in (the imaginary parts of the first and last are not used), Nz reals out, the padding
 // zero; r2c: the reverse.
-template <bool INV>
+template <bool INV, bool ANY>
 __global__ void __launch_bounds__(FX_THREADS, 4) k_field_z(long long nrows, int Nz, int seqs, FxPlan pz,
                                                         const fxtw* __restrict__ tw, double* __restrict__ data) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -567,7 +572,7 @@ __global__ void __launch_bounds__(FX_THREADS, 4) k_field_z(long long nrows, int 
     }
   }
   __syncthreads();
-  const fxc* G = a + fx_fft(0, seqs * ss, ns, ss, pz.L, pz.rad, tw, INV);
+  const fxc* G = a + fx_fft<ANY>(0, seqs * ss, ns, ss, pz.L, pz.rad, tw, INV);
   if (INV) {
 #pragma unroll 2
     for (int i = tid; i < ns * Nz; i += FX_THREADS) {
@@ -598,12 +603,14 @@ template <int FORM>
 cudaError_t run_zphys_fx(const GridDev& g, const FftPlan& pz, const fxtw* tw, int RP, const double2* X, double2* Z,
                          cudaStream_t st) {
   static const bool attr = [] {
-    cudaFuncSetAttribute(k_zphys_fx<FORM>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
+    cudaFuncSetAttribute(k_zphys_fx<FORM, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
+    cudaFuncSetAttribute(k_zphys_fx<FORM, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
     return true;
   }();
   (void)attr;
-  return launch_pdl(k_zphys_fx<FORM>, dim3((g.Nx + RP - 1) / RP, g.Ny), dim3(FX_THREADS),
-                    zphys_smem_bytes<double>(g, FORM, RP), st, g, fx_plan(pz.L), tw, RP, X, Z);
+  const FxPlan p = fx_plan(pz.L);
+  return launch_pdl(p.any ? k_zphys_fx<FORM, true> : k_zphys_fx<FORM, false>, dim3((g.Nx + RP - 1) / RP, g.Ny), dim3(FX_THREADS),
+                    zphys_smem_bytes<double>(g, FORM, RP), st, g, p, tw, RP, X, Z);
 }
 
 size_t xfx_smem(const GridDev& g, int czc, bool curl) {
@@ -642,39 +649,43 @@ static size_t field_smem(int L, int n) { return (2 * sizeof(fxc) * (size_t)(L + 
 cudaError_t launch_field_x(int Nx, int Mz, int nplanes, const void* tw, int sign, double scale,
                            cpx<double>* data, cudaStream_t st) {
   static const bool attr = [] {
-    cudaFuncSetAttribute(k_field_x, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
+    cudaFuncSetAttribute(k_field_x<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
+    cudaFuncSetAttribute(k_field_x<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
     return true;
   }();
   (void)attr;
   int cols = 1;  // about 64 KB of columns: three blocks an SM
   while (cols < Mz && cols < 16 && field_smem(Nx, cols + 1) <= 64 * 1024) ++cols;
-  k_field_x<<<dim3(nplanes, (Mz + cols - 1) / cols), FX_THREADS, field_smem(Nx, cols), st>>>(Nx, Mz, cols, fx_plan(Nx), (const fxtw*)tw,
-                                                                                             sign, scale, (double2*)data);
+  const FxPlan p = fx_plan(Nx);
+  const auto k = p.any ? k_field_x<true> : k_field_x<false>;
+  k<<<dim3(nplanes, (Mz + cols - 1) / cols), FX_THREADS, field_smem(Nx, cols), st>>>(Nx, Mz, cols, p, (const fxtw*)tw, sign,
+                                                                                     scale, (double2*)data);
   return cudaGetLastError();
 }
 
 cudaError_t launch_field_z(long long nrows, int Nz, bool inverse, const void* tw, double* data,
                            cudaStream_t st) {
   static const bool attr = [] {
-    cudaFuncSetAttribute(k_field_z<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
-    cudaFuncSetAttribute(k_field_z<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
+    for (auto k : {k_field_z<false, false>, k_field_z<false, true>, k_field_z<true, false>, k_field_z<true, true>})
+      cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
     return true;
   }();
   (void)attr;
   int seqs = 1;
   while (seqs < 16 && field_smem(Nz, seqs + 1) <= 64 * 1024) ++seqs;
   const unsigned nb = (unsigned)((nrows + 2 * seqs - 1) / (2 * seqs));
-  if (inverse)
-    k_field_z<true><<<nb, FX_THREADS, field_smem(Nz, seqs), st>>>(nrows, Nz, seqs, fx_plan(Nz), (const fxtw*)tw, data);
-  else
-    k_field_z<false><<<nb, FX_THREADS, field_smem(Nz, seqs), st>>>(nrows, Nz, seqs, fx_plan(Nz), (const fxtw*)tw, data);
+  const FxPlan p = fx_plan(Nz);
+  const auto k = inverse ? (p.any ? k_field_z<true, true> : k_field_z<true, false>)
+                         : (p.any ? k_field_z<false, true> : k_field_z<false, false>);
+  k<<<nb, FX_THREADS, field_smem(Nz, seqs), st>>>(nrows, Nz, seqs, p, (const fxtw*)tw, data);
   return cudaGetLastError();
 }
 
 cudaError_t launch_xinv_fx(const GridDev& g, const FftPlan& px, const void* tw, const cpx<double>* W, cpx<double>* X,
                            int ncomp, int czc, bool curl, cudaStream_t st) {
   static const bool attr = [] {
-    cudaFuncSetAttribute(k_xinv_fx, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
+    cudaFuncSetAttribute(k_xinv_fx<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
+    cudaFuncSetAttribute(k_xinv_fx<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
     return true;
   }();
   (void)attr;
@@ -683,8 +694,9 @@ cudaError_t launch_xinv_fx(const GridDev& g, const FftPlan& px, const void* tw, 
     if (e != cudaSuccess) return e;
     curl = false;
   }
-  return launch_pdl(k_xinv_fx, dim3(g.Ny, ncomp, (g.NKz + czc - 1) / czc), dim3(FX_THREADS), xfx_smem(g, czc, curl), st, g, fx_plan(px.L),
-                    (const fxtw*)tw, (const double2*)W, (double2*)X, czc, (int)curl);
+  const FxPlan p = fx_plan(px.L);
+  return launch_pdl(p.any ? k_xinv_fx<true> : k_xinv_fx<false>, dim3(g.Ny, ncomp, (g.NKz + czc - 1) / czc), dim3(FX_THREADS),
+                    xfx_smem(g, czc, curl), st, g, p, (const fxtw*)tw, (const double2*)W, (double2*)X, czc, (int)curl);
 }
 
 cudaError_t launch_curl_points(const GridDev& g, cpx<double>* W, cudaStream_t st) {
@@ -695,13 +707,15 @@ cudaError_t launch_curl_points(const GridDev& g, cpx<double>* W, cudaStream_t st
 cudaError_t launch_xfwd_fx(const GridDev& g, const FftPlan& px, const void* tw, const cpx<double>* Z, cpx<double>* F,
                            int ncomp, int czc, cudaStream_t st) {
   static const bool attr = [] {
-    cudaFuncSetAttribute(k_xfwd_fx, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
+    cudaFuncSetAttribute(k_xfwd_fx<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
+    cudaFuncSetAttribute(k_xfwd_fx<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
     return true;
   }();
   (void)attr;
   const double scale = 1.0 / ((double)g.Nx * (double)g.Nz);
-  return launch_pdl(k_xfwd_fx, dim3(g.Ny, ncomp, (g.NKz + czc - 1) / czc), dim3(FX_THREADS), xfx_smem(g, czc, false), st, g, fx_plan(px.L),
-                    (const fxtw*)tw, (const double2*)Z, (double2*)F, scale, czc);
+  const FxPlan p = fx_plan(px.L);
+  return launch_pdl(p.any ? k_xfwd_fx<true> : k_xfwd_fx<false>, dim3(g.Ny, ncomp, (g.NKz + czc - 1) / czc), dim3(FX_THREADS),
+                    xfx_smem(g, czc, false), st, g, p, (const fxtw*)tw, (const double2*)Z, (double2*)F, scale, czc);
 }
 
 cudaError_t launch_zphys_fx(const GridDev& g, int form, const FftPlan& pz, const void* tw, int RP, const cpx<double>* X,
