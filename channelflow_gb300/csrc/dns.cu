@@ -1015,7 +1015,8 @@ int rotation_term(cfgpu_dns d, const double* U, void* Nout) {
   return CFGPU_OK;
 }
 
-int nonlinear(cfgpu_dns d, const double* U, void* Nout, int which = 0) {
+// bump: advance the fields' constant versions here; a step leaves that to its solve (step_ptrs).
+int nonlinear(cfgpu_dns d, const double* U, void* Nout, int which = 0, bool bump = true) {
   PhaseScope ps(d, 0);
   int form = d->fl.nonlinearity;
   if (form == CFGPU_Alternating || form == CFGPU_Alternating_) {
@@ -1028,7 +1029,7 @@ int nonlinear(cfgpu_dns d, const double* U, void* Nout, int which = 0) {
   // rotation about z (nse.cpp:62-78; not with LinearAboutProfile)
   if (d->fl.rotation != 0.0 && form != CFGPU_LinearAboutProfile)
     CKS(fp64 ? rotation_term<double>(d, U, Nout) : rotation_term<float>(d, U, Nout));
-  if (!fp64) {
+  if (!fp64 && bump) {
     CK(launch_dither_bump(d->dver, d->nb, d->st));  // next evaluation: next version of the FP32 constants
     d->launches++;
   }
@@ -1066,6 +1067,16 @@ SolvePtrs base_ptrs(cfgpu_dns d) {
     p.Wbaseyy = d->dbaseS + 3 * nN;
     p.slot = d->dslot;
     p.base_stride = d->N;
+  }
+  return p;
+}
+
+// Of a step's solve: it follows a nonlinear evaluation and advances the versions of the FP32 constants.
+SolvePtrs step_ptrs(cfgpu_dns d) {
+  SolvePtrs p = base_ptrs(d);
+  if (d->precision != CFGPU_FP64) {
+    p.ver = d->dver;
+    p.nver = d->nb;
   }
   return p;
 }
@@ -1111,11 +1122,11 @@ int ms_step(cfgpu_dns d) {
   Scheme& s = d->main;
   const int K = s.order, J = K - 1;
   const double dt = d->fl.dt;
-  CKS(nonlinear(d, d->Uh[d->perm[0]], d->Nh[d->perm[0]]));
+  CKS(nonlinear(d, d->Uh[d->perm[0]], d->Nh[d->perm[0]], 0, false));
   SolveParams sp = base_params(d);
   sp.kind = 0;
   sp.order = K;
-  SolvePtrs p = base_ptrs(d);
+  SolvePtrs p = step_ptrs(d);
   for (int j = 0; j < K; ++j) {
     sp.a[j] = -s.alpha[j] / dt;
     sp.b[j] = -s.beta[j];
@@ -1218,7 +1229,7 @@ int cnab_step(cfgpu_dns d, int which) {
   {
     for (int j = 0; j < s.nsub; ++j) {
       std::swap(d->fj[which], d->fj1[which]);
-      CKS(nonlinear(d, d->Ucur, d->fj[which], which));
+      CKS(nonlinear(d, d->Ucur, d->fj[which], which, false));
       SolveParams sp = base_params(d);
       sp.kind = 1;
       sp.scheme = which;
@@ -1227,7 +1238,7 @@ int cnab_step(cfgpu_dns d, int which) {
       sp.a_b = s.ca[j] / s.cb[j];
       sp.g_b = s.cg[j] / s.cb[j];
       sp.z_b = s.cz[j] / s.cb[j];
-      SolvePtrs p = base_ptrs(d);
+      SolvePtrs p = step_ptrs(d);
       p.uin[0] = d->Ucur;
       p.nin[0] = d->fj[which];
       p.nin[1] = d->fj1[which];
@@ -1246,7 +1257,7 @@ int rk_step(cfgpu_dns d, int which) {
   Scheme& s = which == 0 ? d->main : d->init;
   {
     for (int j = 0; j < s.nsub; ++j) {
-      CKS(nonlinear(d, d->Ucur, d->rkN, which));
+      CKS(nonlinear(d, d->Ucur, d->rkN, which, false));
       SolveParams sp = base_params(d);
       sp.kind = 2;
       sp.scheme = which;
@@ -1254,7 +1265,7 @@ int rk_step(cfgpu_dns d, int which) {
       sp.lam = s.lambda_t[j];
       sp.rkA = s.rA[j];
       sp.B_C = s.rB[j] / s.rC[j];
-      SolvePtrs p = base_ptrs(d);
+      SolvePtrs p = step_ptrs(d);
       p.uin[0] = d->Ucur;
       p.nin[0] = d->rkN;
       p.Q = d->rkQ[which];
@@ -1278,14 +1289,14 @@ int main_step(cfgpu_dns d) {
 // with order 1): rhs = -alpha_0/dt u_n - beta_0 N(u_n), solved with lambda_t = eta/dt.
 int ms1_init_step(cfgpu_dns d) {
   Scheme& s = d->init;
-  CKS(nonlinear(d, d->Ucur, d->fj[1], 1));
+  CKS(nonlinear(d, d->Ucur, d->fj[1], 1, false));
   SolveParams sp = base_params(d);
   sp.kind = 0;
   sp.order = 1;
   sp.scheme = 1;
   sp.a[0] = -s.alpha[0] / d->fl.dt;
   sp.b[0] = -s.beta[0];
-  SolvePtrs p = base_ptrs(d);
+  SolvePtrs p = step_ptrs(d);
   p.uin[0] = d->Ucur;  // the right-hand side is complete before the solve writes u
   p.nin[0] = d->fj[1];
   p.uout = d->Ucur;

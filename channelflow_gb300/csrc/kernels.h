@@ -305,6 +305,8 @@ struct SolvePtrs {
   double* scratch;       // [8][N][2Md]
   double* dPdx_out;      // device scalars: actual dPdx, dPdz after solve ([field][2] for a batch)
   const SlotParams* slot;  // per-field parameters (null: SolveParams holds them for every field)
+  int* ver;                // constant versions of nver fields to advance (null: none)
+  int nver;
   int base_stride;         // 0: one base flow for all fields; N: Ubase/Wbase/Ubaseyy/Wbaseyy are [field][N]
 };
 

@@ -826,6 +826,11 @@ __device__ void helm_t(int M, int q, const double* __restrict__ hlo, const doubl
   }
 }
 
+// The fields' next versions of the FP32 constants (the nonlinear pass, their only reader, is done).
+__device__ __forceinline__ void bump_versions(const SolvePtrs& P, int tid, int nthr) {
+  for (int f = tid; f < P.nver; f += nthr) P.ver[f] = (P.ver[f] + 1) % DITHER_V;
+}
+
 // ---------------------------------------------------------------------------
 // Right-hand side of a multistep scheme, sum_j a_j u_j + b_j N_j (dnsalgo.cpp:217-224), elementwise: one thread per
 // (component, n, mode), one component a grid layer (blockIdx.z), into the scratch lines 0, 2 and 1.  Bound by its 4
@@ -839,6 +844,7 @@ __global__ void __launch_bounds__(128) k_tau_rhs_ms(GridDev g, int N, SolveParam
   pdl_wait();
   pdl_trigger();
   const int m = blockIdx.x * 128 + threadIdx.x, n = blockIdx.y;
+  if (P.ver && blockIdx.x + blockIdx.y + blockIdx.z == 0) bump_versions(P, threadIdx.x, 128);
   if (m >= g.Md) return;
   const bool m00 = mode_kx(g, m) == 0 && mode_kz(g, m) == 0;
   if (m00 != (blockIdx.z == 3)) return;
@@ -903,6 +909,7 @@ __global__ void __launch_bounds__(32, 10) k_tau_rhs(GridDev g, int N, SolveParam
   const int lane = threadIdx.x;
   const int t = blockIdx.x * 32 + lane;
   const int Md = g.Md;
+  if (P.ver && blockIdx.x + blockIdx.y == 0) bump_versions(P, lane, 32);
   // one component per grid row: the eight lane groups of a warp read eight consecutive modes of one plane
   const int grp = t >> 2;
   const bool act = grp < Md;
@@ -1455,6 +1462,10 @@ cudaError_t launch_tau_solve(const GridDev& g, int N, const SolveParams& sp, con
     const size_t smem_u = sizeof(double) * ((size_t)M0 * 32 + (size_t)4 * N * 4);
     k_tau_uw<R><<<(8 * g.Md + 31) / 32, 32, smem_u, st>>>(g, N, sp, p, hb, tt);
     return cudaGetLastError();
+  }
+  if (p.ver) {
+    const cudaError_t e = launch_dither_bump(p.ver, p.nver, st);
+    if (e != cudaSuccess) return e;
   }
   const int T = 64;
   k_tau_solve<R><<<(4 * g.Md + T - 1) / T, T, 0, st>>>(g, N, sp, p, hb, tt);
