@@ -83,6 +83,29 @@ long double cospi_ratio(long long m, long long d) {
   if (r < 0) r += 2 * d;
   return cosl(3.14159265358979323846264338327950288L * (long double)r / (long double)d);
 }
+long double sinpi_ratio(long long m, long long d) {
+  long long r = m % (2 * d);
+  if (r < 0) r += 2 * d;
+  return sinl(3.14159265358979323846264338327950288L * (long double)r / (long double)d);
+}
+// cos and sin of pi m / M for all m from one table (the host's long double may be a software type).
+struct HalfTurn {
+  long long M;
+  std::vector<long double> c, s;
+  explicit HalfTurn(int M_) : M(M_), c(2 * M_), s(2 * M_) {
+    for (int m = 0; m < 2 * M_; ++m) {
+      c[m] = cospi_ratio(m, M);
+      s[m] = sinpi_ratio(m, M);
+    }
+  }
+  long double cosine(long long m) const { return c[m % (2 * M)]; }
+  // T'_n(y_j) at y_j = cos(pi j / M): n sin(n theta) / sin(theta), +-n^2 at the ends
+  long double cheb_deriv(int n, int j) const {
+    if (j == 0) return (long double)n * n;
+    if (j == M) return (n % 2 ? 1.0L : -1.0L) * n * n;
+    return n * s[(long long)n * j % (2 * M)] / s[j];
+  }
+};
 // Values at Gauss-Lobatto points -> Chebyshev coefficients (chebyfft, chebyshev.cpp:262-284), direct sum.
 std::vector<double> chebyfft_h(const std::vector<double>& x) {
   const int N = (int)x.size();
@@ -239,55 +262,41 @@ struct ChebMats {
   std::vector<double> dfA, dfB;                // diff o chebyfft: even coefs from d (P x KB), odd from s (P x KA)
 };
 
-long double sinpi_ratio(long long m, long long d) {
-  long long r = m % (2 * d);
-  if (r < 0) r += 2 * d;
-  return sinl(3.14159265358979323846264338327950288L * (long double)r / (long double)d);
-}
-
-// T'_n(y_j) at y_j = cos(pi j/(N-1)): n sin(n theta)/sin(theta), n^2 at j = 0
-long double cheb_deriv_at(int n, int j, int N) {
-  if (j == 0) return (long double)n * n;
-  if (2 * j == 2 * (N - 1)) return (n % 2 ? 1.0L : -1.0L) * n * n;
-  return n * sinpi_ratio((long long)n * j, N - 1) / sinpi_ratio(j, N - 1);
-}
 
 ChebMats make_cheb_mats(int N) {
   ChebMats M;
+  const HalfTurn ht(N - 1);
+  auto cospi = [&](long long m) { return ht.cosine(m); };
   const int P = (N + 1) / 2, KA = (N + 1) / 2, KB = (N - 1) / 2, J = (N - 1) / 2;
   M.invA.assign((size_t)P * KA, 0.0);
   M.invB.assign((size_t)P * KB, 0.0);
   M.fwdA.assign((size_t)P * KA, 0.0);
   M.fwdB.assign((size_t)P * KB, 0.0);
   for (int j = 0; j < P; ++j) {
-    for (int k = 0; k < KA; ++k) M.invA[j * KA + k] = (double)cospi_ratio(2LL * k * j, N - 1);
-    for (int k = 0; k < KB; ++k) M.invB[j * KB + k] = (double)cospi_ratio((2LL * k + 1) * j, N - 1);
+    for (int k = 0; k < KA; ++k) M.invA[j * KA + k] = (double)cospi(2LL * k * j);
+    for (int k = 0; k < KB; ++k) M.invB[j * KB + k] = (double)cospi((2LL * k + 1) * j);
   }
   M.derA.assign((size_t)P * KA, 0.0);
   M.derB.assign((size_t)P * KB, 0.0);
   for (int j = 0; j < P; ++j) {
-    for (int k = 0; k < KA; ++k) M.derA[j * KA + k] = (double)(cheb_deriv_at(2 * k, j, N));
-    for (int k = 0; k < KB; ++k) M.derB[j * KB + k] = (double)(cheb_deriv_at(2 * k + 1, j, N));
+    for (int k = 0; k < KA; ++k) M.derA[j * KA + k] = (double)ht.cheb_deriv(2 * k, j);
+    for (int k = 0; k < KB; ++k) M.derB[j * KB + k] = (double)ht.cheb_deriv(2 * k + 1, j);
   }
   {
-    // full forward matrix F[n][j] and coefficient derivative D (diff, chebyshev.cpp:672-697, L = 2 here;
-    // the 2/L factor is applied by the caller), DF = D F split by parity
-    std::vector<long double> F((size_t)N * N), D((size_t)N * N, 0.0L), DF((size_t)N * N, 0.0L);
+    // full forward matrix F[n][j] and its coefficient derivative DF (diff, chebyshev.cpp:672-697, L = 2 here; the
+    // 2/L factor is applied by the caller), split by parity
+    std::vector<long double> F((size_t)N * N), DF((size_t)(N + 2) * N, 0.0L);
     for (int n = 0; n < N; ++n) {
       const long double cn = (n == 0 || n == N - 1) ? 0.5L : 1.0L;
       for (int j = 0; j < N; ++j) {
         const long double w = (j == 0 || j == N - 1) ? 1.0L : 2.0L;
-        F[(size_t)n * N + j] = w * cospi_ratio((long long)n * j, N - 1) * cn / (N - 1);
+        F[(size_t)n * N + j] = w * cospi((long long)n * j) * cn / (N - 1);
       }
     }
-    for (int n = 0; n < N; ++n)
-      for (int m2 = n + 1; m2 < N; m2 += 2) D[(size_t)n * N + m2] = (n == 0 ? 1.0L : 2.0L) * m2;
-    for (int n = 0; n < N; ++n)
-      for (int mm = 0; mm < N; ++mm) {
-        const long double dv = D[(size_t)n * N + mm];
-        if (dv == 0.0L) continue;
-        for (int j = 0; j < N; ++j) DF[(size_t)n * N + j] += dv * F[(size_t)mm * N + j];
-      }
+    for (int n = N - 2; n >= 0; --n)
+      for (int j = 0; j < N; ++j)
+        DF[(size_t)n * N + j] = DF[(size_t)(n + 2) * N + j] + 2.0L * (n + 1) * F[(size_t)(n + 1) * N + j];
+    for (int j = 0; j < N; ++j) DF[j] *= 0.5L;
     M.dfA.assign((size_t)P * KB, 0.0);
     M.dfB.assign((size_t)P * KA, 0.0);
     for (int k = 0; k < P; ++k) {
@@ -301,13 +310,13 @@ ChebMats make_cheb_mats(int N) {
     const long double cn = (n == 0 || n == N - 1) ? 0.5L : 1.0L;
     for (int j = 0; j <= J; ++j) {
       const long double w = (j == 0) ? 1.0L : 2.0L;
-      M.fwdA[k * KA + j] = (double)(w * cospi_ratio((long long)n * j, N - 1) * cn / (N - 1));
+      M.fwdA[k * KA + j] = (double)(w * cospi((long long)n * j) * cn / (N - 1));
     }
     const int no = 2 * k + 1;
     if (no < N)
       for (int j = 0; j < J; ++j) {
         const long double w = (j == 0) ? 1.0L : 2.0L;
-        M.fwdB[k * KB + j] = (double)(w * cospi_ratio((long long)no * j, N - 1) / (N - 1));
+        M.fwdB[k * KB + j] = (double)(w * cospi((long long)no * j) / (N - 1));
       }
   }
   return M;
@@ -542,11 +551,12 @@ int compute_base(const cfgpu_flags& f, const double* Ub, const double* Wb, int N
     B.dPdzAct = B.dPdzRef = f.dPdz;
   }
   B.basey.assign(4 * (size_t)Ny, 0.0);
+  const HalfTurn ht(Ny - 1);
   for (int j = 0; j < Ny; ++j) {
     long double U = 0, Uy = 0, W = 0, Wy = 0;
     for (int n = 0; n < Ny; ++n) {
-      const long double c = cospi_ratio((long long)n * j, Ny - 1);
-      const long double dd = cheb_deriv_at(n, j, Ny) * (2.0L / (b - a));
+      const long double c = ht.cosine((long long)n * j);
+      const long double dd = ht.cheb_deriv(n, j) * (2.0L / (b - a));
       U += B.Ubase[n] * c;
       Uy += B.Ubase[n] * dd;
       W += B.Wbase[n] * c;
@@ -1993,14 +2003,14 @@ int dns_create_impl(cfgpu_dns d, const cfgpu_grid* grid, const cfgpu_flags* flag
   std::vector<std::complex<long double>> twx, twz;
   if (!make_fft_plan(Nx, d->px, twx) || !make_fft_plan(Nz, d->pz, twz))
     return fail(CFGPU_ENOTSUP, "Nx and Nz must factor into primes <= " + std::to_string(FFT_MAX_RADIX));
-  ChebMats cm = make_cheb_mats(Ny);
-  for (auto& v : cm.derA) v *= 2.0 / (b - a);
-  for (auto& v : cm.derB) v *= 2.0 / (b - a);
-  for (auto& v : cm.dfA) v *= 2.0 / (b - a);
-  for (auto& v : cm.dfB) v *= 2.0 / (b - a);
   const std::vector<double>& basey = bf.basey;
   const bool fp64 = d->precision == CFGPU_FP64;
   const std::vector<double> circx = circle_table(Nx), circz = circle_table(Nz);
+  if (fp64) CKS(oz_upload(d, f.nonlinearity != CFGPU_Rotational && f.nonlinearity != CFGPU_Convection));
+  ChebMats cm;  // dense matrices and the FFT form's table: not beside the tensor-core transforms unless asked for
+  if (!d->oz) cm = make_cheb_mats(Ny);
+  for (auto* t : {&cm.derA, &cm.derB, &cm.dfA, &cm.dfB})
+    for (auto& v : *t) v *= 2.0 / (b - a);
   if (fp64) {
     CKS(upload_tw<double>(twx, &d->twx, B, d->st));
     CKS(upload_tw<double>(twz, &d->twz, B, d->st));
@@ -2008,17 +2018,15 @@ int dns_create_impl(cfgpu_dns d, const cfgpu_grid* grid, const cfgpu_flags* flag
     CKS(upload_ints(fx_twiddles(Nz), &d->twzq, B, d->st));
     CKS(upload_as<double>(circx, &d->twxf, B, d->st));
     CKS(upload_as<double>(circz, &d->twzf, B, d->st));
-    CKS(upload_as<double>(cm.invA, &d->cinvA, B, d->st));
-    CKS(upload_as<double>(cm.invB, &d->cinvB, B, d->st));
-    CKS(upload_as<double>(cm.fwdA, &d->cfwdA, B, d->st));
-    CKS(upload_as<double>(cm.fwdB, &d->cfwdB, B, d->st));
-    CKS(upload_as<double>(cm.derA, &d->cderA, B, d->st));
-    CKS(upload_as<double>(cm.derB, &d->cderB, B, d->st));
     CKS(upload_as<double>(basey, &d->basey, B, d->st));
-    CKS(upload_as<double>(cm.dfA, &d->cdfA, B, d->st));
-    CKS(upload_as<double>(cm.dfB, &d->cdfB, B, d->st));
-    if (dct_supported(Ny)) CKS(upload_as<double>(dct_table(Ny), &d->cdct, B, d->st));
-    CKS(oz_upload(d, f.nonlinearity != CFGPU_Rotational && f.nonlinearity != CFGPU_Convection));
+    if (!d->oz) {
+      CKS(upload_as<double>(cm.invA, &d->cinvA, B, d->st));
+      CKS(upload_as<double>(cm.invB, &d->cinvB, B, d->st));
+      CKS(upload_as<double>(cm.fwdA, &d->cfwdA, B, d->st));
+      CKS(upload_as<double>(cm.fwdB, &d->cfwdB, B, d->st));
+    }
+    if (dct_supported(Ny) && (!d->oz || g_cheb_fft.load() == 2))
+      CKS(upload_as<double>(dct_table(Ny), &d->cdct, B, d->st));
   } else {
     // DITHER_V dithered versions of every FP32 constant table in one block (16-byte aligned tables)
     std::vector<std::vector<double>> tabs = {cm.invA, cm.invB, cm.fwdA, cm.fwdB, cm.derA, cm.derB, cm.dfA, cm.dfB};
