@@ -24,8 +24,8 @@
 // Measured against FP64 arithmetic, which the FP64 pipe bounds (one warp instruction per 64 cycles).  128x97x128: curl
 // and inverse transforms 190 us (FFT form) -> 63 us and 15 us more in the x pass, which forms the vorticity; forward 91
 // -> 56 us.  72x57x90, skew-symmetric: gradient 107 -> 28 us, forward with divergence 484 -> 43 us.  Ny = 35, 190 modes:
-// 29 -> 17 us and 24 -> 11 us.  FlowField y transform 128x97x128: 1340 -> 83 and 96 us.  Relative error of one transform
-// 5e-17 (FP64 products 2e-16 ... 5e-16).  Bound by instruction issue and latency of the digits and the sums (16 warps
+// 29 -> 17 us and 24 -> 11 us (10 and 8 with k_cheb_oz_few).  FlowField y transform 128x97x128: 1340 -> 83 and 96 us.
+// Relative error of one transform 5e-17 (FP64 products 2e-16 ... 5e-16).  Bound by instruction issue and latency of the digits and the sums (16 warps
 // an SM).  256 threads (and K steps of 16): 102 and 70 us.
 #include <cuda_fp16.h>
 
@@ -101,7 +101,8 @@ struct OzSum {
   }
 };
 
-// Seven digits (most significant first) of the eight integers x[0..7], |x| < 2^61, as FP16 pairs.
+// Seven digits (most significant first) of the eight integers x[0..7], |x| < 2^61, as FP16 pairs; copies 32 rows apart.
+template <int COPIES>
 __device__ __forceinline__ void oz_store(unsigned char* dst, const long long (&x)[8]) {
   constexpr unsigned long long OFF = 0x4020100804020100ull;  // 256 in every digit
   unsigned lo[8], hi[8];
@@ -134,9 +135,107 @@ __device__ __forceinline__ void oz_store(unsigned char* dst, const long long (&x
       const __half2 h = __hadd2(*reinterpret_cast<const __half2*>(&u), bias);
       w[p] = *reinterpret_cast<const unsigned*>(&h);
     }
-    *reinterpret_cast<uint4*>(dst + d * (OZ_LINES * 32)) = make_uint4(w[0], w[1], w[2], w[3]);
+#pragma unroll
+    for (int c = 0; c < COPIES; ++c)
+      *reinterpret_cast<uint4*>(dst + d * (OZ_LINES * 32) + c * 1024) = make_uint4(w[0], w[1], w[2], w[3]);
   }
 }
+
+// sum_s r_s 2^(9 (6 - s) - 8) of the exact FP32 sums r
+__device__ __forceinline__ long long oz_sum(const uint32_t (&r)[OZ_DIGITS]) {
+            int d[OZ_DIGITS];
+  #pragma unroll
+            for (int s = 0; s < OZ_DIGITS; ++s) d[s] = __float2int_rn(__uint_as_float(r[s]));
+                      long long x = (long long)(2 * d[5] + ((d[6] + 128) >> 8));
+            x = fx_mw(d[4], 1 << 10, x);
+            x = fx_mw(d[3], 1 << 19, x);
+            x = fx_mw(d[2], 1 << 28, x);
+            x += (long long)((unsigned long long)(((unsigned)d[0] << 14) + ((unsigned)d[1] << 5)) << 32);
+  return x;
+}
+
+// K of a line (fx_line_K) from the sums of its four quarters, stride apart
+__device__ __forceinline__ int oz_scale(const unsigned long long* sS, const int* sE, int stride) {
+  int e = 1;
+  bool nz = false;
+  for (int i = 0; i < 4; ++i) {
+    const int ei = sE[i * stride];
+    e = max(e, ei & 0xffff);
+    nz = nz || (ei & 0x10000);
+  }
+  unsigned long long S = 4;
+  for (int i = 0; i < 4; ++i) S += sS[i * stride] >> min(e - (sE[i * stride] & 0xffff), 63);
+  if (!nz) return FX_ZERO;
+  if (e == 2047) return FX_NAN;
+  return min(61 - (64 - __clzll((long long)S)) - (e - 1043), 1083 - e);
+}
+
+// A line of a job: its wavenumbers, its base flow and its points.  FP64 instructions take the whole warp's slot even where
+// no lane needs them: the rare ones stand behind branches over whole groups of points.
+template <bool INV>
+struct OzLine {
+  const OzJob& job;
+  const double *src = nullptr, *base = nullptr;
+  double kx = 0.0, kz = 0.0, shift = 0.0;
+  unsigned ld;
+  int N, gl;
+  bool act, hasb, fd = false;
+  __device__ __forceinline__ OzLine(const OzArgs& a, const OzJob& j, int gl_, bool act_)
+      : job(j), ld(a.ld), N(a.N), gl(gl_), act(act_) {
+    const int m = min(gl, a.nlines - 1) >> 1;
+    if (job.gx || job.pkx) {
+      const int ikx = mode_kx(a.g, m), ikz = mode_kz(a.g, m);
+      const double sg = gl & 1 ? 2.0 * M_PI : -2.0 * M_PI;  // i k f: re = -k f_im, im = k f_re
+      kx = ikx == a.g.kxmax ? 0.0 : sg * ikx / a.g.Lx;
+      kz = ikz == a.g.kzmax ? 0.0 : sg * ikz / a.g.Lz;
+    }
+    if (job.base || job.shift != 0.0) {
+      if (act && !(gl & 1) && mode_kx(a.g, m) == 0 && mode_kz(a.g, m) == 0) {
+        if (job.base) base = job.base + (size_t)job.bstride * mode_field(a.g, m);
+        shift = job.shift;
+      }
+    }
+    hasb = __any_sync(0xffffffffu, base != nullptr || shift != 0.0);
+  }
+      // v[i] = point n0 + i dn of the line, i < cnt, else zero
+      __device__ __forceinline__ void load8(double (&v)[8], int n0, int dn, int cnt) const {
+        unsigned o = (unsigned)n0 * ld + gl;
+  #pragma unroll
+        for (int i = 0; i < 8; ++i, o += (unsigned)dn * ld) v[i] = src && i < cnt ? src[o] : 0.0;
+        if constexpr (INV) {
+          if (hasb) {
+            for (int i = 0; i < 8; ++i)
+              if (i < cnt) {
+                if (base) v[i] += base[n0 + i * dn];
+                if (n0 + i * dn == 0) v[i] -= shift;
+              }
+          }
+        } else if (!fd && job.pkx) {
+          double px[8], pz[8];
+          o = (unsigned)n0 * ld + (gl ^ 1);
+  #pragma unroll
+          for (int i = 0; i < 8; ++i, o += (unsigned)dn * ld) {
+            px[i] = i < cnt ? job.pkx[o] : 0.0;
+            pz[i] = i < cnt ? job.pkz[o] : 0.0;
+          }
+  #pragma unroll
+          for (int i = 0; i < 8; ++i) v[i] = fma(job.wF, v[i], job.wK * fma(kx, px[i], kz * pz[i]));
+        }
+      }
+  // magnitudes of every fourth point
+  __device__ __forceinline__ void magnitudes(OzSum& sum, int quarter) const {
+    if (act)
+      for (int n0 = quarter; n0 < N; n0 += 32) {
+        double v[8];
+        load8(v, n0, 4, (N - n0 + 3) >> 2);
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+          const int n = n0 + 4 * i;
+          if (n < N && !(INV && job.deriv && n == 0)) sum.add(v[i], INV && job.deriv ? (unsigned)n * (n + 1) : 1u);
+        }
+      }
+  }
+};
 
 template <bool INV>
 __global__ void __launch_bounds__(OZ_THREADS, 1) k_cheb_oz(const __grid_constant__ OzArgs a) {
@@ -175,26 +274,8 @@ __global__ void __launch_bounds__(OZ_THREADS, 1) k_cheb_oz(const __grid_constant
   pdl_wait();  // the previous kernel's output is read from here on
   pdl_trigger();
 
-  // This line's wavenumbers and base flow.  FP64 instructions take the whole warp's slot even where no lane needs them:
-  // the rare ones stand behind branches over whole groups of points.
-  double kx = 0.0, kz = 0.0;
-  const double* base = nullptr;
-  double shift = 0.0;
-  if (job.gx || job.pkx) {
-    const int m = min(gl, a.nlines - 1) >> 1;
-    const int ikx = mode_kx(a.g, m), ikz = mode_kz(a.g, m);
-    const double sg = gl & 1 ? 2.0 * M_PI : -2.0 * M_PI;  // i k f: re = -k f_im, im = k f_re
-    kx = ikx == a.g.kxmax ? 0.0 : sg * ikx / a.g.Lx;
-    kz = ikz == a.g.kzmax ? 0.0 : sg * ikz / a.g.Lz;
-  }
-  if (job.base || job.shift != 0.0) {
-    const int m = min(gl, a.nlines - 1) >> 1;
-    if (act && !(gl & 1) && mode_kx(a.g, m) == 0 && mode_kz(a.g, m) == 0) {
-      if (job.base) base = job.base + (size_t)job.bstride * mode_field(a.g, m);
-      shift = job.shift;
-    }
-  }
-  const bool hasb = __any_sync(0xffffffffu, base != nullptr || shift != 0.0);
+  OzLine<INV> ln(a, job, gl, act);
+  const double kx = ln.kx, kz = ln.kz;
   const bool emit_scale = INV && job.deriv && a.dscale != 1.0, emit_grad = INV && job.gx != nullptr;
 
   bool ok = true;
@@ -204,62 +285,15 @@ __global__ void __launch_bounds__(OZ_THREADS, 1) k_cheb_oz(const __grid_constant
   for (int sg = 0; sg < nstage; ++sg) {
     const bool fd = !INV && sg == 1;  // derivative of the forward transform
     const OzMatrix& M = INV ? a.t.T : (fd ? a.t.DF : a.t.F);
-    const double* src = fd ? job.pd : job.in;
-    // v[i] = point n0 + i dn of the line, i < cnt, else zero
-    auto load8 = [&](double (&v)[8], int n0, int dn, int cnt) {
-      unsigned o = (unsigned)n0 * ld + gl;
-#pragma unroll
-      for (int i = 0; i < 8; ++i, o += (unsigned)dn * ld) v[i] = src && i < cnt ? src[o] : 0.0;
-      if constexpr (INV) {
-        if (hasb) {
-          for (int i = 0; i < 8; ++i)
-            if (i < cnt) {
-              if (base) v[i] += base[n0 + i * dn];
-              if (n0 + i * dn == 0) v[i] -= shift;
-            }
-        }
-      } else if (!fd && job.pkx) {
-        double px[8], pz[8];
-        o = (unsigned)n0 * ld + (gl ^ 1);
-#pragma unroll
-        for (int i = 0; i < 8; ++i, o += (unsigned)dn * ld) {
-          px[i] = i < cnt ? job.pkx[o] : 0.0;
-          pz[i] = i < cnt ? job.pkz[o] : 0.0;
-        }
-#pragma unroll
-        for (int i = 0; i < 8; ++i) v[i] = fma(job.wF, v[i], job.wK * fma(kx, px[i], kz * pz[i]));
-      }
-    };
+    ln.src = fd ? job.pd : job.in;
+    ln.fd = fd;
     // scale of the line: its four threads sum the magnitudes of every fourth point
     OzSum sum;
-    if (act)
-      for (int n0 = h; n0 < N; n0 += 32) {
-        double v[8];
-        load8(v, n0, 4, (N - n0 + 3) >> 2);
-#pragma unroll
-        for (int i = 0; i < 8; ++i) {
-          const int n = n0 + 4 * i;
-          if (n < N && !(INV && job.deriv && n == 0)) sum.add(v[i], INV && job.deriv ? (unsigned)n * (n + 1) : 1u);
-        }
-      }
+    ln.magnitudes(sum, h);
     sS[tid] = sum.S;
     sE[tid] = sum.e | (sum.nz ? 0x10000 : 0);
     __syncthreads();
-    int K;
-    {
-      int e = 1;
-      bool nz = false;
-      for (int i = 0; i < 4; ++i) {
-        const int ei = sE[i * OZ_LINES + line];
-        e = max(e, ei & 0xffff);
-        nz = nz || (ei & 0x10000);
-      }
-      unsigned long long S = 4;
-      for (int i = 0; i < 4; ++i) S += sS[i * OZ_LINES + line] >> min(e - (sE[i * OZ_LINES + line] & 0xffff), 63);
-      K = min(61 - (64 - __clzll((long long)S)) - (e - 1043), 1083 - e);
-      if (!nz) K = FX_ZERO;
-      if (e == 2047) K = FX_NAN;
-    }
+    const int K = oz_scale(sS + line, sE + line, OZ_LINES);
     __syncthreads();  // sS is free
     const bool live = act && K != FX_ZERO && K != FX_NAN;
     for (int p = q0; p < q1; ++p) {
@@ -285,7 +319,7 @@ __global__ void __launch_bounds__(OZ_THREADS, 1) k_cheb_oz(const __grid_constant
         double v[8];
         if constexpr (INV) {
           const int n0 = 2 * k0 + q + (job.deriv ? 1 : 0);
-          load8(v, n0, 2, live ? (N - n0 + 1) >> 1 : 0);
+          ln.load8(v, n0, 2, live ? (N - n0 + 1) >> 1 : 0);
 #pragma unroll
           for (int e = 0; e < 8; ++e) x[e] = live ? fx_quant(v[e], K) : 0;
           if (job.deriv) {  // suffix sums: within the thread's points, then over the line's other threads
@@ -310,8 +344,8 @@ __global__ void __launch_bounds__(OZ_THREADS, 1) k_cheb_oz(const __grid_constant
           }
         } else {
           double w[8];
-          load8(v, k0, 1, live ? KR - k0 : 0);
-          load8(w, N - 1 - k0, -1, live ? N / 2 - k0 : 0);  // the middle point stands alone
+          ln.load8(v, k0, 1, live ? KR - k0 : 0);
+          ln.load8(w, N - 1 - k0, -1, live ? N / 2 - k0 : 0);  // the middle point stands alone
 #pragma unroll
           for (int e = 0; e < 8; ++e) {
             const long long xv = live ? fx_quant(v[e], K) : 0, xw = live ? fx_quant(w[e], K) : 0;
@@ -319,7 +353,7 @@ __global__ void __launch_bounds__(OZ_THREADS, 1) k_cheb_oz(const __grid_constant
           }
         }
         if ((h >> 1) < nks)
-          oz_store(As + (st * 2 + (h >> 1)) * OZ_ASTAGE + (line >> 3) * 256 + (h & 1) * 128 + (line & 7) * 16, x);
+          oz_store<1>(As + (st * 2 + (h >> 1)) * OZ_ASTAGE + (line >> 3) * 256 + (h & 1) * 128 + (line & 7) * 16, x);
         asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
         asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
         __syncthreads();
@@ -365,16 +399,10 @@ __global__ void __launch_bounds__(OZ_THREADS, 1) k_cheb_oz(const __grid_constant
         long long v[8];
 #pragma unroll
         for (int c = 0; c < 8; ++c) {
-          int d[OZ_DIGITS];
+          uint32_t w[OZ_DIGITS];
 #pragma unroll
-          for (int s = 0; s < OZ_DIGITS; ++s) d[s] = __float2int_rn(__uint_as_float(r[s][c]));
-          // sum_s d_s 2^(9 (6 - s) - 8)
-          long long x = (long long)(2 * d[5] + ((d[6] + 128) >> 8));
-          x = fx_mw(d[4], 1 << 10, x);
-          x = fx_mw(d[3], 1 << 19, x);
-          x = fx_mw(d[2], 1 << 28, x);
-          x += (long long)((unsigned long long)(((unsigned)d[0] << 14) + ((unsigned)d[1] << 5)) << 32);
-          v[c] = x;
+          for (int s = 0; s < OZ_DIGITS; ++s) w[s] = r[s][c];
+          v[c] = oz_sum(w);
         }
         const int r0 = 8 * cu, nr = min(8, rows - r0);
         if constexpr (INV) {
@@ -465,6 +493,241 @@ __global__ void __launch_bounds__(OZ_THREADS, 1) k_cheb_oz(const __grid_constant
   if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(tmem), "r"(tcols));
 }
 
+// ---------------------------------------------------------------------------
+// The same transforms of few lines of up to 64 points.  A CTA takes 32 lines of one job and both parities.  Its lines
+// stand four times in the MMA's 128 rows, once per quarter of tensor memory (a warp reads one quarter only), so that its 16
+// warps share out the digits (a warp: 8 points of one parity) and the sums (a warp: OZ_COLS columns).  The line scales are
+// summed as in k_cheb_oz and the products are exact: the results are the same bits.
+// Where k_cheb_oz has a few CTAs its time is one CTA's: issue slots 42% active, 3000 instructions a warp.  Ny = 35, 190
+// modes: inverse with curl 17.6 -> 10.0 us, forward 10.3 -> 8.1 us; FP64 steps 24x17x24 72.6 -> 64.4 us, 32x33x32 79.4 ->
+// 70.6 us, 40x41x40 96.8 -> 87.6 us.
+// ---------------------------------------------------------------------------
+constexpr int OZ_LS = 32;
+
+template <int C>
+__device__ __forceinline__ void oz_load(uint32_t ta, uint32_t* r) {
+  if constexpr (C == 4) {
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0, %1, %2, %3}, [%4];\n"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+                 : "r"(ta));
+  } else {
+    static_assert(C == 2, "columns a warp");
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x2.b32 {%0, %1}, [%2];\n" : "=r"(r[0]), "=r"(r[1]) : "r"(ta));
+  }
+}
+
+// C sums from the accumulators at ta (seven weights NT columns apart)
+template <int C>
+__device__ __forceinline__ void oz_sums(uint32_t ta, int NT, long long (&v)[C]) {
+  uint32_t r[OZ_DIGITS][C];
+#pragma unroll
+  for (int s = 0; s < OZ_DIGITS; ++s) oz_load<C>(ta + (uint32_t)(s * NT), r[s]);
+  asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory");
+#pragma unroll
+  for (int c = 0; c < C; ++c) {
+    uint32_t w[OZ_DIGITS];
+#pragma unroll
+    for (int s = 0; s < OZ_DIGITS; ++s) w[s] = r[s][c];
+    v[c] = oz_sum(w);
+  }
+}
+
+template <bool INV>
+__global__ void __launch_bounds__(OZ_THREADS, 1) k_cheb_oz_few(const __grid_constant__ OzArgs a) {
+  constexpr int C = INV ? 2 : 4;  // columns a warp
+  extern __shared__ __align__(128) unsigned char smem[];
+  const int N = a.N, NT = a.NT;
+  const OzJob& job = a.job[blockIdx.y];
+  const int bst = oz_bstage(NT);
+  unsigned char* As = smem;                                                               // [parity][K step]
+  unsigned char* Bs = As + 4 * OZ_ASTAGE;                                                 // [parity's K steps]
+  unsigned long long* sS = reinterpret_cast<unsigned long long*>(Bs + 4 * bst);           // [256]
+  int* sE = reinterpret_cast<int*>(sS + 8 * OZ_LS);                                       // [128]
+  uint64_t* mbar = reinterpret_cast<uint64_t*>(sE + 4 * OZ_LS);                           // matrix landed, products done
+  uint32_t* tslot = reinterpret_cast<uint32_t*>(mbar + 2);
+  const int tid = threadIdx.x, warp = tid >> 5, line = tid & 31;
+  const int gl = blockIdx.x * OZ_LS + line;
+  const bool act = gl < a.nlines;
+  const unsigned ld = a.ld;
+  const int acols = OZ_DIGITS * NT + 8;  // accumulators of a parity
+  uint32_t tcols = 32;
+  while ((int)tcols < 2 * acols) tcols *= 2;
+  const int KR[2] = {(N + 1) / 2, N / 2}, KS[2] = {(KR[0] + 15) / 16, (KR[1] + 15) / 16};
+  const uint32_t full = smem_u32(mbar), done = smem_u32(mbar + 1);
+
+  if (tid == 0) {
+    for (int i = 0; i < 2; ++i) asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;\n" ::"r"(smem_u32(mbar + i)));
+    asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
+  }
+  if (warp == 0) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;\n" ::"r"(smem_u32(tslot)), "r"(tcols));
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;\n");
+  }
+  asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
+  __syncthreads();
+  asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+  const uint32_t tmem = *tslot;
+  pdl_wait();  // the previous kernel's output is read from here on
+  pdl_trigger();
+  OzLine<INV> ln(a, job, gl, act);
+
+  bool ok = true;
+  const int nstage = INV || !job.pd ? 1 : 2;
+  for (int sg = 0; sg < nstage; ++sg) {
+    const bool fd = !INV && sg == 1;
+    const OzMatrix& M = INV ? a.t.T : (fd ? a.t.DF : a.t.F);
+    ln.src = fd ? job.pd : job.in;
+    ln.fd = fd;
+    if (tid == 0) {  // the previous stage's products have read their matrix
+      const uint32_t bytes = (uint32_t)((KS[0] + KS[1]) * bst);
+      asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n" ::"r"(full), "r"(bytes) : "memory");
+      asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];\n" ::"r"(
+                       smem_u32(Bs)),
+                   "l"(M.digits), "r"(bytes), "r"(full)
+                   : "memory");
+    }
+    if (warp < 4) {
+      OzSum sum;
+      ln.magnitudes(sum, warp);
+      sS[tid] = sum.S;
+      sE[tid] = sum.e | (sum.nz ? 0x10000 : 0);
+    }
+    __syncthreads();
+    const int K = oz_scale(sS + line, sE + line, OZ_LS);
+    const bool live = act && K != FX_ZERO && K != FX_NAN;
+    __syncthreads();  // sS is free
+
+    const int q = (warp >> 2) & 1, part = warp & 3, k0 = 8 * part;  // warps 0 ... 7: digits of 8 points of input parity q
+    long long x[8];
+    if (warp < 8) {
+      double v[8];
+      if constexpr (INV) {
+        const int n0 = 2 * k0 + q + (job.deriv ? 1 : 0);
+        ln.load8(v, n0, 2, live ? (N - n0 + 1) >> 1 : 0);
+#pragma unroll
+        for (int e = 0; e < 8; ++e) x[e] = live ? fx_quant(v[e], K) : 0;
+        if (job.deriv) {
+          long long acc = 0;
+#pragma unroll
+          for (int e = 7; e >= 0; --e) {
+            acc += x[e] * (2 * (n0 + 2 * e));
+            x[e] = acc;
+          }
+          sS[tid] = (unsigned long long)acc;
+        }
+      } else {
+        double w[8];
+        ln.load8(v, k0, 1, live ? KR[q] - k0 : 0);
+        ln.load8(w, N - 1 - k0, -1, live ? N / 2 - k0 : 0);  // the middle point stands alone
+#pragma unroll
+        for (int e = 0; e < 8; ++e) {
+          const long long xv = live ? fx_quant(v[e], K) : 0, xw = live ? fx_quant(w[e], K) : 0;
+          x[e] = q ? xv - xw : xv + xw;
+        }
+      }
+    }
+    if (INV && job.deriv) {
+      __syncthreads();
+      if (warp < 8) {
+        long long above = 0;
+        for (int i = part + 1; i < 4; ++i) above += (long long)sS[(4 * q + i) * OZ_LS + line];
+#pragma unroll
+        for (int e = 0; e < 8; ++e) x[e] += above;
+        if (2 * k0 + q == 0) x[0] >>= 1;
+      }
+    }
+    if (warp < 8 && (part >> 1) < KS[q])
+      oz_store<4>(As + (2 * q + (part >> 1)) * OZ_ASTAGE + (line >> 3) * 256 + (part & 1) * 128 + (line & 7) * 16, x);
+    asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
+    asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
+    __syncthreads();
+    if (tid == 0) {
+      asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+      if (mbar_wait(full, (uint32_t)(sg & 1))) {
+        for (int iq = 0; iq < 2; ++iq) {
+          const uint32_t acc = tmem + (uint32_t)((fd ? 1 - iq : iq) * acols);
+          for (int k = 0; k < KS[iq]; ++k) {
+            const uint32_t a0 = smem_u32(As + (2 * iq + k) * OZ_ASTAGE), b0 = smem_u32(Bs + (iq * KS[0] + k) * bst);
+            for (int i = 0; i < OZ_DIGITS; ++i) {
+              const int nc = (NT * (OZ_DIGITS - i) + 15) & ~15;
+              const uint32_t idesc = (1u << 4) | ((uint32_t)(nc >> 3) << 17) | ((uint32_t)(OZ_LINES >> 4) << 24);
+              mma_f16(acc + (uint32_t)(i * NT), oz_desc(a0 + i * (OZ_LINES * 32)), oz_desc(b0), idesc, k != 0 || i != 0);
+            }
+          }
+        }
+      } else {
+        ok = false;
+      }
+      asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n" ::"r"(done) : "memory");
+    }
+    if (!mbar_wait(done, (uint32_t)(sg & 1))) ok = false;
+    asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+    const uint32_t tq = tmem + ((uint32_t)(32 * (warp & 3)) << 16);
+    if constexpr (INV) {
+      for (int r0 = C * warp; r0 < KR[0]; r0 += C * 16) {
+        long long ev[C], od[C];
+        oz_sums<C>(tq + r0, NT, ev);
+        oz_sums<C>(tq + acols + r0, NT, od);
+        double y[2][C];
+#pragma unroll
+        for (int c = 0; c < C; ++c) {
+          y[0][c] = fx_to_double(r0 + c < N / 2 ? ev[c] + od[c] : ev[c], K);
+          y[1][c] = fx_to_double(ev[c] - od[c], K);
+        }
+        if (job.deriv && a.dscale != 1.0) {
+#pragma unroll
+          for (int c = 0; c < C; ++c) {
+            y[0][c] *= a.dscale;
+            y[1][c] *= a.dscale;
+          }
+        }
+        const unsigned o0 = (unsigned)r0 * ld + gl, o1 = (unsigned)(N - 1 - r0) * ld + gl;
+        const bool w0[2] = {act && r0 < KR[0], act && r0 + 1 < KR[0]}, w1[2] = {act && r0 < N / 2, act && r0 + 1 < N / 2};
+#pragma unroll
+        for (int c = 0; c < C; ++c) {
+          if (w0[c]) job.out[o0 + c * ld] = y[0][c];
+          if (w1[c]) job.out[o1 - c * ld] = y[1][c];
+        }
+        if (job.gx) {
+#pragma unroll
+          for (int c = 0; c < C; ++c) {
+            const double y0 = __shfl_xor_sync(0xffffffffu, y[0][c], 1), y1 = __shfl_xor_sync(0xffffffffu, y[1][c], 1);
+            if (w0[c]) {
+              job.gx[o0 + c * ld] = ln.kx * y0;
+              job.gz[o0 + c * ld] = ln.kz * y0;
+            }
+            if (w1[c]) {
+              job.gx[o1 - c * ld] = ln.kx * y1;
+              job.gz[o1 - c * ld] = ln.kz * y1;
+            }
+          }
+        }
+      }
+    } else {
+      const int p = warp >> 3, rows = KR[p];
+      const int* rexp = M.rexp + p * NT;
+      for (int r0 = C * (warp & 7); r0 < rows; r0 += C * 8) {
+        long long v[C];
+        oz_sums<C>(tq + (uint32_t)(p * acols + r0), NT, v);
+        double y[C];
+#pragma unroll
+        for (int c = 0; c < C; ++c) {
+          const bool in = act && r0 + c < rows;
+          y[c] = fx_to_double(v[c], r0 + c < rows ? K + rexp[r0 + c] : 0);
+          double* out = job.out + (unsigned)(2 * (r0 + c) + p) * ld + gl;
+          if (fd && in) y[c] = fma(job.wD, y[c], *out);
+          if (in) *out = y[c];
+        }
+      }
+    }
+    asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
+    __syncthreads();  // sS, sE, accumulators of the next stage
+    asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+  }
+  if (!ok && a.err) atomicExch(a.err, 1);
+  if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(tmem), "r"(tcols));
+}
+
 int oz_nt(int N) { return ((N + 1) / 2 + 7) & ~7; }
 
 uint16_t half_of_int(int d) {  // exact: |d| <= 256
@@ -479,6 +742,26 @@ size_t oz_smem(int N, int ring, bool held) {
   const int NT = oz_nt(N);
   return ring * 2 * (size_t)(OZ_ASTAGE + oz_bstage(NT)) + OZ_THREADS * 12 + 4 * 8 + 16 +
          (held ? (size_t)NT * OZ_LINES * 8 : 0);
+}
+
+// Whether k_cheb_oz_few runs: both parities' accumulators within tensor memory (Ny <= 64) and, beside 152 SMs, CTAs for one
+// wave (forward: k_cheb_oz splits its parities over CTAs) or one and a half (inverse).  FP64 steps with k_cheb_oz and with
+// this: inverse of 155 CTAs (48x49x48) 97.9 and 94.0 us, of 220 (54x33x60) 102.8 and 102.1; forward of 186 CTAs (72x49x64)
+// 124.4 and 130.1; both beyond the lines (72x33x54: 159 and 265 CTAs) 109.4 and 112.5.
+bool oz_few(bool inverse, int N, int nlines, int njobs) {
+  return 2 * (OZ_DIGITS * oz_nt(N) + 8) <= 512 &&
+         (long)((nlines + OZ_LS - 1) / OZ_LS) * njobs <= (inverse ? 152 * 3 / 2 : 152);
+}
+
+template <bool INV>
+cudaError_t run_oz_few(OzArgs& a, int njobs, cudaStream_t st) {
+  static const bool attr = [] {
+    cudaFuncSetAttribute(k_cheb_oz_few<INV>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
+    return true;
+  }();
+  (void)attr;
+  const size_t smem = 4 * (size_t)(OZ_ASTAGE + oz_bstage(a.NT)) + OZ_LS * (8 * 8 + 4 * 4) + 2 * 8 + 16;
+  return launch_pdl(k_cheb_oz_few<INV>, dim3((a.nlines + OZ_LS - 1) / OZ_LS, njobs), dim3(OZ_THREADS), smem, st, a);
 }
 
 template <bool INV>
@@ -602,6 +885,7 @@ cudaError_t launch_cheb_oz(const GridDev& g, int N, bool inverse, int nlines, si
     a.job[i] = jobs[i];
     inplace = inplace || jobs[i].inplace;
   }
+  if (oz_few(inverse, N, nlines, njobs)) return inverse ? run_oz_few<true>(a, njobs, st) : run_oz_few<false>(a, njobs, st);
   if (inverse) return run_oz<true>(a, njobs, inplace, st);
   a.split = !inplace;  // the forward parities are independent: one CTA each
   return run_oz<false>(a, njobs, inplace, st);

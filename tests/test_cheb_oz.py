@@ -88,3 +88,22 @@ def test_nonlinear_matches_oracle(Ny, form):
         finally:
             L.check(L.load().cfgpu_set_fused_xz(1))
         assert rel_l2(f, ref, g) <= 100 * Ny * EPS
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("Ny", [3, 16, 17, 33, 34, 49, 63, 64])
+def test_few_lines_same_bits(Ny):
+    """One component (CTAs of 32 lines) and the same one among seven (CTAs of 128): exact products, equal results."""
+    from channelflow_gb300.flowfield import FlowField, Physical, Spectral
+    Nx, Nz = 30, 36
+    x = np.random.default_rng(Ny).standard_normal((7, Ny, Nx, Nz + 2)) * (0.8 ** np.arange(Ny))[None, :, None, None]
+    x[0, :, 3, 4] = 0
+    x[0, Ny // 2, 5, 6] = np.nan
+    for state, go in ((Spectral, "makePhysical_y"), (Physical, "makeSpectral_y")):
+        got = []
+        for Nd in (7, 1):
+            f = FlowField(Nx, Ny, Nz, Nd, 2.0, 1.0)
+            f.set_raw(np.ascontiguousarray(x[:Nd]), Spectral, state)
+            getattr(f, go)()
+            got.append(f.raw().reshape(x[:Nd].shape)[0])
+        assert np.array_equal(got[0], got[1], equal_nan=True)
