@@ -3,9 +3,10 @@
 // GB300 issues one FP64 warp instruction per 64 cycles and SM sub-partition, but a 64-bit integer addition
 // (IADD3 pair) in about 2 and a 32 x 32 -> 64 bit multiply-add (IMAD.WIDE) in about 5 (measured with a
 // throughput probe).  An FFT is mostly additions, so the FP64 path's transforms run on integers: a sequence is
-// scaled by one power of two such that the sum of the magnitudes of its elements stays below 2^61, which bounds
-// every intermediate value of the transform, and rounded to integers.  Its rounding errors are a few units of
-// 2^-61 of that sum, below those of the same FFT in FP64 (whose units are 2^-53 of the local values).
+// scaled by one power of two such that the sum of the magnitudes of its elements (real plus imaginary) stays below
+// 2^61, which bounds the modulus of every intermediate value of the transform, and rounded to integers.  Its rounding
+// errors are a few units of 2^-61 of that sum, below those of the same FFT in FP64 (whose units are 2^-53 of the local
+// values).
 //
 // Twiddle factors are fixed-point too: c = (h 2^32 + l) 2^-62 with signed 32-bit h, l.  A complex product with
 // components a = ah 2^32 + al (al signed) sums the cross terms ah l + al h of both real products in one 64-bit
@@ -25,7 +26,7 @@ __device__ __forceinline__ fxc fx_add(fxc a, fxc b) { return fxc{a.x + b.x, a.y 
 __device__ __forceinline__ fxc fx_sub(fxc a, fxc b) { return fxc{a.x - b.x, a.y - b.y}; }
 __device__ __forceinline__ long long fx_mw(int a, int b, long long c) { return (long long)a * b + c; }
 
-// a w; |a.x| + |a.y| <= 2^61.
+// a w; |a.x|, |a.y| < 2^61 (of a modulus below 2^61, so that the result's components are too).
 __device__ __forceinline__ fxc fx_cmul(fxc a, fxtw w) {
   const int xh = w.x, xl = w.y, yh = w.z, yl = w.w, nh = -w.z, nl = -w.w;
   const int al = (int)a.x, bl = (int)a.y;
@@ -37,10 +38,17 @@ __device__ __forceinline__ fxc fx_cmul(fxc a, fxtw w) {
   return fxc{fx_mw(b4, nh, fx_mw(a4, xh, mx >> 30)), fx_mw(a4, yh, fx_mw(b4, xh, my >> 30))};
 }
 
-// a c for a real constant c = (h 2^32 + l) 2^-62, |a| <= 2^61.
+// a c for a real constant c = (h 2^32 + l) 2^-62, |a| < 2^61.
 __device__ __forceinline__ long long fx_mulc(long long a, int h, int l) {
   const int al = (int)a, ah = (int)(a >> 32) + (int)((unsigned)al >> 31);
   return fx_mw(ah << 2, h, fx_mw(al, h, fx_mw(ah, l, 1ll << 29)) >> 30);
+}
+
+// The same for |a| < 2^62: the sum of both components of a number whose modulus is below 2^61 reaches sqrt(2) 2^61, which
+// four times its high half would carry out of 32 bits.  The product is shifted instead.
+__device__ __forceinline__ long long fx_mulc_sum(long long a, int h, int l) {
+  const int al = (int)a, ah = (int)(a >> 32) + (int)((unsigned)al >> 31);
+  return ((long long)ah * h << 2) + (fx_mw(al, h, fx_mw(ah, l, 1ll << 29)) >> 30);
 }
 
 // a b 2^-64 for |a|, |b| < 2^61, without the product of the low halves (below one unit).
@@ -48,18 +56,6 @@ __device__ __forceinline__ long long fx_mulhi(long long a, long long b) {
   const int al = (int)a, bl = (int)b;
   const int ah = (int)(a >> 32) + (int)((unsigned)al >> 31), bh = (int)(b >> 32) + (int)((unsigned)bl >> 31);
   return fx_mw(ah, bh, fx_mw(al, bh, (long long)ah * bl) >> 32);
-}
-
-// Host: the split of c (|c| <= 1).
-inline void fx_split(long double c, int& h, int& l) {
-  const long double s = c * 4611686018427387904.0L;  // 2^62
-  long long v = (long long)(s < 0 ? s - 0.5L : s + 0.5L);
-  l = (int)(uint32_t)(v & 0xffffffffll);
-  if (l == INT32_MIN) {  // negated in the conjugate product: keep -l representable
-    l += 1;
-    v += 1;
-  }
-  h = (int)((v - l) >> 32);
 }
 
 // ---------------------------------------------------------------------------

@@ -5,6 +5,7 @@
 
 #include "fft.cuh"
 #include "fx.cuh"
+#include "fx_plan.h"
 
 // Constants of the butterflies, split as above (2^62 times the value, rounded).
 namespace fxk {
@@ -24,6 +25,12 @@ __device__ __forceinline__ long long mul(long long a) {
   return fx_mulc(a, h, l);
 }
 template <long long C>
+__device__ __forceinline__ long long mul_sum(long long a) {
+  constexpr int l = (int)(uint32_t)((unsigned long long)C & 0xffffffffull);
+  constexpr int h = (int)((C - (long long)l) >> 32);
+  return fx_mulc_sum(a, h, l);
+}
+template <long long C>
 __device__ __forceinline__ fxc mul(fxc a) {
   return fxc{mul<C>(a.x), mul<C>(a.y)};
 }
@@ -41,7 +48,7 @@ __device__ __forceinline__ fxc fx_rot(fxc a) {
   } else if constexpr (4 * M == 3 * N) {
     return fxc{-a.y, a.x};
   } else if constexpr (8 * M % N == 0) {  // odd multiples of 45 degrees
-    const long long p = fxk::mul<fxk::kR>(a.x + a.y), q = fxk::mul<fxk::kR>(a.y - a.x);
+    const long long p = fxk::mul_sum<fxk::kR>(a.x + a.y), q = fxk::mul_sum<fxk::kR>(a.y - a.x);
     if constexpr (8 * M == N) return fxc{p, q};
     if constexpr (8 * M == 3 * N) return fxc{q, -p};
     if constexpr (8 * M == 5 * N) return fxc{-p, -q};
@@ -150,22 +157,6 @@ struct FxDft2 {
 };
 template <> struct FxDft<6> : FxDft2<2, 3> {};
 template <> struct FxDft<8> : FxDft2<2, 4> {};
-
-// Stages of a transform of length L: up to eight radices, eight bits each, first stage lowest.  Radices with a
-// butterfly in registers, or primes above 7 (direct DFT, roots behind the stage's twiddles).  Fewest stages first: each
-// costs a pass through shared memory and L (1 - 1 / radix) twiddle products (128 = 8 x 4 x 4: 192 and eighth turns,
-// 4 x 4 x 4 x 2: 256).  Radices up to 8 keep a kernel within 64 registers and four blocks an SM; up to 10 in 80
-// registers were level or slower, up to 16 in 128 registers 20-30% slower (z pass 128x97x128 158 us).
-struct FxPlan {
-  int L;
-  bool any;  // a radix of 7 or a larger prime
-  unsigned long long rad;
-};
-__host__ __device__ constexpr bool fx_composite(int r) {
-  return r >= 2 && r <= 8;
-}
-// twiddle entries of stage (radix R, Ns points before it)
-__host__ __device__ constexpr int fx_stage_tw(int R, int Ns) { return Ns * (R - 1) + (fx_composite(R) ? 0 : R); }
 
 // One Stockham stage over nseq sequences (fft.cuh's formulation), the length and the points before the stage known at
 // compile time (CL, CN) or not (0).  swin / swout: real and imaginary parts change places on the way in / out (an inverse

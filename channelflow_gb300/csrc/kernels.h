@@ -8,6 +8,7 @@
 #include <vector>
 
 #include "fft.cuh"
+#include "fx_plan.h"
 
 // Records the message returned by cfgpu_last_error() on this thread; returns code.
 int cfgpu_record_error(int code, const std::string& msg);
@@ -135,8 +136,7 @@ template <typename R>
 cudaError_t launch_xfwd(const GridDev& g, const FftPlan& px, const cpx<R>* twx, const void* twq, const cpx<R>* Z,
                         cpx<R>* F, int ncomp, cudaStream_t st, int czc = 0, const Dither& dt = kNoDither);
 
-// The FP64 passes on 64-bit integers (xz_fx.cu): fx_twiddles is the table of a length (four ints per entry).
-std::vector<int> fx_twiddles(int L);
+// The FP64 passes on 64-bit integers (xz_fx.cu); tw: fx_twiddles (fx_plan.h).
 // curl: W holds u, v, w, dw/dy, -, du/dy; components 3, 4, 5 transformed are the vorticity (launch_curl_points: in place)
 cudaError_t launch_xinv_fx(const GridDev& g, const FftPlan& px, const void* tw, const cpx<double>* W, cpx<double>* X,
                            int ncomp, int czc, bool curl, cudaStream_t st);

@@ -11,47 +11,8 @@
 // 116 us at 128x97x128, 402 -> 353 us at 192x129x160, 170 -> 143 us at 72x57x90 (skew-symmetric form).
 // Relative error of N(u) against extended precision: 1.5e-16 ... 2.5e-16 at 32x9x32 (FP64 arithmetic 2.7e-16 ...
 // 8.8e-16), for spectra from 0.5^(|kx|+|kz|) to flat.
-#include <algorithm>
-#include <atomic>
-#include <cmath>
-
 #include "fx_fft.cuh"
 #include "kernels.h"
-
-// Fewest stages, then the smallest radices, largest first; primes above 7 last.
-static void fx_search(int m, int maxr, unsigned long long cur, int n, int sum, int& bn, int& bsum, unsigned long long& best) {
-  if (m == 1) {
-    if (n < bn || (n == bn && sum < bsum)) {
-      bn = n;
-      bsum = sum;
-      best = cur;
-    }
-    return;
-  }
-  if (n + 1 > bn) return;
-  for (int r = std::min(maxr, m); r >= 2; --r)
-    if (m % r == 0 && fx_composite(r)) fx_search(m / r, r, cur | (unsigned long long)r << (8 * n), n + 1, sum + r, bn, bsum, best);
-}
-
-static FxPlan fx_plan(int L) {
-  static std::atomic<unsigned long long> known[8192];  // a function of L alone
-  if (L < 8192)
-    if (const unsigned long long k = known[L].load(std::memory_order_relaxed)) return FxPlan{L, k >> 63 != 0, k & ~(1ull << 63)};
-  int m = L, np = 0, primes[8];
-  for (int p = 11; p <= m; p += 2)
-    while (m % p == 0 && p % 3 && p % 5 && p % 7) {
-      primes[np++] = p;
-      m /= p;
-    }
-  int bn = 8, bsum = 0;
-  unsigned long long best = 0;
-  fx_search(m, 8, 0, 0, 0, bn, bsum, best);
-  for (int i = 0; i < np; ++i) best |= (unsigned long long)primes[i] << (8 * (bn + i));
-  bool any = false;
-  for (unsigned long long r = best; r; r >>= 8) any = any || (r & 255) == 7 || (r & 255) > 8;
-  if (L < 8192) known[L].store(best | (unsigned long long)any << 63, std::memory_order_relaxed);
-  return FxPlan{L, any, best};
-}
 
 namespace {
 
@@ -618,30 +579,6 @@ size_t xfx_smem(const GridDev& g, int czc, bool curl) {
 }
 
 }  // namespace
-
-// Per stage: exp(-2 pi i k r / (Ns R)) at [k (R - 1) + r - 1], then a prime's roots exp(-2 pi i e / R).
-std::vector<int> fx_twiddles(int L) {
-  std::vector<int> t;
-  auto push = [&](long long m, long long n) {
-    const long double x = 2 * 3.14159265358979323846264338327950288L * (long double)(m % n) / (long double)n;
-    const bool cz = 4 * (m % n) == n || 4 * (m % n) == 3 * n, sz = 2 * (m % n) % n == 0;
-    int v[4];
-    fx_split(cz ? 0.0L : cosl(x), v[0], v[1]);
-    fx_split(sz ? 0.0L : -sinl(x), v[2], v[3]);
-    t.insert(t.end(), v, v + 4);
-  };
-  unsigned long long rad = fx_plan(L).rad;
-  for (int Ns = 1; Ns < L; rad >>= 8) {
-    const int R = (int)(rad & 255);
-    for (int k = 0; k < Ns; ++k)
-      for (int r = 1; r < R; ++r) push((long long)k * r, (long long)Ns * R);
-    if (!fx_composite(R))
-      for (int e = 0; e < R; ++e) push(e, R);
-    Ns *= R;
-  }
-  if (t.empty()) t.resize(4);
-  return t;
-}
 
 // Shared memory of n sequences of length L with their exponents (two per sequence).
 static size_t field_smem(int L, int n) { return (2 * sizeof(fxc) * (size_t)(L + 1) + 2 * sizeof(int)) * n; }
