@@ -11,8 +11,11 @@
 //
 // Parity: the even and odd coefficients are two systems of half the size (T[N-1-j][n] = (-1)^n T[j][n]): the inverse
 // transform multiplies each parity's coefficients and combines y_j = E_j + O_j, y_{N-1-j} = E_j - O_j; the forward
-// transforms fold x_j +- x_{N-1-j} first.  The derivative of an inverse transform is taken on the integers before it
-// (d_n = d_{n+2} + 2 (n+1) X_{n+1}, exact).
+// transforms fold x_j +- x_{N-1-j} first.  The derivative of an inverse transform is taken before it, d_n = d_{n+2} + 2
+// (n+1) x_{n+1} in integers with 32 fraction bits, rounded once: coefficients rounded before their weights would be off
+// by up to N^2 units at the walls.  Relative error of N(u) for mean profiles with flat spectra, rounded before / here /
+// dense FP64 products: Ny = 49 4.3e-15 / 1.5e-16 / 4.8e-16, 97 2.6e-14 / 1.2e-16 / 6.0e-16, 139 8.9e-14 / 1.9e-16 /
+// 3.9e-16; FP64 step 128x97x128 519 -> 525 us.
 //
 // One CTA: 128 lines (the M rows of the MMA) of one job.  K runs in stages of two steps of 16 through a ring: 512
 // threads quantise 32 points of every line and write the digits as seven K-major operands a step (no swizzle: 8 x
@@ -22,7 +25,7 @@
 // + 8 columns; shared memory).
 //
 // Measured against FP64 arithmetic, which the FP64 pipe bounds (one warp instruction per 64 cycles).  128x97x128: curl
-// and inverse transforms 190 us (FFT form) -> 63 us and 15 us more in the x pass, which forms the vorticity; forward 91
+// and inverse transforms 190 us (FFT form) -> 68 us and 10 us more in the x pass, which forms the vorticity; forward 91
 // -> 56 us.  72x57x90, skew-symmetric: gradient 107 -> 28 us, forward with divergence 484 -> 43 us.  Ny = 35, 190 modes:
 // 29 -> 17 us and 24 -> 11 us (10 and 8 with k_cheb_oz_few).  FlowField y transform 128x97x128: 1340 -> 83 and 96 us.
 // Relative error of one transform 5e-17 (FP64 products 2e-16 ... 5e-16).  Bound by instruction issue and latency of the digits and the sums (16 warps
@@ -100,6 +103,30 @@ struct OzSum {
     S += (unsigned long long)((m >> min(e - ex, 31)) + 1u) * w;
   }
 };
+
+// An integer with 32 fraction bits.
+struct OzFix {
+  long long i;
+  unsigned f;
+};
+__device__ __forceinline__ OzFix oz_add(OzFix a, OzFix b) {
+  const unsigned f = a.f + b.f;
+  return OzFix{a.i + b.i + (f < b.f), f};
+}
+__device__ __forceinline__ long long oz_round(OzFix a) { return a.i + (a.f >> 31); }
+__device__ __forceinline__ OzFix oz_half(OzFix a) { return OzFix{a.i >> 1, (a.f >> 1) | ((unsigned)a.i << 31)}; }
+// w x 2^K for 0 <= w < 2^10 and K from oz_scale of a line whose scale counts x with at least this weight (the product is
+// below 2^61 and its shift at least -8), without what lies below 2^-32
+__device__ __forceinline__ OzFix oz_term(double x, int K, unsigned w) {
+  const int hi = __double2hiint(x);
+  const int e = (hi >> 20) & 0x7ff;
+  const unsigned long long m = ((unsigned long long)((hi & 0xfffff) | (e ? 0x100000 : 0)) << 32) | (unsigned)__double2loint(x);
+  const unsigned long long p = m * w;  // below 2^63
+  const int s = 1075 - K - max(e, 1);  // p 2^-s
+  const long long i = (long long)(s < 0 ? p << -s : p >> min(s, 63));
+  const unsigned f = (unsigned)(s < 32 ? p << (32 - s) : p >> min(s - 32, 63));
+  return hi < 0 ? OzFix{-i - (f != 0), 0u - f} : OzFix{i, f};
+}
 
 // Seven digits (most significant first) of the eight integers x[0..7], |x| < 2^61, as FP16 pairs; copies 32 rows apart.
 template <int COPIES>
@@ -294,13 +321,13 @@ __global__ void __launch_bounds__(OZ_THREADS, 1) k_cheb_oz(const __grid_constant
     sE[tid] = sum.e | (sum.nz ? 0x10000 : 0);
     __syncthreads();
     const int K = oz_scale(sS + line, sE + line, OZ_LINES);
-    __syncthreads();  // sS is free
+    __syncthreads();  // sS, sE are free
     const bool live = act && K != FX_ZERO && K != FX_NAN;
     for (int p = q0; p < q1; ++p) {
       const int q = fd ? 1 - p : p;  // input parity; a CTA's outputs stay of parity p
       const int KR = q ? N / 2 : (N + 1) / 2, KS = (KR + 15) / 16;
       const unsigned char* Mg = reinterpret_cast<const unsigned char*>(M.digits) + (q ? (size_t)(((N + 1) / 2 + 15) / 16) * bst : 0);
-      long long carry = 0;  // running derivative
+      OzFix carry{0, 0};  // running derivative
       const int last = (KS - 1) / 2;
       for (int pr = last; pr >= 0; --pr, ++t) {
         const int st = t % ring, use = t / ring, nks = min(KS - 2 * pr, 2);
@@ -320,27 +347,31 @@ __global__ void __launch_bounds__(OZ_THREADS, 1) k_cheb_oz(const __grid_constant
         if constexpr (INV) {
           const int n0 = 2 * k0 + q + (job.deriv ? 1 : 0);
           ln.load8(v, n0, 2, live ? (N - n0 + 1) >> 1 : 0);
-#pragma unroll
-          for (int e = 0; e < 8; ++e) x[e] = live ? fx_quant(v[e], K) : 0;
           if (job.deriv) {  // suffix sums: within the thread's points, then over the line's other threads
-            long long acc = 0;
+            OzFix d[8], acc{0, 0};
 #pragma unroll
             for (int e = 7; e >= 0; --e) {
-              acc += x[e] * (2 * (n0 + 2 * e));
-              x[e] = acc;
+              if (live) acc = oz_add(acc, oz_term(v[e], K, 2 * (n0 + 2 * e)));
+              d[e] = acc;
             }
-            sS[tid] = (unsigned long long)acc;
+            sS[tid] = (unsigned long long)acc.i;
+            sE[tid] = (int)acc.f;
             __syncthreads();
-            long long above = carry;
+            OzFix above = carry;
 #pragma unroll
             for (int i = 3; i >= 0; --i) {
-              const long long ti = (long long)sS[i * OZ_LINES + line];
-              if (i > h) above += ti;
-              carry += ti;
+              const OzFix ti{(long long)sS[i * OZ_LINES + line], (unsigned)sE[i * OZ_LINES + line]};
+              if (i > h) above = oz_add(above, ti);
+              carry = oz_add(carry, ti);
             }
 #pragma unroll
-            for (int e = 0; e < 8; ++e) x[e] += above;
-            if (n0 == 1) x[0] >>= 1;
+            for (int e = 0; e < 8; ++e) d[e] = oz_add(d[e], above);
+            if (n0 == 1) d[0] = oz_half(d[0]);
+#pragma unroll
+            for (int e = 0; e < 8; ++e) x[e] = oz_round(d[e]);
+          } else {
+#pragma unroll
+            for (int e = 0; e < 8; ++e) x[e] = live ? fx_quant(v[e], K) : 0;
           }
         } else {
           double w[8];
@@ -542,8 +573,8 @@ __global__ void __launch_bounds__(OZ_THREADS, 1) k_cheb_oz_few(const __grid_cons
   unsigned char* As = smem;                                                               // [parity][K step]
   unsigned char* Bs = As + 4 * OZ_ASTAGE;                                                 // [parity's K steps]
   unsigned long long* sS = reinterpret_cast<unsigned long long*>(Bs + 4 * bst);           // [256]
-  int* sE = reinterpret_cast<int*>(sS + 8 * OZ_LS);                                       // [128]
-  uint64_t* mbar = reinterpret_cast<uint64_t*>(sE + 4 * OZ_LS);                           // matrix landed, products done
+  int* sE = reinterpret_cast<int*>(sS + 8 * OZ_LS);                                       // [256]
+  uint64_t* mbar = reinterpret_cast<uint64_t*>(sE + 8 * OZ_LS);                           // matrix landed, products done
   uint32_t* tslot = reinterpret_cast<uint32_t*>(mbar + 2);
   const int tid = threadIdx.x, warp = tid >> 5, line = tid & 31;
   const int gl = blockIdx.x * OZ_LS + line;
@@ -595,25 +626,28 @@ __global__ void __launch_bounds__(OZ_THREADS, 1) k_cheb_oz_few(const __grid_cons
     __syncthreads();
     const int K = oz_scale(sS + line, sE + line, OZ_LS);
     const bool live = act && K != FX_ZERO && K != FX_NAN;
-    __syncthreads();  // sS is free
+    __syncthreads();  // sS, sE are free
 
     const int q = (warp >> 2) & 1, part = warp & 3, k0 = 8 * part;  // warps 0 ... 7: digits of 8 points of input parity q
     long long x[8];
+    OzFix d[8];  // derivative
     if (warp < 8) {
       double v[8];
       if constexpr (INV) {
         const int n0 = 2 * k0 + q + (job.deriv ? 1 : 0);
         ln.load8(v, n0, 2, live ? (N - n0 + 1) >> 1 : 0);
-#pragma unroll
-        for (int e = 0; e < 8; ++e) x[e] = live ? fx_quant(v[e], K) : 0;
         if (job.deriv) {
-          long long acc = 0;
+          OzFix acc{0, 0};
 #pragma unroll
           for (int e = 7; e >= 0; --e) {
-            acc += x[e] * (2 * (n0 + 2 * e));
-            x[e] = acc;
+            if (live) acc = oz_add(acc, oz_term(v[e], K, 2 * (n0 + 2 * e)));
+            d[e] = acc;
           }
-          sS[tid] = (unsigned long long)acc;
+          sS[tid] = (unsigned long long)acc.i;
+          sE[tid] = (int)acc.f;
+        } else {
+#pragma unroll
+          for (int e = 0; e < 8; ++e) x[e] = live ? fx_quant(v[e], K) : 0;
         }
       } else {
         double w[8];
@@ -629,11 +663,16 @@ __global__ void __launch_bounds__(OZ_THREADS, 1) k_cheb_oz_few(const __grid_cons
     if (INV && job.deriv) {
       __syncthreads();
       if (warp < 8) {
-        long long above = 0;
-        for (int i = part + 1; i < 4; ++i) above += (long long)sS[(4 * q + i) * OZ_LS + line];
+        OzFix above{0, 0};
+        for (int i = part + 1; i < 4; ++i) {
+          const int o = (4 * q + i) * OZ_LS + line;
+          above = oz_add(above, OzFix{(long long)sS[o], (unsigned)sE[o]});
+        }
 #pragma unroll
-        for (int e = 0; e < 8; ++e) x[e] += above;
-        if (2 * k0 + q == 0) x[0] >>= 1;
+        for (int e = 0; e < 8; ++e) d[e] = oz_add(d[e], above);
+        if (2 * k0 + q == 0) d[0] = oz_half(d[0]);
+#pragma unroll
+        for (int e = 0; e < 8; ++e) x[e] = oz_round(d[e]);
       }
     }
     if (warp < 8 && (part >> 1) < KS[q])
@@ -760,7 +799,7 @@ cudaError_t run_oz_few(OzArgs& a, int njobs, cudaStream_t st) {
     return true;
   }();
   (void)attr;
-  const size_t smem = 4 * (size_t)(OZ_ASTAGE + oz_bstage(a.NT)) + OZ_LS * (8 * 8 + 4 * 4) + 2 * 8 + 16;
+  const size_t smem = 4 * (size_t)(OZ_ASTAGE + oz_bstage(a.NT)) + OZ_LS * (8 * 8 + 8 * 4) + 2 * 8 + 16;
   return launch_pdl(k_cheb_oz_few<INV>, dim3((a.nlines + OZ_LS - 1) / OZ_LS, njobs), dim3(OZ_THREADS), smem, st, a);
 }
 
