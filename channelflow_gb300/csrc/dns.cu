@@ -635,7 +635,7 @@ struct cfgpu_dns_s {
   // transforms
   FftPlan px{}, pz{};
   void *twx = nullptr, *twz = nullptr;  // R-typed complex
-  void *twxq = nullptr, *twzq = nullptr;  // FP64: fixed-point tables (fx_twiddles)
+  void *twxq = nullptr, *twzq = nullptr;  // FP64 lines of up to FX_LMAX points: fixed-point tables (fx_twiddles)
   // FP64 Chebyshev transforms on the tensor cores (cheb_oz.cu): tables in one block, off where Ny is not covered
   bool oz = false;
   OzTables ozt{};
@@ -930,7 +930,7 @@ int nonlinear_impl(cfgpu_dns d, const double* U, void* Nout, int form) {
       if (d->oz) {
         CKS(oz_curl(d, U, W, d->fl.Vsuck));
         done = true;
-        if (d->xzf) {
+        if (d->xzf || g.Nx > FX_LMAX) {
           CK(launch_curl_points(gp, (cpx<double>*)W, d->st));
           d->launches += 1;
         } else {
@@ -2012,10 +2012,9 @@ int dns_create_impl(cfgpu_dns d, const cfgpu_grid* grid, const cfgpu_flags* flag
   for (auto* t : {&cm.derA, &cm.derB, &cm.dfA, &cm.dfB})
     for (auto& v : *t) v *= 2.0 / (b - a);
   if (fp64) {
-    CKS(upload_tw<double>(twx, &d->twx, B, d->st));
-    CKS(upload_tw<double>(twz, &d->twz, B, d->st));
-    CKS(upload_ints(fx_twiddles(Nx), &d->twxq, B, d->st));
-    CKS(upload_ints(fx_twiddles(Nz), &d->twzq, B, d->st));
+    CKS(Nx <= FX_LMAX ? upload_ints(fx_twiddles(Nx), &d->twxq, B, d->st) : upload_tw<double>(twx, &d->twx, B, d->st));
+    if (Nz <= FX_LMAX) CKS(upload_ints(fx_twiddles(Nz), &d->twzq, B, d->st));
+    CKS(upload_tw<double>(twz, &d->twz, B, d->st));  // the CFL pass at any Nz
     CKS(upload_as<double>(circx, &d->twxf, B, d->st));
     CKS(upload_as<double>(circz, &d->twzf, B, d->st));
     CKS(upload_as<double>(basey, &d->basey, B, d->st));

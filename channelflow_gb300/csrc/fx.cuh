@@ -5,8 +5,8 @@
 // throughput probe).  An FFT is mostly additions, so the FP64 path's transforms run on integers: a sequence is
 // scaled by one power of two such that the sum of the magnitudes of its elements (real plus imaginary) stays below
 // 2^61, which bounds the modulus of every intermediate value of the transform, and rounded to integers.  Its rounding
-// errors are a few units of 2^-61 of that sum, below those of the same FFT in FP64 (whose units are 2^-53 of the local
-// values).
+// errors are a few units of 2^-61 of that sum: up to FX_LMAX points (fx_plan.h) below those of the same FFT in FP64, whose
+// units are 2^-53 of the local values.
 //
 // Twiddle factors are fixed-point too: c = (h 2^32 + l) 2^-62 with signed 32-bit h, l.  A complex product with
 // components a = ah 2^32 + al (al signed) sums the cross terms ah l + al h of both real products in one 64-bit

@@ -9,6 +9,14 @@
 #include <cmath>
 #include <vector>
 
+// Longest line on fixed point; longer ones take FP64 arithmetic (fft.cuh).  The scale allows for the sum of magnitudes,
+// so the error of flat data grows with the length, that of a double-precision FFT only with the root of its logarithm.
+// Relative rms error of flat lines, the worst of their amplitudes within a power of two, fixed point / double: 128
+// 6.9e-17 / 1.9e-16, 300 2.2e-16 / 2.6e-16, 336 2.0e-16 / 2.3e-16, 360 2.4e-16 / 2.4e-16, 512 2.6e-16 / 2.1e-16, 1024
+// 4.9e-16 / 2.3e-16, 3000 1.5e-15 / 2.6e-16.  Lines with decaying spectra are the more exact on fixed point at every
+// length.
+constexpr int FX_LMAX = 336;
+
 // Stages of a transform of length L: up to eight radices, eight bits each, first stage lowest.  Radices with a
 // butterfly in registers, or primes above 7 (direct DFT, roots behind the stage's twiddles).  Fewest stages first: each
 // costs a pass through shared memory and L (1 - 1 / radix) twiddle products (128 = 8 x 4 x 4: 192 and eighth turns,

@@ -100,7 +100,7 @@ size_t zphys_smem_bytes(const GridDev& g, int form, int RP);
 // z pass of the x/z path (c2r, the form's products, r2c).  With twzf (the full-circle twiddle table
 // exp(-2 pi i e / Nz), e < Nz) the FP32 rotational form runs with register-resident FFTs where Nz allows
 // (launch_zrot, csrc/z_reg.cu), else the generic Stockham kernel.  FP64 runs on 64-bit integers (csrc/xz_fx.cu) with
-// the twiddles twq = fx_twiddles(Nz); twz is unused there.
+// the twiddles twq = fx_twiddles(Nz) up to Nz = FX_LMAX, twz unused, and on the generic kernel beyond.
 template <typename R>
 cudaError_t launch_zphys(const GridDev& g, int form, const FftPlan& pz, const cpx<R>* twz, const void* twq, int RP,
                          const cpx<R>* X, cpx<R>* Z, cudaStream_t st, const Dither& dt = kNoDither,
@@ -127,7 +127,8 @@ cudaError_t launch_rotation(const GridDev& g, int N, const double* U, const doub
 template <typename R>
 size_t xfft_smem_bytes(const GridDev& g, int czc = 0);  // czc <= 0: all solved kz columns that fit
 
-// x passes: czc kz columns per block (0: as many as fit in shared memory); FP64 on 64-bit integers, as the z pass
+// x passes: czc kz columns per block (0: as many as fit in shared memory); FP64 on 64-bit integers up to Nx = FX_LMAX, as
+// the z pass; curl (launch_xinv_fx) there only
 template <typename R>
 cudaError_t launch_xinv(const GridDev& g, const FftPlan& px, const cpx<R>* twx, const void* twq, const cpx<R>* W,
                         cpx<R>* X, int ncomp, cudaStream_t st, int czc = 0, const Dither& dt = kNoDither,
@@ -143,8 +144,8 @@ cudaError_t launch_xinv_fx(const GridDev& g, const FftPlan& px, const void* tw, 
 cudaError_t launch_curl_points(const GridDev& g, cpx<double>* W, cudaStream_t st);
 cudaError_t launch_xfwd_fx(const GridDev& g, const FftPlan& px, const void* tw, const cpx<double>* Z, cpx<double>* F,
                            int ncomp, int czc, cudaStream_t st);
-// Whole-FlowField passes, in place: FFT along x of the Mz columns of nplanes planes [x][Mz] (times scale); c2r (inverse)
-// or r2c of nrows rows of Nz + 2 doubles.  One sequence with its copy fits in shared memory: lengths up to 7200.
+// Whole-FlowField passes of lines up to FX_LMAX, in place: FFT along x of the Mz columns of nplanes planes [x][Mz] (times
+// scale); c2r (inverse) or r2c of nrows rows of Nz + 2 doubles.
 cudaError_t launch_field_x(int Nx, int Mz, int nplanes, const void* tw, int sign, double scale,
                            cpx<double>* data, cudaStream_t st);
 cudaError_t launch_field_z(long long nrows, int Nz, bool inverse, const void* tw, double* data,

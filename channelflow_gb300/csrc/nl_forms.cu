@@ -498,7 +498,7 @@ size_t zphys_smem_bytes(const GridDev& g, int form, int RP) {
   if (form == NL_DIVERGENCE) { nc = 3; no = 6; }
   if (form == NL_SKEW) { nc = 12; no = 9; }
   const int nseq = ((nc > no ? nc : no) * RP) / 2;
-  const size_t fx = sizeof(R) == 8 ? 6 * sizeof(int) * (size_t)nseq : 0;  // the FP64 pass's exponents (xz_fx.cu)
+  const size_t fx = sizeof(R) == 8 && g.Nz <= FX_LMAX ? 6 * sizeof(int) * (size_t)nseq : 0;  // exponents (xz_fx.cu)
   return 2 * sizeof(cpx<R>) * (size_t)nseq * (g.Nz + 1) + fx;
 }
 
@@ -519,18 +519,18 @@ template <typename R>
 cudaError_t launch_zphys(const GridDev& g, int form, const FftPlan& pz, const cpx<R>* twz, const void* twq, int RP,
                          const cpx<R>* X, cpx<R>* Z, cudaStream_t st, const Dither& dt, const cpx<R>* twzf) {
   if constexpr (sizeof(R) == 8) {
-    return launch_zphys_fx(g, form, pz, twq, RP, X, Z, st);
+    if (g.Nz <= FX_LMAX) return launch_zphys_fx(g, form, pz, twq, RP, X, Z, st);
   } else {
     if (form == NL_ROTATIONAL && twzf) {
       const cudaError_t e = launch_zrot(g, RP, X, Z, twzf, st, dt);
       if (e != cudaErrorNotSupported) return e;
     }
-    switch (form) {
-      case NL_ROTATIONAL: return launch_zphys_t<R, NL_ROTATIONAL>(g, pz, twz, RP, X, Z, st, dt);
-      case NL_CONVECTION: return launch_zphys_t<R, NL_CONVECTION>(g, pz, twz, RP, X, Z, st, dt);
-      case NL_DIVERGENCE: return launch_zphys_t<R, NL_DIVERGENCE>(g, pz, twz, RP, X, Z, st, dt);
-      default: return launch_zphys_t<R, NL_SKEW>(g, pz, twz, RP, X, Z, st, dt);
-    }
+  }
+  switch (form) {
+    case NL_ROTATIONAL: return launch_zphys_t<R, NL_ROTATIONAL>(g, pz, twz, RP, X, Z, st, dt);
+    case NL_CONVECTION: return launch_zphys_t<R, NL_CONVECTION>(g, pz, twz, RP, X, Z, st, dt);
+    case NL_DIVERGENCE: return launch_zphys_t<R, NL_DIVERGENCE>(g, pz, twz, RP, X, Z, st, dt);
+    default: return launch_zphys_t<R, NL_SKEW>(g, pz, twz, RP, X, Z, st, dt);
   }
 }
 

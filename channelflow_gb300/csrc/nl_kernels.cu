@@ -648,37 +648,34 @@ template <typename R>
 cudaError_t launch_xinv(const GridDev& g, const FftPlan& px, const cpx<R>* twx, const void* twq, const cpx<R>* W,
                         cpx<R>* X, int ncomp, cudaStream_t st, int czc, const Dither& dt, bool curl) {
   if (czc <= 0 || czc > g.NKz) czc = xfft_cols<R>(g);
-  if constexpr (sizeof(R) == 8) {
-    return launch_xinv_fx(g, px, twq, W, X, ncomp, czc, curl, st);
-  } else {
-    // kernel attributes set once per process (thread-safe static initialisation)
-    static const bool attr_set = [] {
-      cudaFuncSetAttribute(k_xinv<R>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
-      return true;
-    }();
-    (void)attr_set;
-    return launch_pdl(k_xinv<R>, dim3(g.Ny, ncomp, (g.NKz + czc - 1) / czc), dim3(256), xfft_smem_bytes<R>(g, czc), st,
-                      g, px, twx, W, X, czc, dt);
-  }
+  if constexpr (sizeof(R) == 8)
+    if (g.Nx <= FX_LMAX) return launch_xinv_fx(g, px, twq, W, X, ncomp, czc, curl, st);
+  if (curl) return cudaErrorInvalidValue;  // of the fixed-point pass
+  // kernel attributes set once per process (thread-safe static initialisation)
+  static const bool attr_set = [] {
+    cudaFuncSetAttribute(k_xinv<R>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
+    return true;
+  }();
+  (void)attr_set;
+  return launch_pdl(k_xinv<R>, dim3(g.Ny, ncomp, (g.NKz + czc - 1) / czc), dim3(256), xfft_smem_bytes<R>(g, czc), st,
+                    g, px, twx, W, X, czc, dt);
 }
 
 template <typename R>
 cudaError_t launch_xfwd(const GridDev& g, const FftPlan& px, const cpx<R>* twx, const void* twq, const cpx<R>* Z,
                         cpx<R>* F, int ncomp, cudaStream_t st, int czc, const Dither& dt) {
   if (czc <= 0 || czc > g.NKz) czc = xfft_cols<R>(g);
-  if constexpr (sizeof(R) == 8) {
-    return launch_xfwd_fx(g, px, twq, Z, F, ncomp, czc, st);
-  } else {
-    // kernel attributes set once per process (thread-safe static initialisation)
-    static const bool attr_set = [] {
-      cudaFuncSetAttribute(k_xfwd<R>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
-      return true;
-    }();
-    (void)attr_set;
-    const double scale = 1.0 / ((double)g.Nx * (double)g.Nz);
-    return launch_pdl(k_xfwd<R>, dim3(g.Ny, ncomp, (g.NKz + czc - 1) / czc), dim3(256), xfft_smem_bytes<R>(g, czc), st,
-                      g, px, twx, Z, F, scale, czc, dt);
-  }
+  if constexpr (sizeof(R) == 8)
+    if (g.Nx <= FX_LMAX) return launch_xfwd_fx(g, px, twq, Z, F, ncomp, czc, st);
+  // kernel attributes set once per process (thread-safe static initialisation)
+  static const bool attr_set = [] {
+    cudaFuncSetAttribute(k_xfwd<R>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
+    return true;
+  }();
+  (void)attr_set;
+  const double scale = 1.0 / ((double)g.Nx * (double)g.Nz);
+  return launch_pdl(k_xfwd<R>, dim3(g.Ny, ncomp, (g.NKz + czc - 1) / czc), dim3(256), xfft_smem_bytes<R>(g, czc), st,
+                    g, px, twx, Z, F, scale, czc, dt);
 }
 
 #define INST_R(R)                                                                                                   \

@@ -23,6 +23,8 @@
 //   launch_field_x (xz_fx.cu)  complex FFT along x of kz columns of one (y, component) plane, in place
 //   launch_field_z (xz_fx.cu)  z transform of x rows: c2r (Hermitian completion, FFTW's convention of taking only the
 //                 real parts of the kz = 0 and Nz/2 terms) or r2c, in place
+//   k_long_x, k_long_z  the same of lines longer than FX_LMAX (fx_plan.h), in FP64 arithmetic (fft.cuh), the more exact
+//                 there
 // The FFTs run on 64-bit integers (fx.cuh); against the same passes in FP64 arithmetic, 128x97x128, three components:
 // z 247 -> 51 us, x 135 -> 48 us.
 #include "../../include/cfgpu.h"
@@ -85,6 +87,53 @@ __global__ void __launch_bounds__(256) k_cheb_full(int N, int nl, size_t cs, con
     }
 }
 
+// Complex FFT along x of columns [z0, z0 + cols) of one plane [x][Mz]; plane blockIdx.x, column chunk blockIdx.y.
+__global__ void __launch_bounds__(256) k_long_x(int Nx, int Mz, int cols, FftPlan px, const cpx<double>* __restrict__ tw,
+                                                int sign, double scale, cpx<double>* __restrict__ data) {
+  extern __shared__ unsigned char smem_raw[];
+  const int ss = Nx + 1, z0 = blockIdx.y * cols, nc = min(cols, Mz - z0);
+  cpx<double>* a = reinterpret_cast<cpx<double>*>(smem_raw);
+  cpx<double>* b = a + (size_t)cols * ss;
+  cpx<double>* plane = data + blockIdx.x * (size_t)Nx * Mz + z0;
+  for (int i = threadIdx.x; i < nc * Nx; i += blockDim.x) {
+    const int x = i / nc, c = i - x * nc;
+    a[c * ss + x] = plane[(size_t)x * Mz + c];
+  }
+  __syncthreads();
+  fft_batch<double>(a, b, nc, ss, px, tw, sign);
+  for (int i = threadIdx.x; i < nc * Nx; i += blockDim.x) {
+    const int x = i / nc, c = i - x * nc;
+    plane[(size_t)x * Mz + c] = cscale(a[c * ss + x], scale);
+  }
+}
+
+// z transform of rows of Nz + 2 doubles, `rows` a block: c2r (inverse, Hermitian completion) or r2c.
+__global__ void __launch_bounds__(256) k_long_z(long long nrows, int Nz, int rows, FftPlan pz,
+                                                const cpx<double>* __restrict__ tw, int inverse, double* __restrict__ data) {
+  extern __shared__ unsigned char smem_raw[];
+  const int Mz = Nz / 2 + 1, Nzpad = 2 * Mz, ss = Nz + 1;
+  cpx<double>* a = reinterpret_cast<cpx<double>*>(smem_raw);
+  cpx<double>* b = a + (size_t)rows * ss;
+  const long long row0 = (long long)rows * blockIdx.x;
+  const int nr = (int)min((long long)rows, nrows - row0);
+  double* first = data + row0 * Nzpad;
+  for (int i = threadIdx.x; i < nr * Nz; i += blockDim.x) {
+    const int r = i / Nz, k = i - r * Nz, m = k < Mz ? k : Nz - k;
+    const double* row = first + (size_t)r * Nzpad;
+    if (inverse)  // only the real parts of the first and last coefficient
+      a[r * ss + k] = cmk<double>(row[2 * m], k == 0 || 2 * k == Nz ? 0.0 : (k < Mz ? row[2 * m + 1] : -row[2 * m + 1]));
+    else
+      a[r * ss + k] = cmk<double>(row[k], 0.0);
+  }
+  __syncthreads();
+  fft_batch<double>(a, b, nr, ss, pz, tw, inverse ? +1 : -1);
+  for (int i = threadIdx.x; i < nr * Nzpad; i += blockDim.x) {
+    const int r = i / Nzpad, z = i - r * Nzpad;
+    const cpx<double>* s = a + r * ss;
+    first[(size_t)r * Nzpad + z] = inverse ? (z < Nz ? s[z].x : 0.0) : (z & 1 ? s[z >> 1].y : s[z >> 1].x);
+  }
+}
+
 long double cospi_frac(long long m, long long d) {  // cos(pi m / d), argument reduced over the integers
   long long r = m % (2 * d);
   if (r < 0) r += 2 * d;
@@ -104,8 +153,9 @@ struct cfgpu_flowfield_s {
   unsigned char* ozblock = nullptr;
   double* Mfwd = nullptr;  // [n][j] chebyfft
   double* Minv = nullptr;  // [j][n] ichebyfft
-  int* twx = nullptr;  // fx_twiddles
-  int* twz = nullptr;
+  void* twx = nullptr;  // fx_twiddles up to FX_LMAX, complex doubles of the plan beyond
+  void* twz = nullptr;
+  FftPlan px{}, pz{};
   cudaStream_t st = nullptr;
 };
 
@@ -144,19 +194,64 @@ int y_transform(cfgpu_flowfield f, bool to_spectral) {
   return CFGPU_OK;
 }
 
-int xz_transform(cfgpu_flowfield f, bool to_spectral) {
+// Lines beside their copies in about 96 KB of shared memory, at most 16 a block.
+int long_lines(int L) { return std::min(16, (int)(96 * 1024 / (2 * sizeof(cpx<double>) * (L + 1)))); }
+
+bool long_attr() {
+  static const bool attr = [] {
+    cudaFuncSetAttribute(k_long_x, cudaFuncAttributeMaxDynamicSharedMemorySize, 96 * 1024);
+    cudaFuncSetAttribute(k_long_z, cudaFuncAttributeMaxDynamicSharedMemorySize, 96 * 1024);
+    return true;
+  }();
+  return attr;
+}
+
+cudaError_t x_pass(cfgpu_flowfield f, int sign, double scale) {
   const int Mz = f->Nz / 2 + 1, planes = f->Ny * f->Nd;
-  const long long rows = (long long)planes * f->Nx;
+  cpx<double>* data = reinterpret_cast<cpx<double>*>(f->data);
+  if (f->Nx <= FX_LMAX) return launch_field_x(f->Nx, Mz, planes, f->twx, sign, scale, data, f->st);
+  long_attr();
+  const int cols = std::min(Mz, long_lines(f->Nx));
+  k_long_x<<<dim3(planes, (Mz + cols - 1) / cols), 256, 2 * sizeof(cpx<double>) * (size_t)cols * (f->Nx + 1), f->st>>>(
+      f->Nx, Mz, cols, f->px, (const cpx<double>*)f->twx, sign, scale, data);
+  return cudaGetLastError();
+}
+
+cudaError_t z_pass(cfgpu_flowfield f, bool inverse) {
+  const long long nrows = (long long)f->Ny * f->Nd * f->Nx;
+  if (f->Nz <= FX_LMAX) return launch_field_z(nrows, f->Nz, inverse, f->twz, f->data, f->st);
+  long_attr();
+  const int rows = long_lines(f->Nz);
+  k_long_z<<<(unsigned)((nrows + rows - 1) / rows), 256, 2 * sizeof(cpx<double>) * (size_t)rows * (f->Nz + 1), f->st>>>(
+      nrows, f->Nz, rows, f->pz, (const cpx<double>*)f->twz, inverse, f->data);
+  return cudaGetLastError();
+}
+
+int xz_transform(cfgpu_flowfield f, bool to_spectral) {
   if (f->Nx > TF_MAX || f->Nz > TF_MAX) return tf_fail(CFGPU_ENOTSUP, "Nx or Nz too large for the shared-memory FFT");
-  cpx<double>* cd = reinterpret_cast<cpx<double>*>(f->data);
   if (to_spectral) {
-    TF_CK(launch_field_z(rows, f->Nz, false, f->twz, f->data, f->st));
-    TF_CK(launch_field_x(f->Nx, Mz, planes, f->twx, -1, 1.0 / ((double)f->Nx * f->Nz), cd, f->st));
+    TF_CK(z_pass(f, false));
+    TF_CK(x_pass(f, -1, 1.0 / ((double)f->Nx * f->Nz)));
   } else {
-    TF_CK(launch_field_x(f->Nx, Mz, planes, f->twx, +1, 1.0, cd, f->st));
-    TF_CK(launch_field_z(rows, f->Nz, true, f->twz, f->data, f->st));
+    TF_CK(x_pass(f, +1, 1.0));
+    TF_CK(z_pass(f, true));
   }
   return CFGPU_OK;
+}
+
+// Twiddles of lines of length L (plan and its table tw).
+int line_twiddles(int L, const std::vector<std::complex<long double>>& tw, void** dst, cudaStream_t st) {
+  std::vector<cpx<double>> t;
+  if (L <= FX_LMAX) {
+    const std::vector<int> q = fx_twiddles(L);  // (x, y, z, w) of an entry in two doubles' place
+    t.resize(q.size() / 4);
+    std::memcpy((void*)t.data(), q.data(), q.size() * sizeof(int));
+  } else {
+    for (const auto& w : tw) t.push_back(cmk<double>((double)w.real(), (double)w.imag()));
+  }
+  const int e = tf_upload(t, (cpx<double>**)dst, st);
+  if (e == CFGPU_OK) TF_CK(cudaStreamSynchronize(st));  // t is a local
+  return e;
 }
 
 int finish(cfgpu_flowfield f, int st) {
@@ -187,10 +282,9 @@ cfgpu_status cfgpu_flowfield_create(const cfgpu_grid* g, int Nd, cfgpu_flowfield
   f->a = g->a;
   f->b = g->b;
   f->n = (size_t)Nd * g->Ny * g->Nx * 2 * (g->Nz / 2 + 1);
-  std::vector<std::complex<long double>> tw;
-  FftPlan plan{};
+  std::vector<std::complex<long double>> twx, twz;
   int st = CFGPU_OK;
-  if (!cfgpu_fft_plan(g->Nx, plan, tw) || !cfgpu_fft_plan(g->Nz, plan, tw))
+  if (!cfgpu_fft_plan(g->Nx, f->px, twx) || !cfgpu_fft_plan(g->Nz, f->pz, twz))
     st = tf_fail(CFGPU_ENOTSUP, "Nx and Nz must factor into primes <= " + std::to_string(FFT_MAX_RADIX));
   if (st == CFGPU_OK && cudaStreamCreateWithFlags(&f->st, cudaStreamNonBlocking) != cudaSuccess)
     st = tf_fail(CFGPU_ECUDA, "cudaStreamCreate failed");
@@ -231,9 +325,8 @@ cfgpu_status cfgpu_flowfield_create(const cfgpu_grid* g, int Nd, cfgpu_flowfield
       if (st == CFGPU_OK) st = tf_upload(Mf, &f->Mfwd, f->st);
       if (st == CFGPU_OK) st = tf_upload(Mi, &f->Minv, f->st);
     }
-    const std::vector<int> tx = fx_twiddles(f->Nx), tz = fx_twiddles(f->Nz);
-    if (st == CFGPU_OK) st = tf_upload(tx, &f->twx, f->st);
-    if (st == CFGPU_OK) st = tf_upload(tz, &f->twz, f->st);
+    if (st == CFGPU_OK) st = line_twiddles(f->Nx, twx, &f->twx, f->st);
+    if (st == CFGPU_OK) st = line_twiddles(f->Nz, twz, &f->twz, f->st);
     // the host vectors go out of scope: wait for the copies
     if (st == CFGPU_OK && cudaStreamSynchronize(f->st) != cudaSuccess) st = tf_fail(CFGPU_ECUDA, "stream sync");
   }

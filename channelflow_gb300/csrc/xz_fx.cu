@@ -626,11 +626,6 @@ cudaError_t launch_xinv_fx(const GridDev& g, const FftPlan& px, const void* tw, 
     return true;
   }();
   (void)attr;
-  if (curl && xfx_smem(g, czc, true) > 227 * 1024) {  // no room for the wavenumbers beside one very long column
-    const cudaError_t e = launch_curl_points(g, const_cast<cpx<double>*>(W), st);
-    if (e != cudaSuccess) return e;
-    curl = false;
-  }
   const FxPlan p = fx_plan(px.L);
   return launch_pdl(p.any ? k_xinv_fx<true> : k_xinv_fx<false>, dim3(g.Ny, ncomp, (g.NKz + czc - 1) / czc), dim3(FX_THREADS),
                     xfx_smem(g, czc, curl), st, g, p, (const fxtw*)tw, (const double2*)W, (double2*)X, czc, (int)curl);
