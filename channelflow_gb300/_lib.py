@@ -65,6 +65,7 @@ _SIGS = {
     "cfgpu_dns_kernel_launches": [C.c_void_p, C.POINTER(C.c_longlong)],
     "cfgpu_dns_destroy": [C.c_void_p],
     "cfgpu_dns_cfl": [C.c_void_p, _PD],
+    "cfgpu_dns_inject_wait_error": [C.c_void_p],
     "cfgpu_dns_nonlinear": [C.c_void_p, _PD, _PD],
     "cfgpu_set_host_access": [C.c_int],
     "cfgpu_dns_reset_time": [C.c_void_p, C.c_double],
@@ -140,6 +141,7 @@ _SIGS = {
     "cfgpu_flowfield_upload": [C.c_void_p, _PD, C.c_int, C.c_int],
     "cfgpu_flowfield_download": [C.c_void_p, _PD],
     "cfgpu_flowfield_state": [C.c_void_p, _PI, _PI],
+    "cfgpu_flowfield_inject_wait_error": [C.c_void_p],
     "cfgpu_flowfield_make_physical": [C.c_void_p],
     "cfgpu_flowfield_make_spectral": [C.c_void_p],
     "cfgpu_flowfield_make_physical_xz": [C.c_void_p],

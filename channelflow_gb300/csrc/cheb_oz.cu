@@ -517,7 +517,7 @@ __global__ void __launch_bounds__(OZ_THREADS, 1) k_cheb_oz(const __grid_constant
     }
     __syncthreads();  // sS, sE of the next stage
   }
-  if (!ok && a.err) atomicExch(a.err, 1);
+  if (!ok && a.err) *static_cast<volatile int*>(a.err) = 1;
   asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
@@ -763,7 +763,7 @@ __global__ void __launch_bounds__(OZ_THREADS, 1) k_cheb_oz_few(const __grid_cons
     __syncthreads();  // sS, sE, accumulators of the next stage
     asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
   }
-  if (!ok && a.err) atomicExch(a.err, 1);
+  if (!ok && a.err) *static_cast<volatile int*>(a.err) = 1;
   if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(tmem), "r"(tcols));
 }
 

@@ -183,7 +183,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
           }
         if (!got) {
           ok = false;
-          if (err) atomicExch(err, 1);
+          if (err) *static_cast<volatile int*>(err) = 1;
         }
       }
       if (ok) {
@@ -213,7 +213,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
         done = true;
         break;
       }
-    if (!done && err) atomicExch(err, 1);
+    if (!done && err) *static_cast<volatile int*>(err) = 1;
     ok = __syncthreads_and(ok && done) != 0;
     asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
     // epilogue: warp w reads TMEM lanes 32 (w % 4) .. + 31 (its sub-partition's) and columns 16 (w / 4) .. + 15;

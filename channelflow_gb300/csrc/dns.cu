@@ -417,6 +417,18 @@ void pinned_free(void* p) {
 
 }  // namespace
 
+int cfgpu_wait_flag(int** p) {
+  const int st = pinned_alloc(p, sizeof(int));
+  if (st == CFGPU_OK) **p = 0;
+  return st;
+}
+void cfgpu_wait_flag_free(int* p) { pinned_free(p); }
+int cfgpu_wait_status(const int* p) {
+  if (p && *static_cast<const volatile int*>(p))
+    return fail(CFGPU_ECUDA, "a wait for copies or tensor products ran out in a kernel: the object's fields are not valid");
+  return CFGPU_OK;
+}
+
 // Programmatic dependent launch between the kernels of a step (cfgpu_set_pdl; declared in common.cuh).  Off: a step is
 // replayed as a graph, whose launch gaps are about a microsecond, and kernels that come early hold the slots of those
 // that still run.  On against off: 32x33x32 mixed 68 / 57 us a step, 12 served requests 37.4 / 33.1 ms, 128x97x128
@@ -649,7 +661,7 @@ struct cfgpu_dns_s {
   bool ydct = false;
   // forward Chebyshev transform of the mixed path on the tensor cores (cheb_tc_matrix(Ny), BF16 splits)
   void* ctc = nullptr;
-  int* dtcerr = nullptr;
+  int* waiterr = nullptr;  // pinned: set by a kernel whose bounded wait ran out (cfgpu_wait_status)
   bool ytc = false;
   void *cinvA = nullptr, *cinvB = nullptr, *cfwdA = nullptr, *cfwdB = nullptr;
   void *cderA = nullptr, *cderB = nullptr, *basey = nullptr;  // fused curl: (2/L) T'_n(y_j); U, U', W, W' at y_j
@@ -796,6 +808,13 @@ int build_slot_tables(cfgpu_dns d, int f) {
   return CFGPU_OK;
 }
 
+// Everything enqueued is done; an error if one of its kernels gave up a wait.  The state stays marked: later steps would
+// start from it.
+int dns_sync(cfgpu_dns d) {
+  CK(cudaStreamSynchronize(d->st));
+  return cfgpu_wait_status(d->waiterr);
+}
+
 // Constant versions of the nonlinear pass (mixed precision; FP64 uses its exact tables).
 Dither dither_of(cfgpu_dns d) {
   Dither dt{};
@@ -811,7 +830,7 @@ Dither dither_of(cfgpu_dns d) {
 
 // FP64 Chebyshev transforms on the tensor cores (d->oz).
 int oz_run(cfgpu_dns d, bool inverse, const OzJob* jobs, int n) {
-  CK(launch_cheb_oz(d->gm, d->N, inverse, (int)d->rowc(), d->rowc(), d->ozt, jobs, n, d->dtcerr, d->st));
+  CK(launch_cheb_oz(d->gm, d->N, inverse, (int)d->rowc(), d->rowc(), d->ozt, jobs, n, d->waiterr, d->st));
   d->launches++;
   return CFGPU_OK;
 }
@@ -980,7 +999,7 @@ int nonlinear_impl(cfgpu_dns d, const double* U, void* Nout, int form) {
   const R* F = (const R*)d->F3;
   if constexpr (sizeof(R) == 4) {
     if ((form == NL_ROTATIONAL || form == NL_CONVECTION) && d->ytc) {
-      CK(launch_cheb_tc(N, (int)row, 3, (const float*)F, row, comp, (float*)Nout, d->ctc, d->dtcerr, d->st));
+      CK(launch_cheb_tc(N, (int)row, 3, (const float*)F, row, comp, (float*)Nout, d->ctc, d->waiterr, d->st));
       d->launches += 1;
       return CFGPU_OK;
     }
@@ -1466,14 +1485,14 @@ int get_fields(cfgpu_dns d, double* u, double* q) {
   if (d->direct) {
     if (u) CK(launch_host_modes(d->g, false, 3, d->nb, 0, d->nb, d->Ucur, u, d->st));
     if (q) CK(launch_host_modes(d->g, false, 1, d->nb, 0, d->nb, d->Qcur, q, d->st));
-    CK(cudaStreamSynchronize(d->st));
+    CKS(dns_sync(d));
     return CFGPU_OK;
   }
   CKS(ensure_stage(d));
   const size_t cd = d->compc();
   CK(cudaMemcpyAsync(d->stage, d->Ucur, 3 * cd * sizeof(double), cudaMemcpyDeviceToHost, d->st));
   CK(cudaMemcpyAsync(d->stage + 3 * cd, d->Qcur, cd * sizeof(double), cudaMemcpyDeviceToHost, d->st));
-  CK(cudaStreamSynchronize(d->st));
+  CKS(dns_sync(d));
   if (u) scatter_modes(d, d->stage, 3, u);
   if (q) scatter_modes(d, d->stage + 3 * cd, 1, q);
   return CFGPU_OK;
@@ -1513,7 +1532,7 @@ int get_slot(cfgpu_dns d, int slot, double* u, double* q) {
   if (d->direct) {
     if (u) CK(launch_host_modes(d->g, false, 3, 1, slot, d->nb, d->Ucur, u, d->st));
     if (q) CK(launch_host_modes(d->g, false, 1, 1, slot, d->nb, d->Qcur, q, d->st));
-    CK(cudaStreamSynchronize(d->st));
+    CKS(dns_sync(d));
     return CFGPU_OK;
   }
   CKS(ensure_stage1(d));
@@ -1523,7 +1542,7 @@ int get_slot(cfgpu_dns d, int slot, double* u, double* q) {
                        w * sizeof(double), 3 * (size_t)d->N, cudaMemcpyDeviceToHost, d->st));
   CK(cudaMemcpy2DAsync(stage + 3 * cd1, w * sizeof(double), d->Qcur + slot * w, pitch * sizeof(double),
                        w * sizeof(double), (size_t)d->N, cudaMemcpyDeviceToHost, d->st));
-  CK(cudaStreamSynchronize(d->st));
+  CKS(dns_sync(d));
   if (u) scatter_modes(d, stage, 3, u, 0, 1, 1);
   if (q) scatter_modes(d, stage + 3 * cd1, 1, q, 0, 1, 1);
   return CFGPU_OK;
@@ -1581,8 +1600,6 @@ int oz_upload(cfgpu_dns d, bool with_df) {
   CKS(dalloc(&p, h.size(), d->bytes));
   d->ozblock = p;
   CK(cudaMemcpyAsync(p, h.data(), h.size(), cudaMemcpyHostToDevice, d->st));
-  CKS(dalloc(&d->dtcerr, 1, d->bytes));
-  CK(cudaMemsetAsync(d->dtcerr, 0, sizeof(int), d->st));
   OzMatrix* m[3] = {&d->ozt.T, &d->ozt.F, &d->ozt.DF};
   for (int k = 0; k < nm; ++k) *m[k] = OzMatrix{p + k * mb, (const int*)(p + nm * mb + k * rb)};
   d->ozt.N = N;
@@ -1857,7 +1874,7 @@ int tune_cheb_tc(cfgpu_dns d) {
                                             (const float*)d->cfwdA, (const float*)d->cfwdB, d->st);
   });
   const float tt = time_ms<float>(d, [&]() {
-    return launch_cheb_tc(N, nl1, 3, (const float*)d->F3, row, comp, out, d->ctc, d->dtcerr, d->st);
+    return launch_cheb_tc(N, nl1, 3, (const float*)d->F3, row, comp, out, d->ctc, d->waiterr, d->st);
   });
   d->ytc = tt < 1e30f && tt < tm;
   CK(cudaStreamSynchronize(d->st));
@@ -1946,6 +1963,7 @@ int dns_create_impl(cfgpu_dns d, const cfgpu_grid* grid, const cfgpu_flags* flag
     d->WbulkAct = bf.WbulkBase + sw;
   }
   long long& B = d->bytes;
+  CKS(cfgpu_wait_flag(&d->waiterr));
   CKS(dalloc(&d->dUbase, Ny, B));
   CKS(dalloc(&d->dWbase, Ny, B));
   CKS(dalloc(&d->dUbaseyy, Ny, B));
@@ -2083,8 +2101,6 @@ int dns_create_impl(cfgpu_dns d, const cfgpu_grid* grid, const cfgpu_flags* flag
       const std::vector<uint16_t> tcm = cheb_tc_matrix(Fm, Ny);
       CKS(dalloc(&d->ctc, tcm.size() * sizeof(uint16_t), B));
       CK(cudaMemcpyAsync(d->ctc, tcm.data(), tcm.size() * sizeof(uint16_t), cudaMemcpyHostToDevice, d->st));
-      CKS(dalloc(&d->dtcerr, 1, B));
-      CK(cudaMemsetAsync(d->dtcerr, 0, sizeof(int), d->st));
     }
     d->cS = (long long)(S * sizeof(float));
     CKS(upload_dithered({basey}, {0}, basey.size(), &d->basey, B, d->st));
@@ -2195,7 +2211,7 @@ int dns_create_impl(cfgpu_dns d, const cfgpu_grid* grid, const cfgpu_flags* flag
   if (d->has_init) CKS(build_tables(d, d->init));
   d->stage_elems = 4 * cd;  // pinned host staging, allocated on first host transfer (ensure_stage)
   CKS(pinned_alloc(&d->cfl_host, (size_t)nb * sizeof(unsigned long long)));
-  CK(cudaStreamSynchronize(d->st));
+  CKS(dns_sync(d));
   return CFGPU_OK;
 }
 
@@ -2208,7 +2224,7 @@ void dns_free(cfgpu_dns d) {
     d->twx = d->twz = d->cinvA = d->cinvB = d->cfwdA = d->cfwdB = d->cderA = d->cderB = d->cdfA = d->cdfB = nullptr;
     d->twxf = d->twzf = d->cdct = nullptr;
   }
-  F(d->twxf); F(d->twzf); F(d->cdct); F(d->ctc); F(d->dtcerr); F(d->ozblock);
+  F(d->twxf); F(d->twzf); F(d->cdct); F(d->ctc); F(d->ozblock);
   F(d->dUbase); F(d->dWbase); F(d->dUbaseyy); F(d->dWbaseyy); F(d->ddPdx);
   F(d->hb_lo); F(d->hb_di); F(d->hb_up);
   F(d->twx); F(d->twz); F(d->twxq); F(d->twzq); F(d->cinvA); F(d->cinvB); F(d->cfwdA); F(d->cfwdB);
@@ -2223,6 +2239,7 @@ void dns_free(cfgpu_dns d) {
     for (auto& t : s->tau) { F(t.f); F(t.s); }
   pinned_free(d->stage);
   pinned_free(d->cfl_host);
+  cfgpu_wait_flag_free(d->waiterr);
   pinned_free(d->stage1);
   for (auto& e : d->ev_pool) cudaEventDestroy(e);
   for (auto& u : d->ev_used) {
@@ -2289,7 +2306,7 @@ void cfl_finish(cfgpu_dns d, double* cfl) {
 template <typename R>
 int cfl_impl(cfgpu_dns d, double* cfl) {
   CKS(cfl_enqueue<R>(d));
-  CK(cudaStreamSynchronize(d->st));
+  CKS(dns_sync(d));
   cfl_finish(d, cfl);
   return CFGPU_OK;
 }
@@ -2301,7 +2318,7 @@ int l2norm_impl(cfgpu_dns d, int field, double* l2) {
   d->launches++;
   std::vector<double> s(d->nb);
   CK(cudaMemcpyAsync(s.data(), out, d->nb * sizeof(double), cudaMemcpyDeviceToHost, d->st));
-  CK(cudaStreamSynchronize(d->st));
+  CKS(dns_sync(d));
   for (int f = 0; f < d->nb; ++f) l2[f] = std::sqrt(s[f]);
   return CFGPU_OK;
 }
@@ -2330,6 +2347,7 @@ int set_priority(cfgpu_dns d, int prio) {
 
 int advance_async(cfgpu_dns d, int nsteps) { return dns_advance_device(d, nsteps); }
 cudaStream_t stream(cfgpu_dns d) { return d->st; }
+int wait_status(cfgpu_dns d) { return cfgpu_wait_status(d->waiterr); }
 long long bytes(cfgpu_dns d) { return d->bytes; }
 int nfields(cfgpu_dns d) { return d->nb; }
 
@@ -2348,7 +2366,7 @@ int store_slot(cfgpu_dns d, int slot, cfgpu_dns dst) {
                        d->st));
   CK(cudaMemcpy2DAsync(dst->Qcur, w * 8, d->Qcur + slot * w, pitch * 8, w * 8, N, cudaMemcpyDeviceToDevice, d->st));
   CK(cudaMemcpyAsync(dst->dver, d->dver + slot, sizeof(int), cudaMemcpyDeviceToDevice, d->st));  // constant version
-  CK(cudaStreamSynchronize(d->st));
+  CKS(dns_sync(d));
   return CFGPU_OK;
 }
 
@@ -2564,7 +2582,7 @@ cfgpu_status cfgpu_ensemble_load_slot(cfgpu_dns d, int slot, cfgpu_dns src) {
     d->main.countdown = 0;
     d->main.full = true;
   }
-  CK(cudaStreamSynchronize(src->st));
+  CKS(dns_sync(src));
   const size_t w = 2 * (size_t)a.Md, pitch = w * d->nb, N = d->N;
   auto copy = [&](void* dst, const void* srcp, size_t esz, size_t rows) -> int {
     CK(cudaMemcpy2DAsync((unsigned char*)dst + slot * w * esz, pitch * esz, srcp, w * esz, w * esz, rows,
@@ -2589,7 +2607,7 @@ cfgpu_status cfgpu_ensemble_load_slot(cfgpu_dns d, int slot, cfgpu_dns src) {
   }
   CK(cudaMemcpyAsync(d->ddPdx + 2 * slot, src->ddPdx, 2 * sizeof(double), cudaMemcpyDeviceToDevice, d->st));
   CK(cudaMemcpyAsync(d->dver + slot, src->dver, sizeof(int), cudaMemcpyDeviceToDevice, d->st));  // constant version
-  CK(cudaStreamSynchronize(d->st));
+  CKS(dns_sync(d));
   return CFGPU_OK;
 }
 
@@ -2623,7 +2641,7 @@ cfgpu_status cfgpu_ensemble_dPdx(cfgpu_dns d, double* dPdx) {
   if (!d || !dPdx) return fail(CFGPU_EINVAL, "bad argument");
   std::vector<double> v(2 * (size_t)d->nb);
   CK(cudaMemcpyAsync(v.data(), d->ddPdx, v.size() * sizeof(double), cudaMemcpyDeviceToHost, d->st));
-  CK(cudaStreamSynchronize(d->st));
+  CKS(dns_sync(d));
   for (int f = 0; f < d->nb; ++f) dPdx[f] = v[2 * f];
   return CFGPU_OK;
 }
@@ -2744,7 +2762,7 @@ cfgpu_status cfgpu_dns_get_fields_device(cfgpu_dns d, int slot, cfgpu_field u, c
   const size_t w = 2 * (size_t)d->g.Md, pitch = w * d->nb, N = d->N;
   if (u) CK(cudaMemcpy2DAsync(u->data, w * 8, d->Ucur + slot * w, pitch * 8, w * 8, 3 * N, cudaMemcpyDeviceToDevice, d->st));
   if (q) CK(cudaMemcpy2DAsync(q->data, w * 8, d->Qcur + slot * w, pitch * 8, w * 8, N, cudaMemcpyDeviceToDevice, d->st));
-  CK(cudaStreamSynchronize(d->st));
+  CKS(dns_sync(d));
   return CFGPU_OK;
 }
 
@@ -2763,7 +2781,7 @@ cfgpu_status cfgpu_dns_get_fields(cfgpu_dns d, double* u, double* q) {
 cfgpu_status cfgpu_dns_advance_resident(cfgpu_dns d, int nsteps) {
   if (!d || nsteps < 0) return fail(CFGPU_EINVAL, "bad argument");
   CKS(dns_advance_device(d, nsteps));
-  CK(cudaStreamSynchronize(d->st));
+  CKS(dns_sync(d));
   return CFGPU_OK;
 }
 
@@ -2788,7 +2806,7 @@ cfgpu_status cfgpu_dns_reset_dt(cfgpu_dns d, double dt) {
     s->tau = keep;
     CKS(build_tables(d, *s));
   }
-  CK(cudaStreamSynchronize(d->st));
+  CKS(dns_sync(d));
   return CFGPU_OK;
 }
 
@@ -2835,7 +2853,7 @@ cfgpu_status cfgpu_dns_dPdx(cfgpu_dns d, double* dPdx) {
   if (!d || !dPdx) return fail(CFGPU_EINVAL, "bad argument");
   double v[2];
   CK(cudaMemcpyAsync(v, d->ddPdx, sizeof(v), cudaMemcpyDeviceToHost, d->st));
-  CK(cudaStreamSynchronize(d->st));
+  CKS(dns_sync(d));
   *dPdx = v[0];
   return CFGPU_OK;
 }
@@ -2894,6 +2912,7 @@ cfgpu_status cfgpu_dns_nonlinear(cfgpu_dns d, const double* u, double* f) {
     if (e != cudaSuccess) st = fail(CFGPU_ECUDA, std::string("nonlinear: ") + cudaGetErrorString(e));
   }
   cudaStreamSynchronize(d->st);
+  if (st == CFGPU_OK) st = cfgpu_wait_status(d->waiterr);
   dfree(Ud);
   dfree(Nd);
   if (st != CFGPU_OK) return st;
@@ -2906,6 +2925,12 @@ cfgpu_status cfgpu_dns_nonlinear(cfgpu_dns d, const double* u, double* f) {
   const GridDev& g = d->g;
   memset(f, 0, sizeof(double) * 3 * (size_t)d->nb * 2 * g.Ny * g.Nx * (g.Nz / 2 + 1));
   scatter_modes(d, out.data(), 3, f);
+  return CFGPU_OK;
+}
+
+cfgpu_status cfgpu_dns_inject_wait_error(cfgpu_dns d) {
+  if (!d) return fail(CFGPU_EINVAL, "null dns");
+  *d->waiterr = 1;
   return CFGPU_OK;
 }
 
@@ -2938,7 +2963,7 @@ cfgpu_status cfgpu_dns_advance_timed(cfgpu_dns d, int nsteps, double* ms) {
   *ms = t;
   d->ev_pool.push_back(a);
   d->ev_pool.push_back(b);
-  return CFGPU_OK;
+  return cfgpu_wait_status(d->waiterr);
 }
 
 cfgpu_status cfgpu_dns_set_profiling(cfgpu_dns d, int enable) {
@@ -2965,7 +2990,7 @@ cfgpu_status cfgpu_dns_symmetry(cfgpu_dns d, const cfgpu_symmetry* y, int projec
   if (std::abs(y->s) != 1 || std::abs(y->sx) != 1 || std::abs(y->sy) != 1 || std::abs(y->sz) != 1)
     return fail(CFGPU_EINVAL, "symmetry signs must be +1 or -1");
   CKS(symmetry_on(d, d->Ucur, 8, 3, SymmetryDev{y->s, y->sx, y->sy, y->sz, y->ax, y->az}, project ? 1 : 0));
-  CK(cudaStreamSynchronize(d->st));
+  CKS(dns_sync(d));
   return CFGPU_OK;
 }
 
@@ -3161,7 +3186,7 @@ cfgpu_status cfgpu_ensemble_field2vector(cfgpu_dns d, int slot, double* v) {
   if (!d || !v || slot < 0 || slot >= d->nb) return fail(CFGPU_EINVAL, "bad argument");
   if (d->g.Kx != d->g.Nx / 3 - 1 || d->g.Kz != d->g.Nz / 3 - 1 || d->N < 5)
     return fail(CFGPU_ENOTSUP, "field2vector needs the 2/3-dealiased mode set");
-  CK(cudaStreamSynchronize(d->st));
+  CKS(dns_sync(d));
   return f2v_device(d->g, slot, d->nb, d->Ucur, v, d->st);
 }
 
@@ -3169,7 +3194,7 @@ cfgpu_status cfgpu_ensemble_vector2field(cfgpu_dns d, int slot, const double* v)
   if (!d || !v || slot < 0 || slot >= d->nb) return fail(CFGPU_EINVAL, "bad argument");
   if (d->g.Kx != d->g.Nx / 3 - 1 || d->g.Kz != d->g.Nz / 3 - 1 || d->N < 5)
     return fail(CFGPU_ENOTSUP, "vector2field needs the 2/3-dealiased mode set");
-  CK(cudaStreamSynchronize(d->st));
+  CKS(dns_sync(d));
   return v2f_device(d->g, slot, d->nb, v, d->Ucur, d->st);
 }
 

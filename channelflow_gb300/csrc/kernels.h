@@ -13,6 +13,13 @@
 // Records the message returned by cfgpu_last_error() on this thread; returns code.
 int cfgpu_record_error(int code, const std::string& msg);
 
+// Flag of an object whose kernels bound their waits (cheb_oz.cu, cheb_tc.cu): page-locked host memory that a kernel sets
+// when a wait ran out, read on the host once the object's stream is synchronised, at no transfer.  cfgpu_wait_status
+// returns CFGPU_ECUDA, with a message, for a flag that is set.
+int cfgpu_wait_flag(int** p);
+void cfgpu_wait_flag_free(int* p);
+int cfgpu_wait_status(const int* p);
+
 // Undithered constants (version 0 only; one field).
 constexpr Dither kNoDither{nullptr, 0, 0, 1, nullptr, nullptr, nullptr};
 

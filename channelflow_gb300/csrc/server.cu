@@ -59,6 +59,7 @@
 namespace cfgpu_rt {
 int advance_async(cfgpu_dns d, int nsteps);
 cudaStream_t stream(cfgpu_dns d);
+int wait_status(cfgpu_dns d);
 long long bytes(cfgpu_dns d);
 int startup_steps(cfgpu_dns d);
 int restart(cfgpu_dns d);
@@ -187,7 +188,7 @@ int wait_stream(Ens* e, cfgpu_dns h) {
   if (cudaEventRecord(e->done, cfgpu_rt::stream(h)) != cudaSuccess) return sfail(CFGPU_ECUDA, "event record");
   const cudaError_t st = cudaEventSynchronize(e->done);
   if (st != cudaSuccess) return sfail(CFGPU_ECUDA, std::string("step failed: ") + cudaGetErrorString(st));
-  return CFGPU_OK;
+  return cfgpu_rt::wait_status(h);
 }
 
 int advance_sync(Ens* e, cfgpu_dns h, int n) {

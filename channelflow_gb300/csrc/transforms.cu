@@ -157,6 +157,7 @@ struct cfgpu_flowfield_s {
   void* twz = nullptr;
   FftPlan px{}, pz{};
   cudaStream_t st = nullptr;
+  int* waiterr = nullptr;  // cfgpu_wait_flag
 };
 
 namespace {
@@ -183,7 +184,7 @@ int y_transform(cfgpu_flowfield f, bool to_spectral) {
         job[c].in = job[c].out = f->data + (c0 + c) * cs;
         job[c].inplace = 1;
       }
-      TF_CK(launch_cheb_oz(g, f->Ny, !to_spectral, nl, nl, f->oz, job, nj, nullptr, f->st));
+      TF_CK(launch_cheb_oz(g, f->Ny, !to_spectral, nl, nl, f->oz, job, nj, f->waiterr, f->st));
     }
     return CFGPU_OK;
   }
@@ -260,7 +261,7 @@ int finish(cfgpu_flowfield f, int st) {
     return st;
   }
   TF_CK(cudaStreamSynchronize(f->st));
-  return CFGPU_OK;
+  return cfgpu_wait_status(f->waiterr);
 }
 
 }  // namespace
@@ -288,6 +289,7 @@ cfgpu_status cfgpu_flowfield_create(const cfgpu_grid* g, int Nd, cfgpu_flowfield
     st = tf_fail(CFGPU_ENOTSUP, "Nx and Nz must factor into primes <= " + std::to_string(FFT_MAX_RADIX));
   if (st == CFGPU_OK && cudaStreamCreateWithFlags(&f->st, cudaStreamNonBlocking) != cudaSuccess)
     st = tf_fail(CFGPU_ECUDA, "cudaStreamCreate failed");
+  if (st == CFGPU_OK) st = cfgpu_wait_flag(&f->waiterr);
   if (st == CFGPU_OK) {
     cudaError_t e = cudaMalloc((void**)&f->data, f->n * sizeof(double));
     if (e == cudaSuccess) e = cudaMemsetAsync(f->data, 0, f->n * sizeof(double), f->st);
@@ -348,6 +350,7 @@ cfgpu_status cfgpu_flowfield_destroy(cfgpu_flowfield f) {
   cudaFree(f->Minv);
   cudaFree(f->twx);
   cudaFree(f->twz);
+  cfgpu_wait_flag_free(f->waiterr);
   if (f->st) cudaStreamDestroy(f->st);
   delete f;
   return CFGPU_OK;
@@ -371,6 +374,7 @@ cfgpu_status cfgpu_flowfield_upload(cfgpu_flowfield f, const double* host, int x
     return tf_fail(CFGPU_EINVAL, "bad argument");
   TF_CK(cudaMemcpyAsync(f->data, host, f->n * sizeof(double), cudaMemcpyHostToDevice, f->st));
   TF_CK(cudaStreamSynchronize(f->st));
+  *f->waiterr = 0;  // whole new data
   f->xzstate = xzstate;
   f->ystate = ystate;
   return CFGPU_OK;
@@ -380,6 +384,12 @@ cfgpu_status cfgpu_flowfield_download(cfgpu_flowfield f, double* host) {
   if (!f || !host) return tf_fail(CFGPU_EINVAL, "bad argument");
   TF_CK(cudaMemcpyAsync(host, f->data, f->n * sizeof(double), cudaMemcpyDeviceToHost, f->st));
   TF_CK(cudaStreamSynchronize(f->st));
+  return cfgpu_wait_status(f->waiterr);
+}
+
+cfgpu_status cfgpu_flowfield_inject_wait_error(cfgpu_flowfield f) {
+  if (!f) return tf_fail(CFGPU_EINVAL, "bad argument");
+  *f->waiterr = 1;
   return CFGPU_OK;
 }
 

@@ -109,6 +109,8 @@ cfgpu_status cfgpu_flowfield_data(cfgpu_flowfield f, double** device_ptr);
 cfgpu_status cfgpu_flowfield_upload(cfgpu_flowfield f, const double* host, int xzstate, int ystate);
 cfgpu_status cfgpu_flowfield_download(cfgpu_flowfield f, double* host);
 cfgpu_status cfgpu_flowfield_state(cfgpu_flowfield f, int* xzstate, int* ystate);
+/* No reference counterpart: as cfgpu_dns_inject_wait_error; an upload clears it. */
+cfgpu_status cfgpu_flowfield_inject_wait_error(cfgpu_flowfield f);
 cfgpu_status cfgpu_flowfield_make_physical(cfgpu_flowfield f);
 cfgpu_status cfgpu_flowfield_make_spectral(cfgpu_flowfield f);
 cfgpu_status cfgpu_flowfield_make_physical_xz(cfgpu_flowfield f);
@@ -175,6 +177,10 @@ cfgpu_status cfgpu_dns_dPdx(cfgpu_dns dns, double* dPdx);
  * DealiasXZ (pi dt otherwise).  Needs Ny <= 111.
  */
 cfgpu_status cfgpu_dns_cfl(cfgpu_dns dns, double* cfl);
+/* No reference counterpart: the tensor-core transforms bound every wait for their copies and products.  Where one runs
+ * out, the calls that wait for a DNS's (ensemble's) results return CFGPU_ECUDA from then on, and the server fails the
+ * requests.  This call marks a DNS that way from the host, for tests of an application's error path. */
+cfgpu_status cfgpu_dns_inject_wait_error(cfgpu_dns dns);
 /* navierstokesNL (channelflow/nse.h:20, nse.cpp:12-91) plus NSE::nonlinear's zeroPaddedModes
  * (nse.cpp:383-391): f = N(u) with the DNS's base flow, nonlinearity, Vsuck and rotation flags, in its
  * precision.  u and f: FlowField buffers of the DNS's nfields velocity fields; the DNS's own fields are not
