@@ -306,6 +306,7 @@ __global__ void __launch_bounds__(OZ_THREADS, 1) k_cheb_oz(const __grid_constant
   const bool emit_scale = INV && job.deriv && a.dscale != 1.0, emit_grad = INV && job.gx != nullptr;
 
   bool ok = true;
+  uint32_t late = 0, lpar = 0;  // thread 0: barrier and parity of a copy given up; none is started after it
   int t = 0;  // K steps issued so far (ring position)
   const int nstage = INV || !job.pd ? 1 : 2;
   const int q0 = a.split ? (int)blockIdx.z : 0, q1 = a.split ? q0 + 1 : 2;  // parities of this CTA
@@ -333,7 +334,7 @@ __global__ void __launch_bounds__(OZ_THREADS, 1) k_cheb_oz(const __grid_constant
         const int st = t % ring, use = t / ring, nks = min(KS - 2 * pr, 2);
         const uint32_t full = smem_u32(mbar + st), done = smem_u32(mbar + 2 + st);
         if (use > 0 && !mbar_wait(done, (uint32_t)((use - 1) & 1))) ok = false;
-        if (tid == 0) {
+        if (tid == 0 && !late) {
           asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n" ::"r"(full), "r"((uint32_t)(nks * bst))
                        : "memory");
           asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];\n" ::"r"(
@@ -390,7 +391,7 @@ __global__ void __launch_bounds__(OZ_THREADS, 1) k_cheb_oz(const __grid_constant
         __syncthreads();
         if (tid == 0) {
           asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
-          if (mbar_wait(full, (uint32_t)(use & 1))) {
+          if (!late && mbar_wait(full, (uint32_t)(use & 1))) {
             for (int k = 0; k < nks; ++k) {
               const uint32_t a0 = smem_u32(As + (st * 2 + k) * OZ_ASTAGE), b0 = smem_u32(Bs + (st * 2 + k) * bst);
               for (int i = 0; i < OZ_DIGITS; ++i) {
@@ -406,6 +407,10 @@ __global__ void __launch_bounds__(OZ_THREADS, 1) k_cheb_oz(const __grid_constant
             }
           } else {
             ok = false;
+            if (!late) {
+              late = full;
+              lpar = (uint32_t)(use & 1);
+            }
           }
           asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n" ::"r"(done)
                        : "memory");
@@ -517,7 +522,11 @@ __global__ void __launch_bounds__(OZ_THREADS, 1) k_cheb_oz(const __grid_constant
     }
     __syncthreads();  // sS, sE of the next stage
   }
-  if (!ok && a.err) *static_cast<volatile int*>(a.err) = 1;
+  if (!ok) {  // copies and products that are still under way end before their memory is given back (bounded again)
+    if (a.err) *static_cast<volatile int*>(a.err) = 1;
+    if (late) mbar_wait(late, lpar);
+    mbar_wait(smem_u32(mbar + 2 + (t - 1) % ring), (uint32_t)(((t - 1) / ring) & 1));
+  }
   asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
@@ -603,13 +612,14 @@ __global__ void __launch_bounds__(OZ_THREADS, 1) k_cheb_oz_few(const __grid_cons
   OzLine<INV> ln(a, job, gl, act);
 
   bool ok = true;
+  int late = -1;  // thread 0: stage of a copy given up; none is started after it
   const int nstage = INV || !job.pd ? 1 : 2;
   for (int sg = 0; sg < nstage; ++sg) {
     const bool fd = !INV && sg == 1;
     const OzMatrix& M = INV ? a.t.T : (fd ? a.t.DF : a.t.F);
     ln.src = fd ? job.pd : job.in;
     ln.fd = fd;
-    if (tid == 0) {  // the previous stage's products have read their matrix
+    if (tid == 0 && late < 0) {  // the previous stage's products have read their matrix
       const uint32_t bytes = (uint32_t)((KS[0] + KS[1]) * bst);
       asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n" ::"r"(full), "r"(bytes) : "memory");
       asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];\n" ::"r"(
@@ -682,7 +692,7 @@ __global__ void __launch_bounds__(OZ_THREADS, 1) k_cheb_oz_few(const __grid_cons
     __syncthreads();
     if (tid == 0) {
       asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
-      if (mbar_wait(full, (uint32_t)(sg & 1))) {
+      if (late < 0 && mbar_wait(full, (uint32_t)(sg & 1))) {
         for (int iq = 0; iq < 2; ++iq) {
           const uint32_t acc = tmem + (uint32_t)((fd ? 1 - iq : iq) * acols);
           for (int k = 0; k < KS[iq]; ++k) {
@@ -696,6 +706,7 @@ __global__ void __launch_bounds__(OZ_THREADS, 1) k_cheb_oz_few(const __grid_cons
         }
       } else {
         ok = false;
+        if (late < 0) late = sg;
       }
       asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n" ::"r"(done) : "memory");
     }
@@ -763,7 +774,12 @@ __global__ void __launch_bounds__(OZ_THREADS, 1) k_cheb_oz_few(const __grid_cons
     __syncthreads();  // sS, sE, accumulators of the next stage
     asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
   }
-  if (!ok && a.err) *static_cast<volatile int*>(a.err) = 1;
+  if (!ok) {  // copies and products that are still under way end before their memory is given back (bounded again)
+    if (a.err) *static_cast<volatile int*>(a.err) = 1;
+    if (late >= 0) mbar_wait(full, (uint32_t)late);
+    mbar_wait(done, (uint32_t)(nstage - 1));
+  }
+  __syncwarp();
   if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(tmem), "r"(tcols));
 }
 

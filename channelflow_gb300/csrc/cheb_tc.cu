@@ -258,6 +258,9 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
     __syncthreads();
   }
   asm volatile("cp.async.wait_all;\n" ::: "memory");
+  if (!ok && tid == 0)  // the matrix, where its copy was given up, lands before its memory is given back (bounded again)
+    for (int w = 0; w < (1 << 20) && !mbar_try_wait(smem_u32(mbar), 0); ++w) {
+    }
   __syncthreads();
   if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(tmem), "r"(512));
 }
