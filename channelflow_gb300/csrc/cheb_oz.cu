@@ -937,6 +937,7 @@ cudaError_t launch_cheb_oz(const GridDev& g, int N, bool inverse, int nlines, si
   a.err = err;
   bool inplace = false;
   for (int i = 0; i < njobs; ++i) {
+    if (jobs[i].inplace && jobs[i].pd) return cudaErrorInvalidValue;  // the held parity has no derivative term
     a.job[i] = jobs[i];
     inplace = inplace || jobs[i].inplace;
   }

@@ -88,7 +88,7 @@ struct OzJob {
   // forward: out = F (wF in + wK (i kx pkx + i kz pkz)) + wD DF pd (pkx null: F in; in may be null beside pkx)
   const double *pkx, *pkz, *pd;
   double wF, wK, wD;
-  int inplace;  // forward: out == in
+  int inplace;  // out == in; forward: not beside pd
 };
 size_t oz_matrix_bytes(int N);
 bool oz_matrix(int N, int kind, std::vector<uint16_t>& digits, std::vector<int>& rexp);
