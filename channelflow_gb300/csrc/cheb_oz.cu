@@ -8,6 +8,8 @@
 // 2^-9(i + j), the 28 pairs with i + j <= 6 are kept.  All pairs of one weight and all K points sum into one FP32
 // accumulator of tensor memory below 2^24 (checked for every matrix row at set-up), so every sum is exact and the
 // result carries about 2^-59 of the line's sum of magnitudes, whatever the order of the sums.
+// (Error-free splitting of a matrix product into digit products: Ozaki, Ogita, Oishi and Rump, 2012.)  The bound of the
+// check holds for every Ny from 3 to 144 but 116, 122, 134-136, 138, 141 and 143.
 //
 // Parity: the even and odd coefficients are two systems of half the size (T[N-1-j][n] = (-1)^n T[j][n]): the inverse
 // transform multiplies each parity's coefficients and combines y_j = E_j + O_j, y_{N-1-j} = E_j - O_j; the forward
@@ -28,8 +30,8 @@
 // and inverse transforms 190 us (FFT form) -> 68 us and 10 us more in the x pass, which forms the vorticity; forward 91
 // -> 56 us.  72x57x90, skew-symmetric: gradient 107 -> 28 us, forward with divergence 484 -> 43 us.  Ny = 35, 190 modes:
 // 29 -> 17 us and 24 -> 11 us (10 and 8 with k_cheb_oz_few).  FlowField y transform 128x97x128: 1340 -> 83 and 96 us.
-// Relative error of one transform 5e-17 (FP64 products 2e-16 ... 5e-16).  Bound by instruction issue and latency of the digits and the sums (16 warps
-// an SM).  256 threads (and K steps of 16): 102 and 70 us.
+// Relative error of one transform 5e-17 (FP64 products 2e-16 ... 5e-16).  Bound by instruction issue and latency of the
+// digits and the sums (16 warps an SM).  256 threads (and K steps of 16): 102 and 70 us.
 #include <cuda_fp16.h>
 
 #include <algorithm>
@@ -170,14 +172,14 @@ __device__ __forceinline__ void oz_store(unsigned char* dst, const long long (&x
 
 // sum_s r_s 2^(9 (6 - s) - 8) of the exact FP32 sums r
 __device__ __forceinline__ long long oz_sum(const uint32_t (&r)[OZ_DIGITS]) {
-            int d[OZ_DIGITS];
-  #pragma unroll
-            for (int s = 0; s < OZ_DIGITS; ++s) d[s] = __float2int_rn(__uint_as_float(r[s]));
-                      long long x = (long long)(2 * d[5] + ((d[6] + 128) >> 8));
-            x = fx_mw(d[4], 1 << 10, x);
-            x = fx_mw(d[3], 1 << 19, x);
-            x = fx_mw(d[2], 1 << 28, x);
-            x += (long long)((unsigned long long)(((unsigned)d[0] << 14) + ((unsigned)d[1] << 5)) << 32);
+  int d[OZ_DIGITS];
+#pragma unroll
+  for (int s = 0; s < OZ_DIGITS; ++s) d[s] = __float2int_rn(__uint_as_float(r[s]));
+  long long x = (long long)(2 * d[5] + ((d[6] + 128) >> 8));
+  x = fx_mw(d[4], 1 << 10, x);
+  x = fx_mw(d[3], 1 << 19, x);
+  x = fx_mw(d[2], 1 << 28, x);
+  x += (long long)((unsigned long long)(((unsigned)d[0] << 14) + ((unsigned)d[1] << 5)) << 32);
   return x;
 }
 
@@ -224,31 +226,31 @@ struct OzLine {
     }
     hasb = __any_sync(0xffffffffu, base != nullptr || shift != 0.0);
   }
-      // v[i] = point n0 + i dn of the line, i < cnt, else zero
-      __device__ __forceinline__ void load8(double (&v)[8], int n0, int dn, int cnt) const {
-        unsigned o = (unsigned)n0 * ld + gl;
-  #pragma unroll
-        for (int i = 0; i < 8; ++i, o += (unsigned)dn * ld) v[i] = src && i < cnt ? src[o] : 0.0;
-        if constexpr (INV) {
-          if (hasb) {
-            for (int i = 0; i < 8; ++i)
-              if (i < cnt) {
-                if (base) v[i] += base[n0 + i * dn];
-                if (n0 + i * dn == 0) v[i] -= shift;
-              }
+  // v[i] = point n0 + i dn of the line, i < cnt, else zero
+  __device__ __forceinline__ void load8(double (&v)[8], int n0, int dn, int cnt) const {
+    unsigned o = (unsigned)n0 * ld + gl;
+#pragma unroll
+    for (int i = 0; i < 8; ++i, o += (unsigned)dn * ld) v[i] = src && i < cnt ? src[o] : 0.0;
+    if constexpr (INV) {
+      if (hasb) {
+        for (int i = 0; i < 8; ++i)
+          if (i < cnt) {
+            if (base) v[i] += base[n0 + i * dn];
+            if (n0 + i * dn == 0) v[i] -= shift;
           }
-        } else if (!fd && job.pkx) {
-          double px[8], pz[8];
-          o = (unsigned)n0 * ld + (gl ^ 1);
-  #pragma unroll
-          for (int i = 0; i < 8; ++i, o += (unsigned)dn * ld) {
-            px[i] = i < cnt ? job.pkx[o] : 0.0;
-            pz[i] = i < cnt ? job.pkz[o] : 0.0;
-          }
-  #pragma unroll
-          for (int i = 0; i < 8; ++i) v[i] = fma(job.wF, v[i], job.wK * fma(kx, px[i], kz * pz[i]));
-        }
       }
+    } else if (!fd && job.pkx) {
+      double px[8], pz[8];
+      o = (unsigned)n0 * ld + (gl ^ 1);
+#pragma unroll
+      for (int i = 0; i < 8; ++i, o += (unsigned)dn * ld) {
+        px[i] = i < cnt ? job.pkx[o] : 0.0;
+        pz[i] = i < cnt ? job.pkz[o] : 0.0;
+      }
+#pragma unroll
+      for (int i = 0; i < 8; ++i) v[i] = fma(job.wF, v[i], job.wK * fma(kx, px[i], kz * pz[i]));
+    }
+  }
   // magnitudes of every fourth point
   __device__ __forceinline__ void magnitudes(OzSum& sum, int quarter) const {
     if (act)

@@ -666,7 +666,7 @@ struct cfgpu_dns_s {
   void *cinvA = nullptr, *cinvB = nullptr, *cfwdA = nullptr, *cfwdB = nullptr;
   void *cderA = nullptr, *cderB = nullptr, *basey = nullptr;  // fused curl: (2/L) T'_n(y_j); U, U', W, W' at y_j
   void *cdfA = nullptr, *cdfB = nullptr;                       // (2/L) diff o chebyfft, parity split
-  void* zbasey = nullptr;  // zero base profiles [nb][4N] (LinearAboutProfile: u, v, w without base flow)
+  void* zbasey = nullptr;  // zero base profiles [nb][4N] (mixed LinearAboutProfile: u, v, w without base flow)
   // Mixed precision: the FP32 constant tables above live in one block of DITHER_V dithered versions (cS bytes
   // apart; the pointers above address version 0), basey/baseyS likewise; dver holds each field's version.
   void* cblock = nullptr;
@@ -2129,7 +2129,7 @@ int dns_create_impl(cfgpu_dns d, const cfgpu_grid* grid, const cfgpu_flags* flag
   CKS(dalloc(&tmp, nout * cd * rs, B));
   d->F3 = tmp;
   CKS(dalloc(&d->scratch, 8 * cd, B));
-  if (f.nonlinearity == CFGPU_LinearAboutProfile) {
+  if (f.nonlinearity == CFGPU_LinearAboutProfile && !fp64) {
     CKS(dalloc(&tmp, 4 * (size_t)Ny * nb * rs, B));
     d->zbasey = tmp;
     CK(cudaMemsetAsync(d->zbasey, 0, 4 * (size_t)Ny * nb * rs, d->st));

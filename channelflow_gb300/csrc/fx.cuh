@@ -1,8 +1,8 @@
 // 64-bit fixed-point arithmetic for the FP64 path (FFTs: fx_fft.cuh).
 //
 // GB300 issues one FP64 warp instruction per 64 cycles and SM sub-partition, but a 64-bit integer addition
-// (IADD3 pair) in about 2 and a 32 x 32 -> 64 bit multiply-add (IMAD.WIDE) in about 5 (measured with a
-// throughput probe).  An FFT is mostly additions, so the FP64 path's transforms run on integers: a sequence is
+// (IADD3 pair) in about 2 and a 32 x 32 -> 64 bit multiply-add (IMAD.WIDE) in 8 to 11 (measured with a
+// throughput probe, 8 warps a sub-partition).  An FFT is mostly additions, so the FP64 path's transforms run on integers: a sequence is
 // scaled by one power of two such that the sum of the magnitudes of its elements (real plus imaginary) stays below
 // 2^61, which bounds the modulus of every intermediate value of the transform, and rounded to integers.  Its rounding
 // errors are a few units of 2^-61 of that sum: up to FX_LMAX points (fx_plan.h) below those of the same FFT in FP64, whose

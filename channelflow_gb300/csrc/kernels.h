@@ -63,7 +63,8 @@ cudaError_t launch_cheb_tc(int N, int nlines, int ncomp, const float* in, size_t
                            const void* Ag, int* err, cudaStream_t st);
 
 // Chebyshev transforms of FP64 lines on the tensor cores by exact integer products (cheb_oz.cu).  Matrix tables:
-// digits and row exponents of oz_matrix, uploaded; false where N is too large for exact accumulation.
+// digits and row exponents of oz_matrix, uploaded; false where its bound for exact accumulation fails (N above 144, and
+// 116, 122, 134-136, 138, 141, 143 for the forward matrix).
 enum { OZ_T = 0, OZ_F = 1, OZ_DF = 2 };  // inverse, forward, derivative of forward (for b - a = 2)
 constexpr int OZ_MAX_JOBS = 6;
 struct OzMatrix {

@@ -313,10 +313,11 @@ __global__ void __launch_bounds__(32, WARPS) k_tau_pv_seg(GridDev g, int N, Solv
 // solve of the (0,0) mode's real part under the bulk-velocity constraint) from q and Rx, Rz.  One warp: one
 // mode, u (lanes 0-15) and w (16-31).
 // ---------------------------------------------------------------------------
-// Warps an SM against registers: beyond 12 rows a lane, 16 warps spill (97 rows: 52 us, 12 warps 44, 10 warps 41).
+// Warps an SM against registers: 16 up to 8 rows a lane (L), 12 with 9 rows, 10 from 10 rows on, where more warps spill
+// (Ny = 97, 13 rows: 16 warps 52 us, 12 warps 44, 10 warps 41).
 template <int L>
-__global__ void __launch_bounds__(32, L >= 10 ? 10 : (L == 9 ? 12 : 16)) k_tau_uw_seg(GridDev g, int N, SolveParams sp, SolvePtrs P, HelmB hb,
-                                                   TauTable tt) {
+__global__ void __launch_bounds__(32, L >= 10 ? 10 : (L == 9 ? 12 : 16)) k_tau_uw_seg(GridDev g, int N, SolveParams sp,
+                                                                                      SolvePtrs P, HelmB hb, TauTable tt) {
   extern __shared__ double sm[];
   pdl_wait();
   pdl_trigger();
@@ -410,7 +411,7 @@ cudaError_t run_seg(const GridDev& g, int N, const SolveParams& sp, const SolveP
   }();
   (void)attr;
   // More warps in flight than 12 an SM hide more of the table loads; with fewer modes than that the registers are the
-  // better use (Ny = 49: 31744 modes 340 us with 12, 304 with 20; 33 rows, 190 modes 17.0 and 18.3)
+  // better use (Ny = 49: 31744 modes 340 us with 12, 304 with 20; Ny = 33, 190 modes 17.0 and 18.3)
   const dim3 grid((g.Md + 1) / 2);
   cudaError_t e;
   if (L <= 8 && grid.x > 12 * 152) {
