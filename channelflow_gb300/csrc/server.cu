@@ -372,6 +372,12 @@ void worker(cfgpu_server_s* s, Ens* e) {
   }
   std::vector<std::pair<Request*, int>> starting;
   std::vector<double> cfl_now(e->nb, 0.0);
+  // a wait ran out in a kernel of the start-up DNS: it stays marked, a new ensemble serves the requests that follow
+  auto marked = [&] {
+    if (cfgpu_rt::wait_status(e->startup_dns()) == CFGPU_OK) return false;
+    fail_all(s, e, cfgpu_last_error());
+    return true;
+  };
   while (st == CFGPU_OK) {
     {
       std::unique_lock<std::mutex> lk(s->mu);
@@ -392,6 +398,7 @@ void worker(cfgpu_server_s* s, Ens* e) {
       if (start_request(s, e, *ri.first, ri.second) != CFGPU_OK)
         fail_request(s, e, *ri.first, ri.second, cfgpu_last_error());
     starting.clear();
+    if (marked()) break;
     // next chunk: the largest step count that ends no request's interval early
     int k = s->max_steps.load();
     bool any = false;
@@ -431,6 +438,7 @@ void worker(cfgpu_server_s* s, Ens* e) {
       if (r && r->left == 0 && interval_end(s, e, i, cfl_now[i]) != CFGPU_OK)
         fail_request(s, e, *r, i, cfgpu_last_error());
     }
+    if (marked()) break;
   }
   release_handles(e);
   std::lock_guard<std::mutex> lk(s->mu);
